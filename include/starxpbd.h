@@ -86,6 +86,10 @@ int sx_jacobi_sweep_variant_info(int variant, int* g, int* block);
  * read with the evict-first cache policy (for batches larger than L2).  Every
  * form gives the same result bit for bit. */
 int sx_jacobi_sweep_variant_form(int variant, int* lanes, int* streaming);
+/* The variant the library recommends for a mesh of n_verts vertices (a rule on
+ * the size, measured on grid cloths; timing the variants on the mesh itself can
+ * only do better). */
+int sx_jacobi_sweep_default_variant(int n_verts, int fast);
 int sx_jacobi_sweep_v(const float* x4, const float* y_in4, float* y_out4, const float* fixed, const int* adj_ptr,
                       const int* adj, int n_verts, float k_spring, float k_bend, int bend_on_y, int variant,
                       void* stream);

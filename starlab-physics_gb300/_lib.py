@@ -49,6 +49,7 @@ SIGNATURES = {
     "sx_predict": ([P, P, P, P, I, F, F, F, F, P], I),
     "sx_jacobi_sweep": ([P, P, P, P, P, P, I, F, F, I, P], I),
     "sx_jacobi_sweep_variants": ([], I),
+    "sx_jacobi_sweep_default_variant": ([I, I], I),
     "sx_jacobi_sweep_variant_info": ([I, P, P], I),
     "sx_jacobi_sweep_variant_form": ([I, P, P], I),
     "sx_set_programmatic_launch": ([I], I),
@@ -189,6 +190,7 @@ class _Calls:
             raise AttributeError(name)
         if SIGNATURES[name][1] is I and name not in ("sx_version", "sx_mlp_param_count", "sx_mlp_bf16_count",
                                                      "sx_jacobi_sweep_variants", "sx_jacobi_sweep_packed_forms",
+                                                     "sx_jacobi_sweep_default_variant",
                                                      "sx_contact_pairs_project_variants",
                                                      "sx_contact_pairs_project_variant_pipelined",
                                                      "sx_batched_substep_variants",

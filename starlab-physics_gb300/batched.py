@@ -190,8 +190,10 @@ class BatchedSolver:
         self._nc = torch.zeros(V, dtype=torch.int32, device=dev)
         # learned warm start (learned.WarmStart) run after each prediction
         self.warm = None
-        # launch configuration of the fixed-count sweep (autotune() picks one)
-        self.sweep_variant = 0
+        # launch configuration of the fixed-count sweep: None = the library's
+        # choice for this batch size (autotune() times all of them)
+        self.sweep_variant = None
+        self._default_variant = [int(sx.sx_jacobi_sweep_default_variant(V, f)) for f in (0, 1)]
         # the sweep over the packed, shared-memory-staged adjacency
         # (sx_jacobi_sweep_packed; same results; autotune() decides)
         self._packed_sweep = False
@@ -361,7 +363,9 @@ class BatchedSolver:
         else:
             sx.sx_jacobi_sweep_mode(ptr(self.x4), ptr(self.y4), ptr(self._y_other), ptr(self.fixed),
                                     ptr(self.adj_ptr), ptr(self.adj), self.num_verts, k_spring, k_bend,
-                                    1 if self.bending_on == "y" else 0, self.sweep_variant, fast, s)
+                                    1 if self.bending_on == "y" else 0,
+                                    self._default_variant[fast] if self.sweep_variant is None else self.sweep_variant,
+                                    fast, s)
         self._swap_y()
         if it == 0:
             sx.sx_batched_obstacle_broadphase(

@@ -472,6 +472,23 @@ constexpr int kNumSweepVariants = sizeof(kSweepVariants) / sizeof(kSweepVariants
 
 extern "C" int sx_jacobi_sweep_variants(void) { return kNumSweepVariants; }
 
+// With few vertices the sweep is one warp's chain of loads and divisions, which
+// lanes shorten; with several warps per scheduler the shuffles cost more than
+// they hide.  Whole sphere-drape frames of 10 x 30 iterations (ms; 4 lanes x 3
+// entries / 2 lanes x 3 / 2 entries x 128 threads / 4 x 128; GB300, 2070 MHz):
+//   exact: 16 384 vertices 4.79 / 4.85 / 5.40 / 5.26, 25 159: 5.32 / 5.33 / 5.78
+//   / 5.68, 36 000: 5.46 / 5.79 / 6.13 / 6.20, 65 536: 8.96 / 9.79 / 8.87 / 8.86;
+//   fast: 16 384: 4.76 / 4.85 / 5.25 / 5.06, 25 159: 5.06 / 5.27 / 5.65 / 5.35,
+//   36 000: 5.76 / 5.54 / 5.98 / 5.82, 65 536: 8.85 / 8.38 / 8.73 / 8.53.
+// Alone, in graphs of back-to-back sweeps (us): exact 359 999 vertices 19.8 /
+// 15.3 / 12.9 / 14.0, 600 000 in a batch 30.5 / 22.6 / 18.9 / 20.6; fast 359 999:
+// 17.5 / 12.9 / 13.8 / 11.5, 600 000: 26.8 / 18.7 / 17.0 / 15.9.
+extern "C" int sx_jacobi_sweep_default_variant(int n_verts, int fast) {
+    if (n_verts <= (fast ? 30000 : 49152)) return 12;  // 4 lanes, 3 entries: a 12-entry vertex in one step
+    if (!fast) return 3;                                // 2 entries x 128 threads
+    return n_verts <= 200000 ? 9 : 5;                   // 2 lanes, 3 entries; 4 entries x 128 threads
+}
+
 extern "C" int sx_jacobi_sweep_variant_info(int variant, int* g, int* block) {
     SX_REQUIRE(variant >= 0 && variant < kNumSweepVariants && g && block, "sx_jacobi_sweep_variant_info: bad variant");
     *g = kSweepVariants[variant].g;

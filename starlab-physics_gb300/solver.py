@@ -119,8 +119,10 @@ class Solver:
         self.enable_edge_edge = False
         self._ee = None
         self._sewing = None  # (sewn, sptr, partner, scratch, stiffness)
-        # launch configuration of the fixed-count sweep (autotune() picks one)
-        self.sweep_variant = 0
+        # launch configuration of the fixed-count sweep: None = the library's
+        # choice for this mesh size (autotune() times all of them)
+        self.sweep_variant = None
+        self._default_variant = [int(sx.sx_jacobi_sweep_default_variant(mesh_dy.num_verts, f)) for f in (0, 1)]
         self._packed_sweep = False
         self.packed_form = 0  # the packed sweep staged per block (0) or read from global memory (1)
         # launch configuration of the contact-pair projection (None: the
@@ -224,7 +226,8 @@ class Solver:
         elif self.tol is None:
             sx.sx_jacobi_sweep_mode(ptr(m.x4), ptr(m.y4), ptr(self._y_other), ptr(m.fixed), ptr(m.adj_ptr),
                                     ptr(m.adj), m.num_verts, k_spring, k_bend, 1 if self.bending_on == "y" else 0,
-                                    self.sweep_variant, fast, stream_handle())
+                                    self._default_variant[fast] if self.sweep_variant is None else self.sweep_variant,
+                                    fast, stream_handle())
         else:
             check = 1 if iteration > 0 and iteration % self.check_every == 0 else 0
             sx.sx_jacobi_sweep_checked_mode(ptr(m.x4), ptr(m.y4), ptr(self._y_other), ptr(m.fixed), ptr(m.adj_ptr),
