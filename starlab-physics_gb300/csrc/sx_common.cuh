@@ -107,17 +107,28 @@ __device__ __forceinline__ bool overlap(V3 a0, V3 a1, V3 b0, V3 b1) {
 __device__ __forceinline__ int f2i_sat(float f) { return __float2int_rz(f); }
 
 // ---- contact accumulation in 64-bit fixed point (40 fractional bits) -----------
-constexpr double kFixScale = 1099511627776.0;      // 2^40
-constexpr double kFixInv = 1.0 / 1099511627776.0;  // 2^-40
-constexpr double kFixMax = 4611686018427387904.0;  // 2^62
+// round(c * 2^40) to nearest even, saturated at +-2^62 (0 for NaN) with *bad set.
+// Without FP64, of which an SM does two operations a clock: c * 2^20 splits
+// exactly into a whole number and a rest of at most 1/2; the whole number times
+// 2^20 is even, so rounding the rest times 2^20 alone also breaks ties as
+// rounding the sum would.
 __device__ __forceinline__ long long to_fix(float c, int* bad) {
-    double d = (double)c * kFixScale;
-    if (d != d) { *bad = 1; return 0; }
-    if (d >= kFixMax) { *bad = 1; return 4611686018427387904LL; }
-    if (d <= -kFixMax) { *bad = 1; return -4611686018427387904LL; }
-    return __double2ll_rn(d);
+    const float t = c * 1048576.0f;  // exact
+    if (fabsf(t) < 1073741824.0f) {
+        const float hi = rintf(t);
+        const int lo = __float2int_rn((t - hi) * 1048576.0f);
+        return (long long)__float2int_rn(hi) * 1048576 + lo;
+    }
+    if (fabsf(c) < 4194304.0f) return __float2ll_rn(t) * 1048576;  // a whole number already
+    *bad = 1;
+    return c != c ? 0 : c > 0.0f ? 4611686018427387904LL : -4611686018427387904LL;
 }
-__device__ __forceinline__ float from_fix(long long a) { return __double2float_rn(__ll2double_rn(a) * kFixInv); }
+// a * 2^-40 rounded to double, then to float; below 2^53 the first step is exact
+__device__ __forceinline__ float from_fix(long long a) {
+    constexpr float inv = 1.0f / 1099511627776.0f;  // 2^-40
+    if ((unsigned long long)(a + 9007199254740992LL) <= 18014398509481984ULL) return __ll2float_rn(a) * inv;
+    return __double2float_rn(__ll2double_rn(a)) * inv;
+}
 
 // In-place scan (exclusive or inclusive) of n uint32 on one block (sx_lbvh.cu).
 int scan_u32(unsigned* data, int n, int inclusive, cudaStream_t s);

@@ -7,59 +7,95 @@
 // integer atomics, so the sum does not depend on the order in which threads
 // arrive (the reference uses float atomics, whose result does).
 #include "sx_common.cuh"
+#include "sx_exact.cuh"
 #include "sx_sweep.cuh"
 
 namespace sx {
 
+// Reciprocals and quotients of the narrow phase, two bodies with the same
+// value: IEEE = false is straight-line code (sx_exact.cuh) that records the
+// operands' magnitudes; when they leave [2^-100, 2^100] (degenerate triangles,
+// coincident points) the caller evaluates the pair again with '/'.  The three
+// 2x2 solves of a classification then run side by side: a pair's chain of
+// dependent divisions, not the chip's throughput, is what a contact sweep over
+// a few thousand pairs waits for.
+template <bool IEEE>
+struct Arith {
+    float lo = 1.0f, hi = 1.0f;
+    __device__ __forceinline__ void note(float v) {
+        lo = fminf(lo, v);
+        hi = fmaxf(hi, v);
+    }
+    __device__ __forceinline__ float rcp(float b) {
+        if (IEEE) return 1.0f / b;
+        note(fabsf(b));
+        return rcp_rn(b);
+    }
+    __device__ __forceinline__ float div(float a, float b) {
+        if (IEEE) return a / b;
+        const float q = div_rn(a, b, rcp(b));
+        note(a == 0.0f ? 1.0f : fabsf(a));
+        note(a == 0.0f ? 1.0f : fabsf(q));
+        return q;
+    }
+    // min and max pass over a NaN: both bodies then give NaN
+    __device__ __forceinline__ bool ok() const {
+        return IEEE || (lo >= 7.88860905e-31f && hi <= 1.26765060e30f);  // 2^-100, 2^100
+    }
+};
+
 // 2x2 solve A^{-1} b with A^{-1} = (1/det) [[a11, -a01], [-a10, a00]]
-__device__ __forceinline__ void solve2(float a00, float a01, float a10, float a11, float b0, float b1, float* p0,
-                                       float* p1) {
+template <typename A>
+__device__ __forceinline__ void solve2(A& ar, float a00, float a01, float a10, float a11, float b0, float b1,
+                                       float* p0, float* p1) {
     float det = a00 * a11 - a01 * a10;
-    float id = 1.0f / det;
+    float id = ar.rcp(det);
     float m00 = id * a11, m01 = id * (-a01), m10 = id * (-a10), m11 = id * a00;
     *p0 = m00 * b0 + m01 * b1;
     *p1 = m10 * b0 + m11 * b1;
 }
 
 // distance.py:5-47
-__device__ int d_type_PT(V3 v0, V3 v1, V3 v2, V3 v3) {
-    V3 v12 = sub(v2, v1), v13 = sub(v3, v1);
-    V3 n = cross(v12, v13);
-    V3 v13n = cross(v12, n);
-    V3 v10 = sub(v0, v1);
-    float p00, p01;
-    solve2(dot(v12, v12), dot(v12, v13n), dot(v13n, v12), dot(v13n, v13n), dot(v12, v10), dot(v13n, v10), &p00,
+template <typename A>
+__device__ __forceinline__ int d_type_PT(A& ar, V3 v0, V3 v1, V3 v2, V3 v3) {
+    const V3 v12 = sub(v2, v1), v13 = sub(v3, v1);
+    const V3 n = cross(v12, v13);
+    const V3 v13n = cross(v12, n);
+    const V3 v10 = sub(v0, v1);
+    const V3 v32 = sub(v3, v2), v32n = cross(v32, n), v20 = sub(v0, v2);
+    const V3 v31 = sub(v1, v3), v31n = cross(v31, n), v30 = sub(v0, v3);
+    float p00, p01, p10, p11, p20, p21;
+    solve2(ar, dot(v12, v12), dot(v12, v13n), dot(v13n, v12), dot(v13n, v13n), dot(v12, v10), dot(v13n, v10), &p00,
            &p01);
-    if (p00 > 0.0f && p00 < 1.0f && p01 >= 0.0f) return 3;
-    V3 v32 = sub(v3, v2), v32n = cross(v32, n), v20 = sub(v0, v2);
-    float p10, p11;
-    solve2(dot(v32, v32), dot(v32, v32n), dot(v32n, v32), dot(v32n, v32n), dot(v32, v20), dot(v32n, v20), &p10,
+    solve2(ar, dot(v32, v32), dot(v32, v32n), dot(v32n, v32), dot(v32n, v32n), dot(v32, v20), dot(v32n, v20), &p10,
            &p11);
-    if (p10 > 0.0f && p10 < 1.0f && p11 >= 0.0f) return 4;
-    V3 v31 = sub(v1, v3), v31n = cross(v31, n), v30 = sub(v0, v3);
-    float p20, p21;
-    solve2(dot(v31, v31), dot(v31, v31n), dot(v31n, v31), dot(v31n, v31n), dot(v31, v30), dot(v31n, v30), &p20,
+    solve2(ar, dot(v31, v31), dot(v31, v31n), dot(v31n, v31), dot(v31n, v31n), dot(v31, v30), dot(v31n, v30), &p20,
            &p21);
-    if (p20 > 0.0f && p20 < 1.0f && p21 >= 0.0f) return 5;
-    if (p00 <= 0.0f && p20 >= 1.0f) return 0;
-    if (p10 <= 0.0f && p00 >= 1.0f) return 1;
-    if (p20 <= 0.0f && p10 >= 1.0f) return 2;
-    return 6;
+    int dt = 6;
+    if (p20 <= 0.0f && p10 >= 1.0f) dt = 2;
+    if (p10 <= 0.0f && p00 >= 1.0f) dt = 1;
+    if (p00 <= 0.0f && p20 >= 1.0f) dt = 0;
+    if (p20 > 0.0f && p20 < 1.0f && p21 >= 0.0f) dt = 5;
+    if (p10 > 0.0f && p10 < 1.0f && p11 >= 0.0f) dt = 4;
+    if (p00 > 0.0f && p00 < 1.0f && p01 >= 0.0f) dt = 3;
+    return dt;
 }
 
 __device__ __forceinline__ float d_PP(V3 a, V3 b) {
     V3 d = sub(a, b);
     return dot(d, d);
 }
-__device__ __forceinline__ float d_PE(V3 p, V3 e0, V3 e1) {
+template <typename A>
+__device__ __forceinline__ float d_PE(A& ar, V3 p, V3 e0, V3 e1) {
     V3 c = cross(sub(e0, p), sub(e1, p));
     V3 e = sub(e1, e0);
-    return dot(c, c) / dot(e, e);
+    return ar.div(dot(c, c), dot(e, e));
 }
-__device__ __forceinline__ float d_PT(V3 p, V3 t0, V3 t1, V3 t2) {
+template <typename A>
+__device__ __forceinline__ float d_PT(A& ar, V3 p, V3 t0, V3 t1, V3 t2) {
     V3 b = cross(sub(t1, t0), sub(t2, t0));
     float s = dot(sub(p, t0), b);
-    return s * s / dot(b, b);
+    return ar.div(s * s, dot(b, b));
 }
 // Closed-form gradients of the squared distances:
 //  PP: g_a = 2(a-b), g_b = -g_a
@@ -73,12 +109,13 @@ __device__ __forceinline__ void g_PP(V3 a, V3 b, V3* ga, V3* gb) {
     *ga = scale(2.0f, sub(a, b));
     *gb = neg(*ga);
 }
-__device__ __forceinline__ void g_PE(V3 p, V3 e0, V3 e1, V3* gp, V3* g0, V3* g1) {
+template <typename A>
+__device__ __forceinline__ void g_PE(A& ar, V3 p, V3 e0, V3 e1, V3* gp, V3* g0, V3* g1) {
     V3 a = sub(e0, p), b = sub(e1, p);
     V3 c = cross(a, b);
     V3 e = sub(e1, e0);
     float L = dot(e, e);
-    float iL = 1.0f / L;
+    float iL = ar.rcp(L);
     float d = dot(c, c) * iL;
     V3 bc = cross(b, c), ca = cross(c, a);
     float td = 2.0f * d;
@@ -88,13 +125,14 @@ __device__ __forceinline__ void g_PE(V3 p, V3 e0, V3 e1, V3* gp, V3* g0, V3* g1)
     *g1 = scale(iL, t1);
     *gp = neg(add(*g0, *g1));
 }
-__device__ __forceinline__ void g_PT(V3 p, V3 t0, V3 t1, V3 t2, V3* gp, V3* g0, V3* g1, V3* g2) {
+template <typename A>
+__device__ __forceinline__ void g_PT(A& ar, V3 p, V3 t0, V3 t1, V3 t2, V3* gp, V3* g0, V3* g1, V3* g2) {
     V3 u = sub(t1, t0), w = sub(t2, t0);
     V3 n = cross(u, w);
     V3 r = sub(p, t0);
     float s = dot(r, n);
     float N = dot(n, n);
-    float iN = 1.0f / N;
+    float iN = ar.rcp(N);
     float d = (s * s) * iN;
     float ts = 2.0f * s, td = 2.0f * d;
     *gp = scale(ts * iN, n);
@@ -105,24 +143,90 @@ __device__ __forceinline__ void g_PT(V3 p, V3 t0, V3 t1, V3 t2, V3* gp, V3* g0, 
     *g0 = neg(add(add(*gp, *g1), *g2));
 }
 
-__device__ float pt_distance(int dtype, V3 x0, V3 x1, V3 x2, V3 x3, V3 g[4], bool want_grad, float dflt) {
-    float d = dflt;
-    switch (dtype) {
-        case 0: d = d_PP(x0, x1); if (want_grad) g_PP(x0, x1, &g[0], &g[1]); break;
-        case 1: d = d_PP(x0, x2); if (want_grad) g_PP(x0, x2, &g[0], &g[2]); break;
-        case 2: d = d_PP(x0, x3); if (want_grad) g_PP(x0, x3, &g[0], &g[3]); break;
-        case 3: d = d_PE(x0, x1, x2); if (want_grad) g_PE(x0, x1, x2, &g[0], &g[1], &g[2]); break;
-        case 4: d = d_PE(x0, x2, x3); if (want_grad) g_PE(x0, x2, x3, &g[0], &g[2], &g[3]); break;
-        case 5: d = d_PE(x0, x1, x3); if (want_grad) g_PE(x0, x1, x3, &g[0], &g[1], &g[3]); break;
-        case 6: d = d_PT(x0, x1, x2, x3); if (want_grad) g_PT(x0, x1, x2, x3, &g[0], &g[1], &g[2], &g[3]); break;
-        default: break;
-    }
-    return d;
-}
 __device__ __forceinline__ int region_mask(int dtype) {
     // bit k set: vertex k (0 = query point, 1..3 = triangle) takes part
     return dtype == 0 ? 0x3 : dtype == 1 ? 0x5 : dtype == 2 ? 0x9 : dtype == 3 ? 0x7 : dtype == 4 ? 0xD
          : dtype == 5 ? 0xB : dtype == 6 ? 0xF : 0;
+}
+
+// The feature of region dt: triangle corner a of a vertex region, the edge
+// (a, b) of an edge region, so that a warp whose pairs lie in several regions
+// runs the point, edge and face code once each, not once per region.
+__device__ __forceinline__ V3 region_a(int dt, const V3 x[4]) {
+    return dt == 0 || dt == 3 || dt == 5 ? x[1] : dt == 1 || dt == 4 ? x[2] : x[3];
+}
+__device__ __forceinline__ V3 region_b(int dt, const V3 x[4]) { return dt == 3 ? x[2] : x[3]; }
+
+template <typename A>
+__device__ __forceinline__ float pt_distance(A& ar, int dt, const V3 x[4]) {
+    if (dt == 6) return d_PT(ar, x[0], x[1], x[2], x[3]);
+    if (dt <= 2) return d_PP(x[0], region_a(dt, x));
+    return d_PE(ar, x[0], region_a(dt, x), region_b(dt, x));
+}
+// zero for the vertices that do not take part
+template <typename A>
+__device__ __forceinline__ void pt_gradient(A& ar, int dt, const V3 x[4], V3 g[4]) {
+    if (dt == 6) {
+        g_PT(ar, x[0], x[1], x[2], x[3], &g[0], &g[1], &g[2], &g[3]);
+        return;
+    }
+    const V3 zero{0.0f, 0.0f, 0.0f};
+    V3 ga, gb = zero;
+    if (dt <= 2)
+        g_PP(x[0], region_a(dt, x), &g[0], &ga);
+    else
+        g_PE(ar, x[0], region_a(dt, x), region_b(dt, x), &g[0], &ga, &gb);
+    g[1] = dt == 0 || dt == 3 || dt == 5 ? ga : zero;
+    g[2] = dt == 1 || dt == 4 ? ga : dt == 3 ? gb : zero;
+    g[3] = dt == 2 ? ga : dt == 4 || dt == 5 ? gb : zero;
+}
+
+// One candidate: its region, squared distance and, where d < dHat, gradients,
+// schur complement and multiplier of its kind.
+//   VT_ST (collision_constraints_x.py:6-69): dynamic vertex vs static triangle;
+//     w[0] = m_inv, schur = w0 g0.g0, ld = c (dHat - d) / (c schur + 1)
+//   VT_DY (:176-310): self contact; w[k] = fixed m_inv, schur = the sum of
+//     w_k g_k.g_k over the region's vertices + 1e-4, ld = (dHat - d) / schur
+//   TV_ST (:72-173): static vertex vs dynamic triangle; as VT_ST with the sum
+//     over the triangle's vertices
+// The kind is a run-time value: one copy of the classification serves a warp
+// whose lanes hold different kinds, and fits the instruction cache.
+enum PairKind { VT_ST, VT_DY, TV_ST };
+struct PairSolve {
+    int dt;
+    float d, schur, ld;
+    V3 g[4];
+};
+// the vertices a kind corrects, among those of the region
+__device__ __forceinline__ int moved_mask(int kind, int dt) {
+    return region_mask(dt) & (kind == VT_ST ? 0x1 : kind == TV_ST ? 0xE : 0xF);
+}
+template <bool IEEE>
+__device__ __forceinline__ bool pair_solve(int kind, const V3 x[4], const float w[4], float dHat, float compliance,
+                                           PairSolve& r) {
+    Arith<IEEE> ar;
+    r.dt = d_type_PT(ar, x[0], x[1], x[2], x[3]);
+    r.d = pt_distance(ar, r.dt, x);
+    r.schur = r.ld = 0.0f;
+    if (r.d < dHat) {
+        pt_gradient(ar, r.dt, x, r.g);
+        const int m = moved_mask(kind, r.dt);
+        float s = 0.0f;
+        bool first = true;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float t = w[k] * dot(r.g[k], r.g[k]);
+            if (m & (1 << k)) {
+                s = first ? t : s + t;
+                first = false;
+            }
+        }
+        const float gap = dHat - r.d;
+        if (kind == VT_DY) s = s + 1e-4f;
+        r.ld = ar.div(kind == VT_DY ? gap : compliance * gap, kind == VT_DY ? s : compliance * s + 1.0f);
+        r.schur = s;
+    }
+    return ar.ok();
 }
 
 __device__ __forceinline__ void acc_add(long long* dx, int* nc, int v, float a, V3 g, int* bad) {
@@ -151,95 +255,71 @@ struct PairOut {
     }
 };
 
-// One candidate of each kind.  g receives the four gradients (zero where the
-// feature excludes a vertex); *schur_out the value the reference records.
-// __vt_st (collision_constraints_x.py:6-69): dynamic vertex y vs static triangle x
-__device__ __forceinline__ bool project_vt_st(int vid, V3 x0, V3 x1, V3 x2, V3 x3, float wv, float dHat,
-                                              float compliance, long long* dx, int* nc, int* bad, V3 g[4],
-                                              int* dtype, float* schur_out) {
-    const int dt = d_type_PT(x0, x1, x2, x3);
-    *dtype = dt;
-    const float d = pt_distance(dt, x0, x1, x2, x3, g, true, dHat);
-    if (d < dHat) {
-        const float schur = wv * dot(g[0], g[0]);
-        const float ld = (compliance * (dHat - d)) / (compliance * schur + 1.0f);
-        acc_add(dx, nc, vid, wv * ld, g[0], bad);  // no `fixed` factor (collision_constraints_x.py:58)
-        *schur_out = schur;
-        return true;
+// The corrections of one candidate in contact.  mi: m_inv, w: the kind's weights.
+__device__ __forceinline__ void pair_apply(int kind, const int vv[4], const float mi[4], const float w[4],
+                                           const PairSolve& r, long long* dx, int* nc, int* bad) {
+    const int m = moved_mask(kind, r.dt);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        if (!(m & (1 << k))) continue;
+        // region 0 of VT_DY applies m_inv without `fixed` (collision_constraints_x.py:199-200)
+        acc_add(dx, nc, vv[k], (kind == VT_DY && r.dt == 0 ? mi[k] : w[k]) * r.ld, r.g[k], bad);
     }
-    return false;
 }
 
-// __vt_dy (collision_constraints_x.py:176-310): self contact, all four on y.
-// vt_dy_contact is the part after the region and distance are known.
-__device__ __forceinline__ float vt_dy_contact(int dt, float d, const int vv[4], const V3 x[4],
-                                               const float* __restrict__ fixed, const float* __restrict__ m_inv,
-                                               float dHat, long long* dx, int* nc, int* bad, V3 g[4]);
-
-__device__ __forceinline__ void project_vt_dy(const int vv[4], const V3 x[4], const float* __restrict__ fixed,
-                                              const float* __restrict__ m_inv, float dHat, long long* dx, int* nc,
-                                              int* bad, V3 g[4], int* dtype, float* schur_out) {
-    const int dt = d_type_PT(x[0], x[1], x[2], x[3]);
-    *dtype = dt;
-    const float d = pt_distance(dt, x[0], x[1], x[2], x[3], g, false, dHat);
-    *schur_out = vt_dy_contact(dt, d, vv, x, fixed, m_inv, dHat, dx, nc, bad, g);
+// Weights of a candidate: VT_ST has no `fixed` factor (collision_constraints_x.py:58);
+// vertices of the static mesh have none.
+__device__ __forceinline__ void pair_weights(int kind, const int vv[4], const float* __restrict__ fixed,
+                                             const float* __restrict__ m_inv, float mi[4], float w[4]) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const bool dyn = kind == VT_DY || (k == 0) == (kind == VT_ST);
+        mi[k] = dyn ? m_inv[vv[k]] : 0.0f;
+        w[k] = !dyn ? 0.0f : kind == VT_ST ? mi[k] : fixed[vv[k]] * mi[k];
+    }
 }
 
-__device__ __forceinline__ float vt_dy_contact(int dt, float d, const int vv[4], const V3 x[4],
-                                               const float* __restrict__ fixed, const float* __restrict__ m_inv,
-                                               float dHat, long long* dx, int* nc, int* bad, V3 g[4]) {
-    float schur = 0.0f;
-    if (d < dHat) {
-        pt_distance(dt, x[0], x[1], x[2], x[3], g, true, dHat);
-        const int m = region_mask(dt);
-        float s = 0.0f;
-        bool first = true;
-        for (int k = 0; k < 4; ++k) {
-            if (!(m & (1 << k))) continue;
-            const float t = (fixed[vv[k]] * m_inv[vv[k]]) * dot(g[k], g[k]);
-            s = first ? t : s + t;
-            first = false;
-        }
-        schur = s + 1e-4f;
-        const float ld = (dHat - d) / schur;
-        for (int k = 0; k < 4; ++k) {
-            if (!(m & (1 << k))) continue;
-            // region 0 applies m_inv without `fixed` (collision_constraints_x.py:199-200)
-            const float w = dt == 0 ? m_inv[vv[k]] : fixed[vv[k]] * m_inv[vv[k]];
-            acc_add(dx, nc, vv[k], w * ld, g[k], bad);
-        }
-    }
-    return schur;
+// The same candidate with the compiler's divisions, out of line: rare.
+__device__ __noinline__ int pair_project_ieee(int kind, int4 v, V3 x0, V3 x1, V3 x2, V3 x3,
+                                              const float* __restrict__ fixed, const float* __restrict__ m_inv,
+                                              float dHat, float compliance, long long* dx, int* nc) {
+    const int vv[4] = {v.x, v.y, v.z, v.w};
+    const V3 x[4] = {x0, x1, x2, x3};
+    float mi[4], w[4];
+    pair_weights(kind, vv, fixed, m_inv, mi, w);
+    PairSolve r;
+    int bad = 0;
+    pair_solve<true>(kind, x, w, dHat, compliance, r);
+    if (r.d < dHat) pair_apply(kind, vv, mi, w, r, dx, nc, &bad);
+    return bad;
 }
 
-// __tv_st (collision_constraints_x.py:72-173): static vertex x vs dynamic triangle y
-__device__ __forceinline__ void project_tv_st(const int vv[4], const V3 x[4], const float* __restrict__ fixed,
-                                              const float* __restrict__ m_inv, float dHat, float compliance,
-                                              long long* dx, int* nc, int* bad, V3 g[4], int* dtype,
-                                              float* schur_out) {
-    const int dt = d_type_PT(x[0], x[1], x[2], x[3]);
-    *dtype = dt;
-    const float d = pt_distance(dt, x[0], x[1], x[2], x[3], g, false, dHat);
-    float schur = 0.0f;
-    if (d < dHat) {
-        pt_distance(dt, x[0], x[1], x[2], x[3], g, true, dHat);
-        const int m = region_mask(dt) & ~1;
-        float s = 0.0f;
-        bool first = true;
-        for (int k = 1; k < 4; ++k) {
-            if (!(m & (1 << k))) continue;
-            const float t = (fixed[vv[k]] * m_inv[vv[k]]) * dot(g[k], g[k]);
-            s = first ? t : s + t;
-            first = false;
-        }
-        schur = s;
-        const float ld = (compliance * (dHat - d)) / (compliance * schur + 1.0f);
-        for (int k = 1; k < 4; ++k) {
-            if (!(m & (1 << k))) continue;
-            acc_add(dx, nc, vv[k], (fixed[vv[k]] * m_inv[vv[k]]) * ld, g[k], bad);
-        }
-    }
-    *schur_out = schur;
+// One candidate's corrections (__vt_st, __vt_dy or __tv_st); the weights are
+// loaded before the classification, which hides their latency.
+__device__ __forceinline__ void pair_project(int kind, int4 v, const V3 x[4], const float* __restrict__ fixed,
+                                             const float* __restrict__ m_inv, float dHat, float compliance,
+                                             long long* dx, int* nc, int* bad) {
+    const int vv[4] = {v.x, v.y, v.z, v.w};
+    float mi[4], w[4];
+    pair_weights(kind, vv, fixed, m_inv, mi, w);
+    PairSolve r;
+    if (!pair_solve<false>(kind, x, w, dHat, compliance, r))
+        *bad |= pair_project_ieee(kind, v, x[0], x[1], x[2], x[3], fixed, m_inv, dHat, compliance, dx, nc);
+    else if (r.d < dHat)
+        pair_apply(kind, vv, mi, w, r, dx, nc, bad);
+}
+
+// The same, for the walk that records its pairs: r also receives the region,
+// the gradients (zero where d >= dHat) and the schur complement.
+__device__ __forceinline__ void pair_project_recorded(int kind, const int vv[4], const V3 x[4],
+                                                      const float* __restrict__ fixed,
+                                                      const float* __restrict__ m_inv, float dHat, float compliance,
+                                                      long long* dx, int* nc, int* bad, PairSolve& r) {
+    float mi[4], w[4];
+    pair_weights(kind, vv, fixed, m_inv, mi, w);
+    for (int k = 0; k < 4; ++k) r.g[k] = V3{0.0f, 0.0f, 0.0f};
+    pair_solve<true>(kind, x, w, dHat, compliance, r);
+    if (r.d < dHat) pair_apply(kind, vv, mi, w, r, dx, nc, bad);
 }
 
 #define SX_ZERO_G {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}}
@@ -425,16 +505,15 @@ __global__ void __launch_bounds__(128) collision_project_kernel(
         const int vid = i;
         const int n = min(vt_st_n[vid], cap);
         const V3 x0 = mk(y4[vid]);
-        const float wv = m_inv[vid];
         for (int j = 0; j < n; ++j) {
             const int fs = vt_st_c[(size_t)vid * cap + j];
             const V3 x1 = mk(xs4[faces_st[3 * fs]]), x2 = mk(xs4[faces_st[3 * fs + 1]]),
                      x3 = mk(xs4[faces_st[3 * fs + 2]]);
-            V3 g[4] = SX_ZERO_G;
-            int dt;
-            float schur;
-            if (project_vt_st(vid, x0, x1, x2, x3, wv, dHat, compliance, dx, nc, &bad, g, &dt, &schur))
-                po.rec((size_t)vid, cnt, fs, dt, g, schur);
+            const int vv[4] = {vid, -1, -1, -1};
+            const V3 x[4] = {x0, x1, x2, x3};
+            PairSolve r;
+            pair_project_recorded(VT_ST, vv, x, fixed, m_inv, dHat, compliance, dx, nc, &bad, r);
+            if (r.d < dHat) po.rec((size_t)vid, cnt, fs, r.dt, r.g, r.schur);
         }
         if (po.num) po.num[vid] = cnt;
     } else if (i < 2 * Vd) {
@@ -446,11 +525,9 @@ __global__ void __launch_bounds__(128) collision_project_kernel(
             if (a == vid || b == vid || c == vid) continue;  // Solver.is_in_face, XPBD.py:121-127
             const int vv[4] = {vid, a, b, c};
             const V3 x[4] = {mk(y4[vid]), mk(y4[a]), mk(y4[b]), mk(y4[c])};
-            V3 g[4] = SX_ZERO_G;
-            int dt;
-            float schur;
-            project_vt_dy(vv, x, fixed, m_inv, dHat, dx, nc, &bad, g, &dt, &schur);
-            po.rec((size_t)Vd + vid, cnt, fd, dt, g, schur);
+            PairSolve r;
+            pair_project_recorded(VT_DY, vv, x, fixed, m_inv, dHat, compliance, dx, nc, &bad, r);
+            po.rec((size_t)Vd + vid, cnt, fd, r.dt, r.g, r.schur);
         }
         if (po.num) po.num[Vd + vid] = cnt;
     } else {
@@ -460,11 +537,9 @@ __global__ void __launch_bounds__(128) collision_project_kernel(
             const int fd = tv_st_c[(size_t)vis * cap + j];
             const int vv[4] = {-1, faces_dy[3 * fd], faces_dy[3 * fd + 1], faces_dy[3 * fd + 2]};
             const V3 x[4] = {mk(xs4[vis]), mk(y4[vv[1]]), mk(y4[vv[2]]), mk(y4[vv[3]])};
-            V3 g[4] = SX_ZERO_G;
-            int dt;
-            float schur;
-            project_tv_st(vv, x, fixed, m_inv, dHat, compliance, dx, nc, &bad, g, &dt, &schur);
-            po.rec((size_t)2 * Vd + vis, cnt, fd, dt, g, schur);
+            PairSolve r;
+            pair_project_recorded(TV_ST, vv, x, fixed, m_inv, dHat, compliance, dx, nc, &bad, r);
+            po.rec((size_t)2 * Vd + vis, cnt, fd, r.dt, r.g, r.schur);
         }
         if (po.num) po.num[2 * Vd + vis] = cnt;
     }
@@ -698,29 +773,6 @@ __device__ __forceinline__ void pair_points(const PairCtx& c, int t, int4 pr, V3
     x[3] = mk(tri[pr.w]);
 }
 
-__device__ __forceinline__ void project_pair_x(const PairCtx& c, int t, int4 pr, const V3 x[4], int* bad) {
-    V3 g[4] = SX_ZERO_G;
-    int dt;
-    float schur;
-    if (t < c.st_end) {
-        project_vt_st(pr.x, x[0], x[1], x[2], x[3], c.m_inv[pr.x], c.dHat, c.compliance, c.dx, c.nc, bad, g, &dt,
-                      &schur);
-    } else if (t < c.dy_end) {
-        const int vv[4] = {pr.x, pr.y, pr.z, pr.w};
-        project_vt_dy(vv, x, c.fixed, c.m_inv, c.dHat, c.dx, c.nc, bad, g, &dt, &schur);
-    } else {
-        const int vv[4] = {-1, pr.y, pr.z, pr.w};
-        project_tv_st(vv, x, c.fixed, c.m_inv, c.dHat, c.compliance, c.dx, c.nc, bad, g, &dt, &schur);
-    }
-}
-
-__device__ __forceinline__ void project_pair(const PairCtx& c, int t, int* bad) {
-    const int4 pr = c.pairs[t];
-    V3 x[4];
-    pair_points(c, t, pr, x);
-    project_pair_x(c, t, pr, x, bad);
-}
-
 constexpr int PP_BLOCK = 256;
 
 // With the cull on, most pairs end at the box test, most of the rest at the
@@ -730,9 +782,19 @@ constexpr int PP_BLOCK = 256;
 // U batches of loads are in flight) and appends the survivors to a stack in
 // shared memory (ballot); 32 at a time they go through the separating-axis
 // test onto a second stack, and 32 at a time from there through the
-// projection, every stage with all lanes busy.  The contact sums are order
-// independent, so U and the stacking change the speed only.
-template <int U, int MINB>
+// projection, every stage with all lanes busy.  The projection stands in one
+// place of the loop, which keeps the kernel's code and registers small.  The
+// contact sums are order independent, so U and the stacking change the speed
+// only.
+//
+// PIPE: the two kinds against the obstacle (vertex vs obstacle face, obstacle
+// vertex vs cloth face) are few pairs of which most reach the classification;
+// the last warps take them one per lane from the box test straight to the
+// projection, on the positions already in registers.  The vertex-vs-cloth pairs then go through the stages
+// above, with the next step's pair records loaded while the current step's
+// positions are gathered, so that a warp waits on one round trip per step
+// instead of two.
+template <int U, int MINB, bool PIPE>
 __global__ void __launch_bounds__(PP_BLOCK, MINB) pairs_project_kernel(const int* __restrict__ meta,
                                                                        const int4* __restrict__ pairs,
                                                                        const float4* __restrict__ y4,
@@ -745,179 +807,114 @@ __global__ void __launch_bounds__(PP_BLOCK, MINB) pairs_project_kernel(const int
     pdl_entry();
     if (iteration_skipped(conv, iter)) return;
     const PairCtx c{pairs, y4, xs4, fixed, m_inv, dHat, compliance, dx, nc, meta[0], meta[1]};
-    const int P = meta[2];
-    int bad = 0;
-    if (!(cull_d2 > 0.0f)) {
-        for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < P; t += gridDim.x * blockDim.x)
-            project_pair(c, t, &bad);
-    } else {
-        __shared__ int box_stack[PP_BLOCK / 32][32 * U + 32];
-        __shared__ int sat_stack[PP_BLOCK / 32][64];
-        const int lane = threadIdx.x & 31;
-        const unsigned below = (1u << lane) - 1u;
-        int* s1 = box_stack[threadIdx.x >> 5];
-        int* s2 = sat_stack[threadIdx.x >> 5];
-        int n1 = 0, n2 = 0;  // warp-uniform
-        // the top cnt (<= 32) entries of s1 through the separating-axis test
-        // onto s2; projects the top 32 of s2 once it holds that many
-        auto sat_stage = [&](int cnt) {
-            const int t = lane < cnt ? s1[n1 - cnt + lane] : -1;
-            bool keep = false;
-            if (t >= 0) {
-                V3 x[4];
-                pair_points(c, t, pairs[t], x);
-                keep = !sat_far(x[0], x[1], x[2], x[3], cull_d2);
-            }
-            n1 -= cnt;
-            const unsigned m = __ballot_sync(0xffffffffu, keep);
-            if (keep) s2[n2 + __popc(m & below)] = t;
-            n2 += __popc(m);
-            __syncwarp();
-            if (n2 >= 32) {
-                project_pair(c, s2[n2 - 32 + lane], &bad);
-                n2 -= 32;
-                __syncwarp();
-            }
-        };
-        const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
-        for (int base = gw * 32 * U; base < P; base += nw * 32 * U) {
-            int4 pr[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int t = base + 32 * u + lane;
-                pr[u] = t < P ? pairs[t] : make_int4(0, 0, 0, 0);
-            }
-            V3 x[U][4];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int t = base + 32 * u + lane;
-                if (t < P) pair_points(c, t, pr[u], x[u]);
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int t = base + 32 * u + lane;
-                const bool keep = t < P && !box_far(x[u][0], x[u][1], x[u][2], x[u][3], cull_d2);
-                const unsigned m = __ballot_sync(0xffffffffu, keep);
-                if (keep) s1[n1 + __popc(m & below)] = t;
-                n1 += __popc(m);
-            }
-            __syncwarp();
-            while (n1 >= 32) sat_stage(32);
-        }
-        if (n1 > 0) sat_stage(n1);
-        if (lane < n2) project_pair(c, s2[lane], &bad);
-    }
-    if (bad) atomicOr(status, SX_STATUS_FIXED_RANGE);
-}
-
-// Pipelined form of pairs_project_kernel (same sums).  The two kinds against
-// the obstacle (vertex vs obstacle face, obstacle vertex vs cloth face) are
-// few pairs of which most reach the classification; the first warps take them
-// one per lane and run box test, separating-axis test and projection on the
-// positions already in registers, without re-loading them through the
-// stacks.  The vertex-vs-cloth pairs then go through the stacked stages as in
-// pairs_project_kernel, with the next step's pair records loaded while the
-// current step's positions are gathered, so that a warp waits on one round
-// trip per step instead of two.
-template <int U, int MINB>
-__global__ void __launch_bounds__(PP_BLOCK, MINB) pairs_project_pipe_kernel(const int* __restrict__ meta,
-                                                                            const int4* __restrict__ pairs,
-                                                                            const float4* __restrict__ y4,
-                                                                            const float4* __restrict__ xs4,
-                                                                            const float* __restrict__ fixed,
-                                                                            const float* __restrict__ m_inv,
-                                                                            float dHat, float compliance,
-                                                                            float cull_d2, long long* dx, int* nc,
-                                                                            int* status, const int* conv, int iter) {
-    pdl_entry();
-    if (iteration_skipped(conv, iter)) return;
-    const PairCtx c{pairs, y4, xs4, fixed, m_inv, dHat, compliance, dx, nc, meta[0], meta[1]};
     const int P = meta[2], st_end = c.st_end, dy_end = c.dy_end;
-    const int lane = threadIdx.x & 31;
-    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
-    int bad = 0;
-    if (!(cull_d2 > 0.0f)) {  // no cull: every pair is classified
-        for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < P; t += gridDim.x * blockDim.x)
-            project_pair(c, t, &bad);
-        if (bad) atomicOr(status, SX_STATUS_FIXED_RANGE);
-        return;
-    }
-    // the obstacle kinds, one pair per lane
-    const int H = st_end + (P - dy_end);
-    for (int h0 = gw * 32; h0 < H; h0 += nw * 32) {
-        const int h = h0 + lane;
-        if (h < H) {
-            const int t = h < st_end ? h : dy_end + (h - st_end);
-            const int4 pr = pairs[t];
-            V3 x[4];
-            pair_points(c, t, pr, x);
-            if (!box_far(x[0], x[1], x[2], x[3], cull_d2) && !sat_far(x[0], x[1], x[2], x[3], cull_d2))
-                project_pair_x(c, t, pr, x, &bad);
-        }
-    }
-    // the vertex-vs-cloth pairs [st_end, dy_end)
+    const bool cull = cull_d2 > 0.0f;  // without it every pair is classified
     __shared__ int box_stack[PP_BLOCK / 32][32 * U + 32];
     __shared__ int sat_stack[PP_BLOCK / 32][64];
+    const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
     int* s1 = box_stack[threadIdx.x >> 5];
     int* s2 = sat_stack[threadIdx.x >> 5];
     int n1 = 0, n2 = 0;  // warp-uniform
-    auto sat_stage = [&](int cnt) {
-        const int t = lane < cnt ? s1[n1 - cnt + lane] : -1;
-        bool keep = false;
-        if (t >= 0) {
-            V3 x[4];
-            pair_points(c, t, pairs[t], x);
-            keep = !sat_far(x[0], x[1], x[2], x[3], cull_d2);
-        }
-        n1 -= cnt;
+    int bad = 0;
+    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+    const bool split = PIPE && cull;
+    const int first = split ? st_end : 0, last = split ? dy_end : P, chunk = cull ? 32 * U : 32;
+    // the obstacle kinds go to the last warps, which have the fewest chunks
+    const int H = split ? st_end + (P - dy_end) : 0;
+    int h0 = (nw - 1 - gw) * 32, base = first + gw * chunk;
+    auto push = [&](int* s, int& n, int t, bool keep) {
         const unsigned m = __ballot_sync(0xffffffffu, keep);
-        if (keep) s2[n2 + __popc(m & below)] = t;
-        n2 += __popc(m);
-        __syncwarp();
-        if (n2 >= 32) {
-            project_pair(c, s2[n2 - 32 + lane], &bad);
-            n2 -= 32;
-            __syncwarp();
-        }
+        if (keep) s[n + __popc(m & below)] = t;
+        n += __popc(m);
     };
-    const int step = nw * 32 * U, first = st_end + gw * 32 * U, last = dy_end;
     int4 nx[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-        const int t = first + 32 * u + lane;
-        nx[u] = t < last ? pairs[t] : make_int4(0, 0, 0, 0);
-    }
-    for (int base = first; base < last; base += step) {
-        V3 x[U][4];
+    if (split) {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const int t = base + 32 * u + lane;
-            if (t < last) {
-                x[u][0] = mk(y4[nx[u].x]);
-                x[u][1] = mk(y4[nx[u].y]);
-                x[u][2] = mk(y4[nx[u].z]);
-                x[u][3] = mk(y4[nx[u].w]);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int t = base + step + 32 * u + lane;
             nx[u] = t < last ? pairs[t] : make_int4(0, 0, 0, 0);
         }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int t = base + 32 * u + lane;
-            const bool keep = t < last && !box_far(x[u][0], x[u][1], x[u][2], x[u][3], cull_d2);
-            const unsigned m = __ballot_sync(0xffffffffu, keep);
-            if (keep) s1[n1 + __popc(m & below)] = t;
-            n1 += __popc(m);
-        }
-        __syncwarp();
-        while (n1 >= 32) sat_stage(32);
     }
-    if (n1 > 0) sat_stage(n1);
-    if (lane < n2) project_pair(c, s2[lane], &bad);
+    for (;;) {
+        int t = -1;  // the pair this lane projects
+        int4 pr = make_int4(0, 0, 0, 0);
+        V3 x[4];
+        if (h0 < H) {
+            const int h = h0 + lane;
+            if (h < H) {
+                t = h < st_end ? h : dy_end + (h - st_end);
+                pr = pairs[t];
+                pair_points(c, t, pr, x);
+                if (box_far(x[0], x[1], x[2], x[3], cull_d2)) t = -1;
+            }
+            h0 += nw * 32;
+        } else {
+            // fill the second stack to at least 32 entries, or to what is left
+            bool more = true;
+            while (n2 < 32 && more) {
+                if (n1 >= 32 || (n1 > 0 && base >= last)) {
+                    // the top of s1 through the separating-axis test onto s2
+                    const int cnt = n1 < 32 ? n1 : 32;
+                    const int q = lane < cnt ? s1[n1 - cnt + lane] : -1;
+                    bool keep = false;
+                    if (q >= 0) {
+                        V3 z[4];
+                        pair_points(c, q, pairs[q], z);
+                        keep = !sat_far(z[0], z[1], z[2], z[3], cull_d2);
+                    }
+                    n1 -= cnt;
+                    push(s2, n2, q, keep);
+                } else if (base < last) {
+                    if (!cull) {
+                        push(s2, n2, base + lane, base + lane < last);
+                    } else {
+                        V3 z[U][4];
+#pragma unroll
+                        for (int u = 0; u < U; ++u) {
+                            const int q = base + 32 * u + lane;
+                            if (PIPE) {
+                                z[u][0] = mk(y4[nx[u].x]);
+                                z[u][1] = mk(y4[nx[u].y]);
+                                z[u][2] = mk(y4[nx[u].z]);
+                                z[u][3] = mk(y4[nx[u].w]);
+                            } else if (q < last) {
+                                pair_points(c, q, pairs[q], z[u]);
+                            }
+                        }
+                        if (PIPE) {
+#pragma unroll
+                            for (int u = 0; u < U; ++u) {
+                                const int q = base + nw * chunk + 32 * u + lane;
+                                nx[u] = q < last ? pairs[q] : make_int4(0, 0, 0, 0);
+                            }
+                        }
+#pragma unroll
+                        for (int u = 0; u < U; ++u) {
+                            const int q = base + 32 * u + lane;
+                            push(s1, n1, q, q < last && !box_far(z[u][0], z[u][1], z[u][2], z[u][3], cull_d2));
+                        }
+                    }
+                    base += nw * chunk;
+                } else {
+                    more = false;
+                }
+                __syncwarp();
+            }
+            if (n2 == 0) break;
+            const int cnt = n2 < 32 ? n2 : 32;
+            if (lane < cnt) {
+                t = s2[n2 - cnt + lane];
+                pr = pairs[t];
+                pair_points(c, t, pr, x);
+            }
+            n2 -= cnt;
+            __syncwarp();
+        }
+        if (t >= 0)
+            pair_project(t < st_end ? VT_ST : t < dy_end ? VT_DY : TV_ST, pr, x, fixed, m_inv, dHat, compliance, dx,
+                         nc, &bad);
+    }
     if (bad) atomicOr(status, SX_STATUS_FIXED_RANGE);
 }
 
@@ -1091,16 +1088,13 @@ __global__ void __launch_bounds__(256) batched_contacts_kernel(
         if (m) {
             const int f0 = ob_fptr[vinst[i]];
             const V3 x0 = mk(y4[i]);
-            const float wv = m_inv[i];
             while (m) {
                 const int k = __ffs(m) - 1;
                 m &= m - 1;
                 const int f = f0 + k;
-                V3 g[4] = SX_ZERO_G;
-                int dt;
-                float schur;
-                project_vt_st(i, x0, mk(xs4[ob_faces[3 * f]]), mk(xs4[ob_faces[3 * f + 1]]),
-                              mk(xs4[ob_faces[3 * f + 2]]), wv, dHat, compliance, dx, nc, &bad, g, &dt, &schur);
+                const V3 x[4] = {x0, mk(xs4[ob_faces[3 * f]]), mk(xs4[ob_faces[3 * f + 1]]),
+                                 mk(xs4[ob_faces[3 * f + 2]])};
+                pair_project(VT_ST, make_int4(i, -1, -1, -1), x, fixed, m_inv, dHat, compliance, dx, nc, &bad);
             }
         }
     } else if (i < V + S) {  // __tv_st: obstacle vertex vs its cloth's faces
@@ -1108,12 +1102,9 @@ __global__ void __launch_bounds__(256) batched_contacts_kernel(
         const int n = min(tv_num[s], cap);
         for (int j = 0; j < n; ++j) {
             const int fd = tv_cand[(size_t)s * cap + j];
-            const int vv[4] = {-1, cl_faces[3 * fd], cl_faces[3 * fd + 1], cl_faces[3 * fd + 2]};
-            const V3 x[4] = {mk(xs4[s]), mk(y4[vv[1]]), mk(y4[vv[2]]), mk(y4[vv[3]])};
-            V3 g[4] = SX_ZERO_G;
-            int dt;
-            float schur;
-            project_tv_st(vv, x, fixed, m_inv, dHat, compliance, dx, nc, &bad, g, &dt, &schur);
+            const int4 vv = make_int4(-1, cl_faces[3 * fd], cl_faces[3 * fd + 1], cl_faces[3 * fd + 2]);
+            const V3 x[4] = {mk(xs4[s]), mk(y4[vv.y]), mk(y4[vv.z]), mk(y4[vv.w])};
+            pair_project(TV_ST, vv, x, fixed, m_inv, dHat, compliance, dx, nc, &bad);
         }
     }
     }
@@ -1130,8 +1121,8 @@ __global__ void __launch_bounds__(256) batched_contacts_kernel(
 // so no grid-wide synchronisation is needed.  The instance's positions and
 // adjacency stay in L1/L2 across its iterations instead of streaming the
 // whole batch from HBM in every sweep.  Every phase evaluates the same
-// expressions as the grid-wide kernels (sweep_vertex, project_vt_st /
-// project_tv_st, the broad-phase tests, update_dx, compute_velocity +
+// expressions as the grid-wide kernels (sweep_vertex, pair_project,
+// the broad-phase tests, update_dx, compute_velocity +
 // update_x), and contact sums are order independent, so the result equals the
 // graph of grid-wide launches bit for bit.  Chunk boxes (32 faces) are
 // aligned to each instance's first face (cptr); they only select which faces
@@ -1366,17 +1357,14 @@ __global__ void __launch_bounds__(BLOCK, MINB) batched_substep_kernel(BatchedSub
                     if (m) {
                         const int of0 = A.ob_fptr[i];
                         const V3 x0 = mk(yout[v]);
-                        const float wv = A.m_inv[v];
                         while (m) {
                             const int kk = __ffs(m) - 1;
                             m &= m - 1;
                             const int f = of0 + kk;
-                            V3 g[4] = SX_ZERO_G;
-                            int dt_;
-                            float schur;
-                            project_vt_st(v, x0, mk(A.xs4[A.ob_faces[3 * f]]), mk(A.xs4[A.ob_faces[3 * f + 1]]),
-                                          mk(A.xs4[A.ob_faces[3 * f + 2]]), wv, A.dHat, A.compliance, A.dx, A.nc,
-                                          &bad, g, &dt_, &schur);
+                            const V3 x[4] = {x0, mk(A.xs4[A.ob_faces[3 * f]]), mk(A.xs4[A.ob_faces[3 * f + 1]]),
+                                             mk(A.xs4[A.ob_faces[3 * f + 2]])};
+                            pair_project(VT_ST, make_int4(v, -1, -1, -1), x, A.fixed, A.m_inv, A.dHat, A.compliance,
+                                         A.dx, A.nc, &bad);
                         }
                     }
                 } else {
@@ -1384,13 +1372,9 @@ __global__ void __launch_bounds__(BLOCK, MINB) batched_substep_kernel(BatchedSub
                     const int n = min(A.tv_num[s], A.cap);
                     for (int j = 0; j < n; ++j) {
                         const int fd = A.tv_cand[(size_t)s * A.cap + j];
-                        const int vv[4] = {-1, A.faces[3 * fd], A.faces[3 * fd + 1], A.faces[3 * fd + 2]};
-                        const V3 x[4] = {mk(A.xs4[s]), mk(yout[vv[1]]), mk(yout[vv[2]]), mk(yout[vv[3]])};
-                        V3 g[4] = SX_ZERO_G;
-                        int dt_;
-                        float schur;
-                        project_tv_st(vv, x, A.fixed, A.m_inv, A.dHat, A.compliance, A.dx, A.nc, &bad, g, &dt_,
-                                      &schur);
+                        const int4 vv = make_int4(-1, A.faces[3 * fd], A.faces[3 * fd + 1], A.faces[3 * fd + 2]);
+                        const V3 x[4] = {mk(A.xs4[s]), mk(yout[vv.y]), mk(yout[vv.z]), mk(yout[vv.w])};
+                        pair_project(TV_ST, vv, x, A.fixed, A.m_inv, A.dHat, A.compliance, A.dx, A.nc, &bad);
                     }
                 }
             }
@@ -1827,25 +1811,24 @@ static int sm_count() {
 // Launch configurations of the pair projection: pair batches box-tested per
 // warp step (U) and resident blocks per SM (the grid is that many blocks per
 // SM; registers are capped to keep them resident).  All give identical
-// results.  The default (the pipelined form, one pair batch per warp step, 4
-// blocks per SM) was the fastest inside the drape256 frame; timed alone on a
-// fixed state the ranking differs, so Solver.autotune_contacts times whole
-// frames.
+// results.  The default is the pipelined form with two pair batches per warp
+// step and 3 blocks per SM (80 registers; at 64 the projection spills): us per
+// launch for it / pipelined 1 x 4 / stacked 2 x 3 on the 64 x 64 box scene (63 K
+// pairs) 4.7 / 5.4 / 6.3, a 181 x 139 sphere drape (74 K) 5.5 / 6.1 / 9.1, a 256
+// x 256 one (1.43 M) 13.7 / 14.0 / 19.3.  With three copies of a branching
+// narrow phase and FP64 fixed point the same launches took 7.8 / 9.8 / 19.0.
 struct PairsProjectVariant {
     int unroll, blocks_per_sm, pipelined;
-    decltype(&pairs_project_kernel<1, 4>) kern;
+    decltype(&pairs_project_kernel<1, 4, false>) kern;
 };
 static const PairsProjectVariant kPairsProjectVariants[] = {
-    {2, 3, 0, pairs_project_kernel<2, 3>},
-    {1, 4, 0, pairs_project_kernel<1, 4>},
-    {2, 6, 0, pairs_project_kernel<2, 3>},
-    {4, 2, 0, pairs_project_kernel<4, 2>},
-    {2, 3, 1, pairs_project_pipe_kernel<2, 3>},
-    {1, 4, 1, pairs_project_pipe_kernel<1, 4>},
-    {2, 4, 1, pairs_project_pipe_kernel<2, 4>},
+    {2, 3, 0, pairs_project_kernel<2, 3, false>}, {1, 4, 0, pairs_project_kernel<1, 4, false>},
+    {2, 6, 0, pairs_project_kernel<2, 3, false>}, {4, 2, 0, pairs_project_kernel<4, 2, false>},
+    {2, 3, 1, pairs_project_kernel<2, 3, true>},  {1, 4, 1, pairs_project_kernel<1, 4, true>},
+    {2, 4, 1, pairs_project_kernel<2, 4, true>},
 };
 constexpr int kNumPairsProjectVariants = sizeof(kPairsProjectVariants) / sizeof(kPairsProjectVariants[0]);
-constexpr int kPairsProjectDefault = 5;
+constexpr int kPairsProjectDefault = 4;
 
 extern "C" int sx_contact_pairs_project_variants(void) { return kNumPairsProjectVariants; }
 
