@@ -919,24 +919,42 @@ __global__ void __launch_bounds__(PP_BLOCK, MINB) pairs_project_kernel(const int
 }
 
 // update_dx (XPBD.py:384-387) from the fixed-point accumulators; clears them.
+// Few vertices have a correction: the kernel is bound by reading every count,
+// so a thread reads N of them with one load (N = 4 where nc is 16-byte aligned).
+template <int N>
 __global__ void collision_apply_kernel(int V, float4* __restrict__ y4, const float* __restrict__ fixed,
                                        long long* __restrict__ dx, int* __restrict__ nc, const int* conv, int iter) {
     pdl_entry();
     if (iteration_skipped(conv, iter)) return;
-    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
-        const int c = nc[v];
-        if (c > 0) {
-            const float cf = (float)c;
-            const float f = fixed[v];
-            float4 y = y4[v];
-            y.x = y.x + f * (from_fix(dx[3 * v]) / cf);
-            y.y = y.y + f * (from_fix(dx[3 * v + 1]) / cf);
-            y.z = y.z + f * (from_fix(dx[3 * v + 2]) / cf);
-            y4[v] = y;
-            dx[3 * v] = 0;
-            dx[3 * v + 1] = 0;
-            dx[3 * v + 2] = 0;
-            nc[v] = 0;
+    const long long stride = (long long)gridDim.x * blockDim.x * N;
+    for (long long v0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * N; v0 < V; v0 += stride) {
+        int c[N];
+        if (N == 4 && v0 + 4 <= V) {
+            const int4 q = *reinterpret_cast<const int4*>(nc + v0);
+            c[0] = q.x;
+            c[N > 1 ? 1 : 0] = q.y;
+            c[N > 2 ? 2 : 0] = q.z;
+            c[N > 3 ? 3 : 0] = q.w;
+        } else {
+#pragma unroll
+            for (int j = 0; j < N; ++j) c[j] = v0 + j < V ? nc[v0 + j] : 0;
+        }
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            if (c[j] > 0) {
+                const long long v = v0 + j;
+                const float cf = (float)c[j];
+                const float f = fixed[v];
+                float4 y = y4[v];
+                y.x = y.x + f * (from_fix(dx[3 * v]) / cf);
+                y.y = y.y + f * (from_fix(dx[3 * v + 1]) / cf);
+                y.z = y.z + f * (from_fix(dx[3 * v + 2]) / cf);
+                y4[v] = y;
+                dx[3 * v] = 0;
+                dx[3 * v + 1] = 0;
+                dx[3 * v + 2] = 0;
+                nc[v] = 0;
+            }
         }
     }
 }
@@ -946,6 +964,17 @@ template <typename K>
 inline int capped_grid(K kernel, long long n, int block) {
     const int g = grid_for(n, block), cap = resident_blocks(kernel, block);
     return g < cap ? g : cap;
+}
+
+// collision_apply_kernel: four vertices a thread once one a thread is more
+// than one resident wave (600 000 vertices 8.4 us in three waves of one-vertex
+// threads)
+static void launch_apply(int V, float4* y4, const float* fixed, long long* dx, int* nc, const int* conv, int iter,
+                         cudaStream_t s) {
+    const bool wide = V > 262144 && ((uintptr_t)nc & 15) == 0;
+    const auto k = wide ? collision_apply_kernel<4> : collision_apply_kernel<1>;
+    const long long n = wide ? (V + 3LL) / 4 : V;
+    launch(k, conv ? capped_grid(k, n, 256) : grid_for(n, 256), 256, 0, s, V, y4, fixed, dx, nc, conv, iter);
 }
 
 // ---------------------------------------------------------------------------
@@ -973,23 +1002,39 @@ __device__ __forceinline__ float ord2f_c(unsigned u) {
 }
 
 // AABB of each segment of a point array (one block per segment), +- padding,
-// with the reference's 1e5 initial bounds (meshTaichiWrapper.py:335-347).
-__global__ void __launch_bounds__(256) segment_aabb_kernel(const float4* __restrict__ p4, const int* __restrict__ seg,
-                                                           float pad, float* __restrict__ box6) {
+// with the reference's 1e5 initial bounds (meshTaichiWrapper.py:335-347).  A
+// block reads a segment of some 10 000 points alone, so it is bound by the
+// round trips of its loads: 1024 threads with four in flight each (24 cloths of
+// up to 128 x 128: 34 us with 256 threads, one load each).
+constexpr int SEG_BLOCK = 1024;
+__global__ void __launch_bounds__(SEG_BLOCK) segment_aabb_kernel(const float4* __restrict__ p4,
+                                                                 const int* __restrict__ seg, float pad,
+                                                                 float* __restrict__ box6) {
     pdl_entry();
     const int s = blockIdx.x;
     float lo[3] = {1e5f, 1e5f, 1e5f}, hi[3] = {-1e5f, -1e5f, -1e5f};
-    for (int i = seg[s] + threadIdx.x; i < seg[s + 1]; i += blockDim.x) {
-        const float4 p = p4[i];
-        lo[0] = fminf(lo[0], p.x); lo[1] = fminf(lo[1], p.y); lo[2] = fminf(lo[2], p.z);
-        hi[0] = fmaxf(hi[0], p.x); hi[1] = fmaxf(hi[1], p.y); hi[2] = fmaxf(hi[2], p.z);
+    const int e = seg[s + 1];
+    for (int i = seg[s] + threadIdx.x; i < e; i += 4 * SEG_BLOCK) {
+        float4 p[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) p[j] = i + j * SEG_BLOCK < e ? p4[i + j * SEG_BLOCK] : make_float4(NAN, NAN, NAN, 0.0f);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {  // fminf and fmaxf pass over a NaN
+            lo[0] = fminf(lo[0], p[j].x); lo[1] = fminf(lo[1], p[j].y); lo[2] = fminf(lo[2], p[j].z);
+            hi[0] = fmaxf(hi[0], p[j].x); hi[1] = fmaxf(hi[1], p[j].y); hi[2] = fmaxf(hi[2], p[j].z);
+        }
     }
     __shared__ unsigned red[6];
     if (threadIdx.x < 6) red[threadIdx.x] = threadIdx.x < 3 ? f2ord_c(1e5f) : f2ord_c(-1e5f);
     __syncthreads();
+#pragma unroll
     for (int k = 0; k < 3; ++k) {
-        atomicMin(red + k, f2ord_c(lo[k]));
-        atomicMax(red + 3 + k, f2ord_c(hi[k]));
+        const unsigned l = __reduce_min_sync(0xffffffffu, f2ord_c(lo[k]));
+        const unsigned h = __reduce_max_sync(0xffffffffu, f2ord_c(hi[k]));
+        if ((threadIdx.x & 31) == 0) {
+            atomicMin(red + k, l);
+            atomicMax(red + 3 + k, h);
+        }
     }
     __syncthreads();
     if (threadIdx.x < 6) {
@@ -1051,19 +1096,31 @@ __global__ void batched_tv_st_broad_kernel(int S, const float4* __restrict__ xs4
     if (!query_skipped(a, b, cl_box6 + 6 * inst)) {
         const int f0 = cl_fptr[inst], f1 = cl_fptr[inst + 1];
         const int c0 = f0 >> 5, c1 = (f1 + 31) >> 5;  // chunks touching [f0, f1)
-        for (int cb = c0; cb < c1; cb += 32) {
-            const int c = cb + lane;
-            const bool near = c < c1 && overlap(a, b, mk(cl_cmin4[c]), mk(cl_cmax4[c]));
-            unsigned hits = __ballot_sync(0xffffffffu, near);
-            while (hits) {  // warp-uniform, ascending chunks
-                const int ch = cb + __ffs(hits) - 1;
-                hits &= hits - 1u;
-                const int f = 32 * ch + lane;
-                const bool hit = f >= f0 && f < f1 && overlap(a, b, mk(cl_fmin4[f]), mk(cl_fmax4[f]));
-                const unsigned ball = __ballot_sync(0xffffffffu, hit);
-                const int slot = count + __popc(ball & ((1u << lane) - 1u));
-                if (hit && slot < cap) cand[(size_t)w * cap + slot] = f;
-                count += __popc(ball);
+        // four batches of chunk boxes in flight: a warp alone reads its cloth's
+        constexpr int N = 4;
+        for (int cb0 = c0; cb0 < c1; cb0 += 32 * N) {
+            float4 lo[N], hi[N];
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                const int c = cb0 + 32 * i + lane;
+                lo[i] = c < c1 ? cl_cmin4[c] : make_float4(INFINITY, INFINITY, INFINITY, 0.0f);
+                hi[i] = c < c1 ? cl_cmax4[c] : make_float4(-INFINITY, -INFINITY, -INFINITY, 0.0f);
+            }
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                const int cb = cb0 + 32 * i;
+                const bool near = cb + lane < c1 && overlap(a, b, mk(lo[i]), mk(hi[i]));
+                unsigned hits = __ballot_sync(0xffffffffu, near);
+                while (hits) {  // warp-uniform, ascending chunks
+                    const int ch = cb + __ffs(hits) - 1;
+                    hits &= hits - 1u;
+                    const int f = 32 * ch + lane;
+                    const bool hit = f >= f0 && f < f1 && overlap(a, b, mk(cl_fmin4[f]), mk(cl_fmax4[f]));
+                    const unsigned ball = __ballot_sync(0xffffffffu, hit);
+                    const int slot = count + __popc(ball & ((1u << lane) - 1u));
+                    if (hit && slot < cap) cand[(size_t)w * cap + slot] = f;
+                    count += __popc(ball);
+                }
             }
         }
     }
@@ -1073,7 +1130,20 @@ __global__ void batched_tv_st_broad_kernel(int S, const float4* __restrict__ xs4
     }
 }
 
-__global__ void __launch_bounds__(256) batched_contacts_kernel(
+// Obstacle contacts of one iteration.  A candidate is an (obstacle vertex,
+// cloth face) slot or a set bit of a cloth vertex's face mask; few vertices have
+// any, and a corner of an obstacle under a lying cloth has as many as its list
+// holds.  One thread per vertex would walk such a list alone (40 dependent
+// classifications: 99 us per launch on 24 cloths lying on their boxes, 160 000
+// vertices); here each warp lays the candidates of its tasks end to end, tests
+// them 32 at a time with the pair list's culls (box_far, sat_far: of a box
+// side's two triangles most vertices reach one) and projects the survivors 32
+// at a time.  Tasks are 32 slots of the obstacle vertices' lists, then 32 cloth
+// vertices, dealt to the warps in turn; a warp loads the masks of four tasks
+// together.  Contact sums are order independent.
+constexpr int BC_BLOCK = 256, BC_PER_SM = 2;
+
+__global__ void __launch_bounds__(BC_BLOCK, BC_PER_SM) batched_contacts_kernel(
     int V, int S, const float4* __restrict__ y4, const float* __restrict__ fixed, const float* __restrict__ m_inv,
     const int* __restrict__ vinst, const int* __restrict__ ob_fptr, const int* __restrict__ ob_faces,
     const float4* __restrict__ xs4, const unsigned* __restrict__ vmask, const int* __restrict__ tv_cand,
@@ -1081,32 +1151,114 @@ __global__ void __launch_bounds__(256) batched_contacts_kernel(
     long long* dx, int* nc, int* status, const int* conv, int iter) {
     pdl_entry();
     if (iteration_skipped(conv, iter)) return;
-    int bad = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < V + S; i += gridDim.x * blockDim.x) {
-    if (i < V) {  // __vt_st: cloth vertex vs its obstacle's faces
-        unsigned m = vmask[i];
-        if (m) {
-            const int f0 = ob_fptr[vinst[i]];
-            const V3 x0 = mk(y4[i]);
-            while (m) {
-                const int k = __ffs(m) - 1;
-                m &= m - 1;
-                const int f = f0 + k;
-                const V3 x[4] = {x0, mk(xs4[ob_faces[3 * f]]), mk(xs4[ob_faces[3 * f + 1]]),
-                                 mk(xs4[ob_faces[3 * f + 2]])};
-                pair_project(VT_ST, make_int4(i, -1, -1, -1), x, fixed, m_inv, dHat, compliance, dx, nc, &bad);
+    __shared__ unsigned short items[BC_BLOCK / 32][32 * 32];  // the current task's (lane, face bit)s
+    __shared__ int2 stack[BC_BLOCK / 32][64];                 // (vertex, face) past the culls; ~s for obstacle vertex s
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    unsigned short* it = items[threadIdx.x >> 5];
+    int2* st = stack[threadIdx.x >> 5];
+    const long long gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+    const float cull_d2 = dHat * 1.0625f;
+    const long long slots = (long long)S * cap;
+    long long h0 = gw * 32;                                  // first list slot of the warp's next task
+    // vertex tasks from the other end, so that they start on the warps without list slots
+    const long long ntasks = ((long long)V + 31) / 32;
+    long long task = nw - 1 - gw;
+    unsigned m[4] = {0u, 0u, 0u, 0u};  // masks of the tasks task, task + nw, ...
+    int held = 0;                      // of them not yet laid out
+    int v0 = 0, f_first = 0, T = 0, pos = 0, n = 0, bad = 0;
+
+    // positions and vertex ids of a candidate
+    auto load = [&](int2 c, V3 x[4], int4* pr) {
+        const bool tv = c.x < 0;
+        const int* f = tv ? cl_faces + 3 * (size_t)c.y : ob_faces + 3 * (size_t)c.y;
+        const float4* tri = tv ? y4 : xs4;
+        *pr = make_int4(tv ? -1 : c.x, f[0], f[1], f[2]);
+        x[0] = mk(tv ? xs4[~c.x] : y4[c.x]);
+        x[1] = mk(tri[pr->y]);
+        x[2] = mk(tri[pr->z]);
+        x[3] = mk(tri[pr->w]);
+    };
+    for (;;) {
+        bool more = true;
+        while (n < 32 && more) {
+            int2 c = make_int2(0, 0);
+            bool have = false;
+            if (h0 < slots) {
+                const long long h = h0 + lane;
+                if (h < slots) {
+                    const int s = (int)(h / cap), j = (int)(h - (long long)s * cap);
+                    if (j < tv_num[s]) {
+                        c = make_int2(~s, tv_cand[h]);
+                        have = true;
+                    }
+                }
+                h0 += nw * 32;
+            } else if (pos < T) {
+                if (pos + lane < T) {
+                    const int q = it[pos + lane];
+                    c = make_int2(v0 + (q >> 5), 0);
+                    c.y = ob_fptr[vinst[c.x]] + (q & 31);
+                    have = true;
+                }
+                pos += 32;
+            } else if (held > 0) {
+                // the next task's candidates, end to end
+                const unsigned mask = m[0];
+                m[0] = m[1];
+                m[1] = m[2];
+                m[2] = m[3];
+                v0 = (int)(task * 32);
+                task += nw;
+                --held;
+                T = pos = 0;
+                if (__any_sync(0xffffffffu, mask != 0u)) {
+                    const int k = __popc(mask);
+                    int incl = k;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int t = __shfl_up_sync(0xffffffffu, incl, o);
+                        if (lane >= o) incl += t;
+                    }
+                    T = __shfl_sync(0xffffffffu, incl, 31);
+                    int at = incl - k;
+                    for (unsigned r = mask; r != 0u; r &= r - 1u) it[at++] = (unsigned short)(lane * 32 + __ffs(r) - 1);
+                    __syncwarp();
+                }
+                continue;
+            } else if (task < ntasks) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const long long v = (task + i * nw) * 32 + lane;
+                    m[i] = v < V ? vmask[v] : 0u;
+                    if (task + i * nw < ntasks) held = i + 1;
+                }
+                continue;
+            } else {
+                more = false;
             }
+            if (have) {
+                V3 x[4];
+                int4 pr;
+                load(c, x, &pr);
+                have = !box_far(x[0], x[1], x[2], x[3], cull_d2) && !sat_far(x[0], x[1], x[2], x[3], cull_d2);
+            }
+            const unsigned hits = __ballot_sync(0xffffffffu, have);
+            if (have) st[n + __popc(hits & below)] = c;
+            n += __popc(hits);
+            __syncwarp();
         }
-    } else if (i < V + S) {  // __tv_st: obstacle vertex vs its cloth's faces
-        const int s = i - V;
-        const int n = min(tv_num[s], cap);
-        for (int j = 0; j < n; ++j) {
-            const int fd = tv_cand[(size_t)s * cap + j];
-            const int4 vv = make_int4(-1, cl_faces[3 * fd], cl_faces[3 * fd + 1], cl_faces[3 * fd + 2]);
-            const V3 x[4] = {mk(xs4[s]), mk(y4[vv.y]), mk(y4[vv.z]), mk(y4[vv.w])};
-            pair_project(TV_ST, vv, x, fixed, m_inv, dHat, compliance, dx, nc, &bad);
+        if (n == 0) break;
+        const int cnt = n < 32 ? n : 32;
+        if (lane < cnt) {
+            const int2 c = st[n - cnt + lane];
+            V3 x[4];
+            int4 pr;
+            load(c, x, &pr);
+            pair_project(c.x < 0 ? TV_ST : VT_ST, pr, x, fixed, m_inv, dHat, compliance, dx, nc, &bad);
         }
-    }
+        n -= cnt;
+        __syncwarp();
     }
     if (bad) atomicOr(status, SX_STATUS_FIXED_RANGE);
 }
@@ -1749,8 +1901,7 @@ extern "C" int sx_collision_sweep(int n_dy, int n_st, const int* faces_dy, const
         vsc, vsn, vt_dy_cand, vt_dy_num, tv_st_cand, tv_st_num, dx_fix, nc, po, status);
     int rc = check_launch("collision_project_kernel");
     if (rc) return rc;
-    launch(collision_apply_kernel, grid_for(n_dy, 256), 256, 0, s, n_dy, (float4*)y4, fixed, dx_fix, nc,
-           (const int*)nullptr, 0);
+    launch_apply(n_dy, (float4*)y4, fixed, dx_fix, nc, nullptr, 0, s);
     return check_launch("collision_apply_kernel");
 }
 
@@ -1877,8 +2028,7 @@ extern "C" int sx_contact_apply(int n_dy, float* y4, const float* fixed, long lo
     SX_REQUIRE(n_dy >= 0, "sx_contact_apply: bad size");
     if (n_dy == 0) return SX_OK;
     SX_REQUIRE(y4 && fixed && dx_fix && nc, "sx_contact_apply: null pointer");
-    launch(collision_apply_kernel, conv ? capped_grid(collision_apply_kernel, n_dy, 256) : grid_for(n_dy, 256), 256, 0,
-           as_stream(stream), n_dy, (float4*)y4, fixed, dx_fix, nc, conv, iter);
+    launch_apply(n_dy, (float4*)y4, fixed, dx_fix, nc, conv, iter, as_stream(stream));
     return check_launch("collision_apply_kernel");
 }
 
@@ -1897,7 +2047,7 @@ extern "C" int sx_segment_aabbs(const float* p4, const int* seg_ptr, int n_seg, 
     SX_REQUIRE(n_seg >= 0, "sx_segment_aabbs: n_seg < 0");
     if (n_seg == 0) return SX_OK;
     SX_REQUIRE(p4 && seg_ptr && box6, "sx_segment_aabbs: null pointer");
-    launch(segment_aabb_kernel, n_seg, 256, 0, as_stream(stream), (const float4*)p4, seg_ptr, padding, box6);
+    launch(segment_aabb_kernel, n_seg, SEG_BLOCK, 0, as_stream(stream), (const float4*)p4, seg_ptr, padding, box6);
     return check_launch("segment_aabb_kernel");
 }
 
@@ -1937,17 +2087,14 @@ extern "C" int sx_batched_obstacle_contacts(int n_verts, float* y4, const float*
                "sx_batched_obstacle_contacts: null pointer");
     SX_REQUIRE(n_ob_verts == 0 || (tv_cand && tv_num && cl_faces), "sx_batched_obstacle_contacts: null pointer");
     cudaStream_t s = as_stream(stream);
-    launch(batched_contacts_kernel,
-           conv ? capped_grid(batched_contacts_kernel, (long long)n_verts + n_ob_verts, 256)
-                : grid_for((long long)n_verts + n_ob_verts, 256),
-           256, 0, s, n_verts, n_ob_verts,
+    const long long tasks = ((long long)n_ob_verts * cap + 31) / 32 + ((long long)n_verts + 31) / 32;
+    const long long full = (long long)sm_count() * BC_PER_SM, need = (tasks + BC_BLOCK / 32 - 1) / (BC_BLOCK / 32);
+    launch(batched_contacts_kernel, (int)(need < full ? need : full), BC_BLOCK, 0, s, n_verts, n_ob_verts,
            (const float4*)y4, fixed, m_inv, vinst, ob_fptr, ob_faces, (const float4*)xs4, vmask, tv_cand, tv_num,
            cap, cl_faces, dHat, compliance, dx_fix, nc, status, conv, iter);
     int rc = check_launch("batched_contacts_kernel");
     if (rc) return rc;
-    launch(collision_apply_kernel, conv ? capped_grid(collision_apply_kernel, n_verts, 256) : grid_for(n_verts, 256),
-           256, 0, s, n_verts, (float4*)y4, fixed, dx_fix, nc, conv,
-           iter);
+    launch_apply(n_verts, (float4*)y4, fixed, dx_fix, nc, conv, iter, s);
     return check_launch("collision_apply_kernel");
 }
 

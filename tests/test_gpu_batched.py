@@ -161,3 +161,56 @@ def test_persistent_substep_batched512(pkg):
     a.forward(10)
     torch.cuda.synchronize()
     assert torch.equal(a.x4, b.x4) and torch.equal(a.v4, b.v4)
+
+
+@pytest.mark.parametrize("n,cap,offset", [(6, 40, 0.0), (33, 40, 0.0), (33, 40, 0.31), (64, 64, 0.0)])
+def test_batched_lying_cloths(pkg, po, n, cap, offset):
+    """Cloths that start in contact range of their boxes: most vertices hold
+    obstacle candidates, so the contact kernel's tasks fill (partial last tasks
+    included) and the obstacle's corners have full lists."""
+    rng = np.random.default_rng(n)
+    insts = []
+    for i in range(3):
+        ox = 1.5 * i
+        x, f = pkg.grid_cloth(n, origin=(ox, 0.0), height=1.0)
+        x = (x + rng.uniform(-1e-4, 1e-4, x.shape).astype(np.float32)).astype(np.float32)
+        bx, bf = pkg.box_mesh(0.5, center=(ox + 0.5 + offset, 0.5 - offset, 0.7475))
+        insts.append(pkg.Instance(x, f, np.array([(n - 1) * n, n * n - 1]), bx, bf))
+    kw = dict(dt=1 / 60, g=(0.0, 0.0, -9.81), k_stretch_stiffness=1e5, k_bend_stiffness=1e8, dHat=(4e-3) ** 2,
+              damping=0.001, padding=8e-3, n_iter=5, cap=cap)
+    sim = pkg.BatchedSolver(insts, dHat=kw["dHat"], stiffness_stretch=1e5, stiffness_bending=1e8, g=kw["g"],
+                            dt=kw["dt"], n_iter=5, padding=8e-3, cap=cap)
+    sim.forward(10)
+    torch.cuda.synchronize()
+    for i, inst in enumerate(insts):
+        orc = _oracle_instance(pkg, po, inst, 1, kw)
+        assert np.array_equal(sim.instance_positions(i).cpu().numpy(), orc.x4[:, :3])
+
+
+@pytest.mark.parametrize("V", [1, 255, 262144, 262145, 262147, 300002])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_contact_apply_widths(pkg, V, shift):
+    """update_dx at one and at four vertices a thread, ragged tails and an
+    unaligned count array: y + fixed * (sum / count), accumulators cleared."""
+    from starlab_physics_gb300 import _lib
+
+    rng = np.random.default_rng(V + shift)
+    y = rng.normal(0, 1, (V, 4)).astype(np.float32)
+    fixed = (rng.random(V) < 0.8).astype(np.float32)
+    nc = np.where(rng.random(V) < 0.3, rng.integers(1, 9, V), 0).astype(np.int32)
+    nc[-1] = 3
+    acc = (rng.normal(0, 1e-3, (V, 3)) * 2.0 ** 40).astype(np.int64)
+    acc[::7] = (rng.normal(0, 1.0, acc[::7].shape) * 2.0 ** 58).astype(np.int64)
+    acc[nc == 0] = 0
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    Y, F, A = t(y), t(fixed), t(acc)
+    N = torch.zeros(V + 4, dtype=torch.int32, device="cuda")
+    N[shift:shift + V] = t(nc)
+    _lib.sx.sx_contact_apply(V, Y.data_ptr(), F.data_ptr(), A.data_ptr(), N.data_ptr() + 4 * shift, None, 0,
+                             torch.cuda.current_stream().cuda_stream)
+    want = y.copy()
+    on = nc > 0
+    d = (acc[on].astype(np.float64) * 2.0 ** -40).astype(np.float32)
+    want[on, :3] = y[on, :3] + fixed[on, None] * (d / nc[on, None].astype(np.float32))
+    assert np.array_equal(Y.cpu().numpy(), want)
+    assert int(A.abs().max()) == 0 and int(N.abs().max()) == 0
