@@ -518,6 +518,23 @@ int sx_batched_obstacle_contacts(int n_verts, float* y4, const float* fixed, con
                                  int n_ob_verts, const int* tv_cand, const int* tv_num, int cap, const int* cl_faces,
                                  float dHat, float compliance, long long* dx_fix, int* nc, int* status, const int* conv,
                                  int iter, void* stream);
+/* The substep's obstacle candidates (the broad phase's masks and lists) as one
+ * dense list for sx_batched_obstacle_contacts_listed, whose iterations then
+ * read it instead of scanning the masks of every vertex: the same contacts.
+ * list: sx_batched_contact_list_bytes bytes, 16-byte aligned; it holds 8
+ * candidates per vertex and every obstacle-vertex slot, and when a scene has
+ * more the contacts are taken from the masks and lists as without it (list
+ * NULL).  The masks and lists must not change between the two calls. */
+size_t sx_batched_contact_list_bytes(int n_verts, int n_ob_verts, int cap);
+int sx_batched_contact_list(int n_verts, const unsigned* vmask, const int* vinst, const int* ob_fptr,
+                            const int* ob_faces, int n_ob_verts, const int* tv_cand, const int* tv_num, int cap,
+                            const int* cl_faces, void* list, size_t list_bytes, void* stream);
+int sx_batched_obstacle_contacts_listed(int n_verts, float* y4, const float* fixed, const float* m_inv,
+                                        const int* vinst, const int* ob_fptr, const int* ob_faces, const float* xs4,
+                                        const unsigned* vmask, int n_ob_verts, const int* tv_cand, const int* tv_num,
+                                        int cap, const int* cl_faces, const void* list, float dHat, float compliance,
+                                        long long* dx_fix, int* nc, int* status, const int* conv, int iter,
+                                        void* stream);
 
 /* ---- constraint-graph colouring (framework/utilities/graph_coloring.py) --- */
 

@@ -105,6 +105,9 @@ SIGNATURES = {
     "sx_cell_bvh_traverse_edges": ([P, I, P, F, P, P, P, P, P, P, I, P, P, P, P], I),
     "sx_segment_aabbs": ([P, P, I, F, P, P], I),
     "sx_batched_obstacle_broadphase": ([I, P, P, P, P, P, P, F, P, I, P, P, P, P, P, P, P, P, I, P, P, P, P], I),
+    "sx_batched_contact_list_bytes": ([I, I, I], Z),
+    "sx_batched_contact_list": ([I, P, P, P, P, I, P, P, I, P, P, Z, P], I),
+    "sx_batched_obstacle_contacts_listed": ([I, P, P, P, P, P, P, P, P, I, P, P, I, P, P, F, F, P, P, P, P, I, P], I),
     "sx_batched_obstacle_contacts": ([I, P, P, P, P, P, P, P, P, I, P, P, I, P, F, F, P, P, P, P, I, P], I),
     "sx_mlp_param_count": ([], I),
     "sx_mlp_bf16_count": ([], I),

@@ -188,6 +188,9 @@ class BatchedSolver:
         self.status = torch.zeros(1, dtype=torch.int32, device=dev)
         self._dx_fix = torch.zeros(3 * V, dtype=torch.int64, device=dev)
         self._nc = torch.zeros(V, dtype=torch.int32, device=dev)
+        # the substep's obstacle candidates as one dense list
+        self._list = torch.zeros(int(sx.sx_batched_contact_list_bytes(V, self.n_ob_verts, cap)), dtype=torch.uint8,
+                                 device=dev)
         # learned warm start (learned.WarmStart) run after each prediction
         self.warm = None
         # launch configuration of the fixed-count sweep: None = the library's
@@ -374,11 +377,14 @@ class BatchedSolver:
                 ptr(self.xs4), ptr(self.svinst), ptr(self.cl_box6), ptr(self.fptr), ptr(self.fmin4),
                 ptr(self.fmax4), ptr(self.cmin4), ptr(self.cmax4), self.cap, ptr(self.tv_cand), ptr(self.tv_num),
                 ptr(self.status), s)
-        sx.sx_batched_obstacle_contacts(
+            sx.sx_batched_contact_list(self.num_verts, ptr(self.vmask), ptr(self.vinst), ptr(self.ob_fptr),
+                                       ptr(self.ob_faces), self.n_ob_verts, ptr(self.tv_cand), ptr(self.tv_num),
+                                       self.cap, ptr(self.faces), ptr(self._list), self._list.numel(), s)
+        sx.sx_batched_obstacle_contacts_listed(
             self.num_verts, ptr(self.y4), ptr(self.fixed), ptr(self.m_inv), ptr(self.vinst), ptr(self.ob_fptr),
             ptr(self.ob_faces), ptr(self.xs4), ptr(self.vmask), self.n_ob_verts, ptr(self.tv_cand),
-            ptr(self.tv_num), self.cap, ptr(self.faces), self.dHat, self.compliance_collision, ptr(self._dx_fix),
-            ptr(self._nc), ptr(self.status), None if in_loop else conv, it, s)
+            ptr(self.tv_num), self.cap, ptr(self.faces), ptr(self._list), self.dHat, self.compliance_collision,
+            ptr(self._dx_fix), ptr(self._nc), ptr(self.status), None if in_loop else conv, it, s)
 
     def _forward_eager(self, n_substeps):
         if self._ob_built_for != self.padding:

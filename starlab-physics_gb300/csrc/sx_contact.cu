@@ -919,42 +919,27 @@ __global__ void __launch_bounds__(PP_BLOCK, MINB) pairs_project_kernel(const int
 }
 
 // update_dx (XPBD.py:384-387) from the fixed-point accumulators; clears them.
-// Few vertices have a correction: the kernel is bound by reading every count,
-// so a thread reads N of them with one load (N = 4 where nc is 16-byte aligned).
-template <int N>
+// One vertex a thread: four a thread (their counts in one load, or strided by
+// 32) saves waves but serialises the corrections of a resting cloth's
+// neighbouring vertices; a frame of 96 cloths took 9.45 instead of 8.44 ms.
 __global__ void collision_apply_kernel(int V, float4* __restrict__ y4, const float* __restrict__ fixed,
                                        long long* __restrict__ dx, int* __restrict__ nc, const int* conv, int iter) {
     pdl_entry();
     if (iteration_skipped(conv, iter)) return;
-    const long long stride = (long long)gridDim.x * blockDim.x * N;
-    for (long long v0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * N; v0 < V; v0 += stride) {
-        int c[N];
-        if (N == 4 && v0 + 4 <= V) {
-            const int4 q = *reinterpret_cast<const int4*>(nc + v0);
-            c[0] = q.x;
-            c[N > 1 ? 1 : 0] = q.y;
-            c[N > 2 ? 2 : 0] = q.z;
-            c[N > 3 ? 3 : 0] = q.w;
-        } else {
-#pragma unroll
-            for (int j = 0; j < N; ++j) c[j] = v0 + j < V ? nc[v0 + j] : 0;
-        }
-#pragma unroll
-        for (int j = 0; j < N; ++j) {
-            if (c[j] > 0) {
-                const long long v = v0 + j;
-                const float cf = (float)c[j];
-                const float f = fixed[v];
-                float4 y = y4[v];
-                y.x = y.x + f * (from_fix(dx[3 * v]) / cf);
-                y.y = y.y + f * (from_fix(dx[3 * v + 1]) / cf);
-                y.z = y.z + f * (from_fix(dx[3 * v + 2]) / cf);
-                y4[v] = y;
-                dx[3 * v] = 0;
-                dx[3 * v + 1] = 0;
-                dx[3 * v + 2] = 0;
-                nc[v] = 0;
-            }
+    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
+        const int c = nc[v];
+        if (c > 0) {
+            const float cf = (float)c;
+            const float f = fixed[v];
+            float4 y = y4[v];
+            y.x = y.x + f * (from_fix(dx[3 * v]) / cf);
+            y.y = y.y + f * (from_fix(dx[3 * v + 1]) / cf);
+            y.z = y.z + f * (from_fix(dx[3 * v + 2]) / cf);
+            y4[v] = y;
+            dx[3 * v] = 0;
+            dx[3 * v + 1] = 0;
+            dx[3 * v + 2] = 0;
+            nc[v] = 0;
         }
     }
 }
@@ -966,15 +951,10 @@ inline int capped_grid(K kernel, long long n, int block) {
     return g < cap ? g : cap;
 }
 
-// collision_apply_kernel: four vertices a thread once one a thread is more
-// than one resident wave (600 000 vertices 8.4 us in three waves of one-vertex
-// threads)
 static void launch_apply(int V, float4* y4, const float* fixed, long long* dx, int* nc, const int* conv, int iter,
                          cudaStream_t s) {
-    const bool wide = V > 262144 && ((uintptr_t)nc & 15) == 0;
-    const auto k = wide ? collision_apply_kernel<4> : collision_apply_kernel<1>;
-    const long long n = wide ? (V + 3LL) / 4 : V;
-    launch(k, conv ? capped_grid(k, n, 256) : grid_for(n, 256), 256, 0, s, V, y4, fixed, dx, nc, conv, iter);
+    launch(collision_apply_kernel, conv ? capped_grid(collision_apply_kernel, V, 256) : grid_for(V, 256), 256, 0, s, V,
+           y4, fixed, dx, nc, conv, iter);
 }
 
 // ---------------------------------------------------------------------------
@@ -1130,17 +1110,71 @@ __global__ void batched_tv_st_broad_kernel(int S, const float4* __restrict__ xs4
     }
 }
 
+// The candidates of a substep as one dense list of quads, in no particular
+// order (contact sums are order independent): (vertex, obstacle triangle) for
+// the set bits of the vertices' face masks, (~obstacle vertex, cloth triangle)
+// for the obstacle vertices' lists.  *count is the number found, also past the
+// capacity; the list is then not used.
+__global__ void __launch_bounds__(256) batched_list_kernel(int V, int S, const unsigned* __restrict__ vmask,
+                                                           const int* __restrict__ vinst,
+                                                           const int* __restrict__ ob_fptr,
+                                                           const int* __restrict__ ob_faces,
+                                                           const int* __restrict__ tv_cand,
+                                                           const int* __restrict__ tv_num, int cap,
+                                                           const int* __restrict__ cl_faces, int4* list,
+                                                           long long capacity, unsigned long long* count) {
+    pdl_entry();
+    const int lane = threadIdx.x & 31;
+    const long long nv = ((long long)V + 31) / 32 * 32, total = nv + (long long)S * cap;
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i - lane >= total) return;
+    unsigned mask = 0u;
+    const int* face = nullptr;  // the first candidate's triangle
+    int who = 0;
+    if (i < V) {
+        mask = vmask[i];
+        who = (int)i;
+        if (mask) face = ob_faces + 3 * (size_t)ob_fptr[vinst[i]];
+    } else if (i >= nv && i < total) {
+        const long long h = i - nv;
+        const int s = (int)(h / cap), j = (int)(h - (long long)s * cap);
+        if (j < tv_num[s]) {
+            mask = 1u;
+            who = ~s;
+            face = cl_faces + 3 * (size_t)tv_cand[h];
+        }
+    }
+    if (!__any_sync(0xffffffffu, mask != 0u)) return;
+    const int k = __popc(mask);
+    int incl = k;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+    }
+    unsigned long long at = 0;
+    if (lane == 31) at = atomicAdd(count, (unsigned long long)incl);
+    at = __shfl_sync(0xffffffffu, at, 31) + (unsigned long long)(incl - k);
+    for (unsigned r = mask; r != 0u; r &= r - 1u, ++at) {
+        const int* f = face + 3 * (__ffs(r) - 1);
+        if (at < (unsigned long long)capacity) list[at] = make_int4(who, f[0], f[1], f[2]);
+    }
+}
+
 // Obstacle contacts of one iteration.  A candidate is an (obstacle vertex,
 // cloth face) slot or a set bit of a cloth vertex's face mask; few vertices have
 // any, and a corner of an obstacle under a lying cloth has as many as its list
 // holds.  One thread per vertex would walk such a list alone (40 dependent
 // classifications: 99 us per launch on 24 cloths lying on their boxes, 160 000
-// vertices); here each warp lays the candidates of its tasks end to end, tests
-// them 32 at a time with the pair list's culls (box_far, sat_far: of a box
-// side's two triangles most vertices reach one) and projects the survivors 32
-// at a time.  Tasks are 32 slots of the obstacle vertices' lists, then 32 cloth
-// vertices, dealt to the warps in turn; a warp loads the masks of four tasks
-// together.  Contact sums are order independent.
+// vertices); here a warp tests candidates 32 at a time with the pair list's
+// culls (box_far, sat_far: of a box side's two triangles most vertices reach
+// one) and projects the survivors 32 at a time.  With the substep's list
+// (batched_list_kernel) the candidates are dealt evenly and one load away from
+// their positions; without it, or when it overflowed, the warps take 32 slots of
+// the obstacle vertices' lists, then 32 cloth vertices at a time, and lay the
+// set bits end to end themselves (24 cloths 19 us against 9.6 with the list, 96
+// cloths 40 against 17.5 per launch, caches cold).
+// Contact sums are order independent.
 constexpr int BC_BLOCK = 256, BC_PER_SM = 2;
 
 __global__ void __launch_bounds__(BC_BLOCK, BC_PER_SM) batched_contacts_kernel(
@@ -1148,57 +1182,60 @@ __global__ void __launch_bounds__(BC_BLOCK, BC_PER_SM) batched_contacts_kernel(
     const int* __restrict__ vinst, const int* __restrict__ ob_fptr, const int* __restrict__ ob_faces,
     const float4* __restrict__ xs4, const unsigned* __restrict__ vmask, const int* __restrict__ tv_cand,
     const int* __restrict__ tv_num, int cap, const int* __restrict__ cl_faces, float dHat, float compliance,
-    long long* dx, int* nc, int* status, const int* conv, int iter) {
+    const int4* __restrict__ list, long long capacity, const unsigned long long* __restrict__ count, long long* dx,
+    int* nc, int* status, const int* conv, int iter) {
     pdl_entry();
     if (iteration_skipped(conv, iter)) return;
     __shared__ unsigned short items[BC_BLOCK / 32][32 * 32];  // the current task's (lane, face bit)s
-    __shared__ int2 stack[BC_BLOCK / 32][64];                 // (vertex, face) past the culls; ~s for obstacle vertex s
+    __shared__ int4 stack[BC_BLOCK / 32][64];                 // quads past the culls
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
     unsigned short* it = items[threadIdx.x >> 5];
-    int2* st = stack[threadIdx.x >> 5];
+    int4* st = stack[threadIdx.x >> 5];
     const long long gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
     const float cull_d2 = dHat * 1.0625f;
-    const long long slots = (long long)S * cap;
-    long long h0 = gw * 32;                                  // first list slot of the warp's next task
+    const unsigned long long found = list != nullptr ? *count : ~0ull;
+    const bool listed = found <= (unsigned long long)capacity;
+    const long long slots = listed ? (long long)found : (long long)S * cap;
+    long long h0 = gw * 32;  // first list entry or slot of the warp's next task
     // vertex tasks from the other end, so that they start on the warps without list slots
-    const long long ntasks = ((long long)V + 31) / 32;
+    const long long ntasks = listed ? 0 : ((long long)V + 31) / 32;
     long long task = nw - 1 - gw;
     unsigned m[4] = {0u, 0u, 0u, 0u};  // masks of the tasks task, task + nw, ...
     int held = 0;                      // of them not yet laid out
-    int v0 = 0, f_first = 0, T = 0, pos = 0, n = 0, bad = 0;
+    int v0 = 0, T = 0, pos = 0, n = 0, bad = 0;
 
-    // positions and vertex ids of a candidate
-    auto load = [&](int2 c, V3 x[4], int4* pr) {
+    auto points = [&](int4 c, V3 x[4]) {
         const bool tv = c.x < 0;
-        const int* f = tv ? cl_faces + 3 * (size_t)c.y : ob_faces + 3 * (size_t)c.y;
         const float4* tri = tv ? y4 : xs4;
-        *pr = make_int4(tv ? -1 : c.x, f[0], f[1], f[2]);
         x[0] = mk(tv ? xs4[~c.x] : y4[c.x]);
-        x[1] = mk(tri[pr->y]);
-        x[2] = mk(tri[pr->z]);
-        x[3] = mk(tri[pr->w]);
+        x[1] = mk(tri[c.y]);
+        x[2] = mk(tri[c.z]);
+        x[3] = mk(tri[c.w]);
     };
+    auto quad = [](int who, const int* f) { return make_int4(who, f[0], f[1], f[2]); };
     for (;;) {
         bool more = true;
         while (n < 32 && more) {
-            int2 c = make_int2(0, 0);
+            int4 c = make_int4(0, 0, 0, 0);
             bool have = false;
             if (h0 < slots) {
                 const long long h = h0 + lane;
-                if (h < slots) {
+                if (h < slots && listed) {
+                    c = list[h];
+                    have = true;
+                } else if (h < slots) {
                     const int s = (int)(h / cap), j = (int)(h - (long long)s * cap);
                     if (j < tv_num[s]) {
-                        c = make_int2(~s, tv_cand[h]);
+                        c = quad(~s, cl_faces + 3 * (size_t)tv_cand[h]);
                         have = true;
                     }
                 }
                 h0 += nw * 32;
             } else if (pos < T) {
                 if (pos + lane < T) {
-                    const int q = it[pos + lane];
-                    c = make_int2(v0 + (q >> 5), 0);
-                    c.y = ob_fptr[vinst[c.x]] + (q & 31);
+                    const int q = it[pos + lane], v = v0 + (q >> 5);
+                    c = quad(v, ob_faces + 3 * (size_t)(ob_fptr[vinst[v]] + (q & 31)));
                     have = true;
                 }
                 pos += 32;
@@ -1239,8 +1276,7 @@ __global__ void __launch_bounds__(BC_BLOCK, BC_PER_SM) batched_contacts_kernel(
             }
             if (have) {
                 V3 x[4];
-                int4 pr;
-                load(c, x, &pr);
+                points(c, x);
                 have = !box_far(x[0], x[1], x[2], x[3], cull_d2) && !sat_far(x[0], x[1], x[2], x[3], cull_d2);
             }
             const unsigned hits = __ballot_sync(0xffffffffu, have);
@@ -1251,11 +1287,10 @@ __global__ void __launch_bounds__(BC_BLOCK, BC_PER_SM) batched_contacts_kernel(
         if (n == 0) break;
         const int cnt = n < 32 ? n : 32;
         if (lane < cnt) {
-            const int2 c = st[n - cnt + lane];
+            const int4 c = st[n - cnt + lane];
             V3 x[4];
-            int4 pr;
-            load(c, x, &pr);
-            pair_project(c.x < 0 ? TV_ST : VT_ST, pr, x, fixed, m_inv, dHat, compliance, dx, nc, &bad);
+            points(c, x);
+            pair_project(c.x < 0 ? TV_ST : VT_ST, c, x, fixed, m_inv, dHat, compliance, dx, nc, &bad);
         }
         n -= cnt;
         __syncwarp();
@@ -2075,27 +2110,70 @@ extern "C" int sx_batched_obstacle_broadphase(int n_verts, const float* y4, cons
     return check_launch("sx_batched_obstacle_broadphase");
 }
 
+// list workspace: [count, 256 bytes][quads]
+static long long list_capacity(int n_verts, int n_ob_verts, int cap) {
+    return 8LL * n_verts + (long long)n_ob_verts * cap;
+}
+
+extern "C" size_t sx_batched_contact_list_bytes(int n_verts, int n_ob_verts, int cap) {
+    if (n_verts < 0 || n_ob_verts < 0 || cap < 1) return 0;
+    return 256 + (size_t)list_capacity(n_verts, n_ob_verts, cap) * sizeof(int4);
+}
+
+extern "C" int sx_batched_contact_list(int n_verts, const unsigned* vmask, const int* vinst, const int* ob_fptr,
+                                       const int* ob_faces, int n_ob_verts, const int* tv_cand, const int* tv_num,
+                                       int cap, const int* cl_faces, void* list, size_t list_bytes, void* stream) {
+    SX_REQUIRE(n_verts >= 0 && n_ob_verts >= 0 && cap >= 1, "sx_batched_contact_list: bad sizes");
+    SX_REQUIRE(list && ((uintptr_t)list & 15) == 0 &&
+                   list_bytes >= sx_batched_contact_list_bytes(n_verts, n_ob_verts, cap),
+               "sx_batched_contact_list: list must be 16-byte aligned and sx_batched_contact_list_bytes long");
+    SX_REQUIRE(n_verts == 0 || (vmask && vinst && ob_fptr && ob_faces), "sx_batched_contact_list: null pointer");
+    SX_REQUIRE(n_ob_verts == 0 || (tv_cand && tv_num && cl_faces), "sx_batched_contact_list: null pointer");
+    cudaStream_t s = as_stream(stream);
+    SX_CUDA(cudaMemsetAsync(list, 0, 256, s));
+    const long long total = ((long long)n_verts + 31) / 32 * 32 + (long long)n_ob_verts * cap;
+    if (total == 0) return SX_OK;
+    launch(batched_list_kernel, grid_for(total, 256), 256, 0, s, n_verts, n_ob_verts, vmask, vinst, ob_fptr, ob_faces,
+           tv_cand, tv_num, cap, cl_faces, (int4*)((char*)list + 256), list_capacity(n_verts, n_ob_verts, cap),
+           (unsigned long long*)list);
+    return check_launch("batched_list_kernel");
+}
+
+extern "C" int sx_batched_obstacle_contacts_listed(int n_verts, float* y4, const float* fixed, const float* m_inv,
+                                                   const int* vinst, const int* ob_fptr, const int* ob_faces,
+                                                   const float* xs4, const unsigned* vmask, int n_ob_verts,
+                                                   const int* tv_cand, const int* tv_num, int cap,
+                                                   const int* cl_faces, const void* list, float dHat,
+                                                   float compliance, long long* dx_fix, int* nc, int* status,
+                                                   const int* conv, int iter, void* stream) {
+    SX_REQUIRE(n_verts >= 0 && n_ob_verts >= 0 && cap >= 1, "sx_batched_obstacle_contacts: bad sizes");
+    if (n_verts == 0) return SX_OK;
+    SX_REQUIRE(y4 && fixed && m_inv && vinst && ob_fptr && ob_faces && xs4 && vmask && dx_fix && nc && status,
+               "sx_batched_obstacle_contacts: null pointer");
+    SX_REQUIRE(n_ob_verts == 0 || (tv_cand && tv_num && cl_faces), "sx_batched_obstacle_contacts: null pointer");
+    SX_REQUIRE(((uintptr_t)list & 15) == 0, "sx_batched_obstacle_contacts: list must be 16-byte aligned");
+    cudaStream_t s = as_stream(stream);
+    const long long tasks = ((long long)n_ob_verts * cap + 31) / 32 + ((long long)n_verts + 31) / 32;
+    const long long full = (long long)sm_count() * BC_PER_SM, need = (tasks + BC_BLOCK / 32 - 1) / (BC_BLOCK / 32);
+    launch(batched_contacts_kernel, (int)(need < full ? need : full), BC_BLOCK, 0, s, n_verts, n_ob_verts,
+           (const float4*)y4, fixed, m_inv, vinst, ob_fptr, ob_faces, (const float4*)xs4, vmask, tv_cand, tv_num,
+           cap, cl_faces, dHat, compliance, (const int4*)(list ? (const char*)list + 256 : nullptr),
+           list_capacity(n_verts, n_ob_verts, cap), (const unsigned long long*)list, dx_fix, nc, status, conv, iter);
+    int rc = check_launch("batched_contacts_kernel");
+    if (rc) return rc;
+    launch_apply(n_verts, (float4*)y4, fixed, dx_fix, nc, conv, iter, s);
+    return check_launch("collision_apply_kernel");
+}
+
 extern "C" int sx_batched_obstacle_contacts(int n_verts, float* y4, const float* fixed, const float* m_inv,
                                             const int* vinst, const int* ob_fptr, const int* ob_faces,
                                             const float* xs4, const unsigned* vmask, int n_ob_verts,
                                             const int* tv_cand, const int* tv_num, int cap, const int* cl_faces,
                                             float dHat, float compliance, long long* dx_fix, int* nc, int* status,
                                             const int* conv, int iter, void* stream) {
-    SX_REQUIRE(n_verts >= 0 && n_ob_verts >= 0 && cap >= 1, "sx_batched_obstacle_contacts: bad sizes");
-    if (n_verts == 0) return SX_OK;
-    SX_REQUIRE(y4 && fixed && m_inv && vinst && ob_fptr && ob_faces && xs4 && vmask && dx_fix && nc && status,
-               "sx_batched_obstacle_contacts: null pointer");
-    SX_REQUIRE(n_ob_verts == 0 || (tv_cand && tv_num && cl_faces), "sx_batched_obstacle_contacts: null pointer");
-    cudaStream_t s = as_stream(stream);
-    const long long tasks = ((long long)n_ob_verts * cap + 31) / 32 + ((long long)n_verts + 31) / 32;
-    const long long full = (long long)sm_count() * BC_PER_SM, need = (tasks + BC_BLOCK / 32 - 1) / (BC_BLOCK / 32);
-    launch(batched_contacts_kernel, (int)(need < full ? need : full), BC_BLOCK, 0, s, n_verts, n_ob_verts,
-           (const float4*)y4, fixed, m_inv, vinst, ob_fptr, ob_faces, (const float4*)xs4, vmask, tv_cand, tv_num,
-           cap, cl_faces, dHat, compliance, dx_fix, nc, status, conv, iter);
-    int rc = check_launch("batched_contacts_kernel");
-    if (rc) return rc;
-    launch_apply(n_verts, (float4*)y4, fixed, dx_fix, nc, conv, iter, s);
-    return check_launch("collision_apply_kernel");
+    return sx_batched_obstacle_contacts_listed(n_verts, y4, fixed, m_inv, vinst, ob_fptr, ob_faces, xs4, vmask,
+                                               n_ob_verts, tv_cand, tv_num, cap, cl_faces, nullptr, dHat, compliance,
+                                               dx_fix, nc, status, conv, iter, stream);
 }
 
 // Launch configurations of the persistent batched substep: threads per CTA

@@ -187,14 +187,13 @@ def test_batched_lying_cloths(pkg, po, n, cap, offset):
         assert np.array_equal(sim.instance_positions(i).cpu().numpy(), orc.x4[:, :3])
 
 
-@pytest.mark.parametrize("V", [1, 255, 262144, 262145, 262147, 300002])
-@pytest.mark.parametrize("shift", [0, 1])
-def test_contact_apply_widths(pkg, V, shift):
-    """update_dx at one and at four vertices a thread, ragged tails and an
-    unaligned count array: y + fixed * (sum / count), accumulators cleared."""
+@pytest.mark.parametrize("V", [1, 255, 4099])
+def test_contact_apply_values(pkg, V):
+    """update_dx from the fixed-point sums, small ones and ones past 2^53:
+    y + fixed * (sum / count), accumulators cleared."""
     from starlab_physics_gb300 import _lib
 
-    rng = np.random.default_rng(V + shift)
+    rng = np.random.default_rng(V)
     y = rng.normal(0, 1, (V, 4)).astype(np.float32)
     fixed = (rng.random(V) < 0.8).astype(np.float32)
     nc = np.where(rng.random(V) < 0.3, rng.integers(1, 9, V), 0).astype(np.int32)
@@ -203,10 +202,8 @@ def test_contact_apply_widths(pkg, V, shift):
     acc[::7] = (rng.normal(0, 1.0, acc[::7].shape) * 2.0 ** 58).astype(np.int64)
     acc[nc == 0] = 0
     t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
-    Y, F, A = t(y), t(fixed), t(acc)
-    N = torch.zeros(V + 4, dtype=torch.int32, device="cuda")
-    N[shift:shift + V] = t(nc)
-    _lib.sx.sx_contact_apply(V, Y.data_ptr(), F.data_ptr(), A.data_ptr(), N.data_ptr() + 4 * shift, None, 0,
+    Y, F, A, N = t(y), t(fixed), t(acc), t(nc)
+    _lib.sx.sx_contact_apply(V, Y.data_ptr(), F.data_ptr(), A.data_ptr(), N.data_ptr(), None, 0,
                              torch.cuda.current_stream().cuda_stream)
     want = y.copy()
     on = nc > 0
@@ -214,3 +211,43 @@ def test_contact_apply_widths(pkg, V, shift):
     want[on, :3] = y[on, :3] + fixed[on, None] * (d / nc[on, None].astype(np.float32))
     assert np.array_equal(Y.cpu().numpy(), want)
     assert int(A.abs().max()) == 0 and int(N.abs().max()) == 0
+
+
+@pytest.mark.parametrize("mask,n", [(0, 9), (0x3, 9), (0x421, 33), (0xFF, 33), (0xFFF, 33)])
+def test_listed_contacts_equal_mask_walk(pkg, mask, n):
+    """The dense candidate list against the walk of the masks, also when the
+    list overflows (more than 8 candidates a vertex) and the walk takes over."""
+    from starlab_physics_gb300 import _lib
+    from starlab_physics_gb300._lib import ptr
+
+    insts = []
+    for i in range(3):
+        x, f = pkg.grid_cloth(n + i, origin=(1.5 * i, 0.0), height=1.0)
+        bx, bf = pkg.box_mesh(0.5, center=(1.5 * i + 0.6, 0.5, 0.7475))
+        insts.append(pkg.Instance(x, f, np.array([0]), bx, bf))
+    sim = pkg.BatchedSolver(insts, dHat=1.6e-5, stiffness_stretch=1e5, stiffness_bending=1e8, g=(0, 0, -9.81),
+                            dt=1 / 60, n_iter=2, padding=8e-3)
+    sim.forward(10)
+    sim.vmask.fill_(mask)
+    s = torch.cuda.current_stream().cuda_stream
+    y0 = sim.y4.clone()
+    outs = []
+    for listed in (False, True):
+        sim.y4.copy_(y0)
+        args = [sim.num_verts, ptr(sim.y4), ptr(sim.fixed), ptr(sim.m_inv), ptr(sim.vinst), ptr(sim.ob_fptr),
+                ptr(sim.ob_faces), ptr(sim.xs4), ptr(sim.vmask), sim.n_ob_verts, ptr(sim.tv_cand), ptr(sim.tv_num),
+                sim.cap, ptr(sim.faces)]
+        tail = [sim.dHat, 1e8, ptr(sim._dx_fix), ptr(sim._nc), ptr(sim.status), None, 0, s]
+        if listed:
+            _lib.sx.sx_batched_contact_list(sim.num_verts, ptr(sim.vmask), ptr(sim.vinst), ptr(sim.ob_fptr),
+                                            ptr(sim.ob_faces), sim.n_ob_verts, ptr(sim.tv_cand), ptr(sim.tv_num),
+                                            sim.cap, ptr(sim.faces), ptr(sim._list), sim._list.numel(), s)
+            _lib.sx.sx_batched_obstacle_contacts_listed(*args, ptr(sim._list), *tail)
+        else:
+            _lib.sx.sx_batched_obstacle_contacts(*args, *tail)
+        outs.append(sim.y4.clone())
+    found = int(sim._list[:8].view(torch.int64).item())
+    slots = int(torch.clamp(sim.tv_num, max=sim.cap).sum().item())
+    assert found == bin(mask).count("1") * sim.num_verts + slots
+    assert torch.equal(outs[0], outs[1])
+    assert int(sim._nc.abs().max().item()) == 0
