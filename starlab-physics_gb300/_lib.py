@@ -165,41 +165,62 @@ def load(build_if_missing: bool = True):
         return _lib
 
 
-def _call(name, *args):
-    L = load()
-    rc = getattr(L, name)(*args)
-    if rc != SX_OK:
-        raise SxError(name, rc, L.sx_last_error().decode(errors="replace"))
-    return rc
-
-
 def ptr(t) -> int | None:
     """Device pointer of a tensor (None for None)."""
     return None if t is None else t.data_ptr()
 
 
+_raw_stream = None  # (current device, current raw stream of a device) of torch's C module
+
+
 def stream_handle(stream=None) -> int:
+    """cudaStream_t of ``stream`` (default: torch's current stream).  Once CUDA is
+    initialised the current stream's handle is read from torch's C module: the
+    Stream object of ``torch.cuda.current_stream()`` costs more than the launch
+    it is made for (some 4 us, a few hundred times per eager frame)."""
+    global _raw_stream
+    if stream is not None:
+        return stream.cuda_stream
+    if _raw_stream is not None:
+        device, handle = _raw_stream
+        return handle(device())
     import torch
 
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return s.cuda_stream
+    s = torch.cuda.current_stream().cuda_stream  # initialises CUDA, or raises without a device
+    device = getattr(torch._C, "_cuda_getDevice", None)
+    handle = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    if device is not None and handle is not None and handle(device()) == s:
+        _raw_stream = (device, handle)
+    return s
+
+
+# entry points whose int result is a value, not a status
+_VALUES = ("sx_version", "sx_mlp_param_count", "sx_mlp_bf16_count", "sx_jacobi_sweep_variants",
+           "sx_jacobi_sweep_packed_forms", "sx_jacobi_sweep_default_variant", "sx_contact_pairs_project_variants",
+           "sx_contact_pairs_project_variant_pipelined", "sx_batched_substep_variants",
+           "sx_batched_substep_variant_cluster")
 
 
 class _Calls:
-    """Attribute access returns a checked caller: ``sx.sx_predict(...)``."""
+    """Attribute access returns a checked caller: ``sx.sx_predict(...)``.  Each is
+    made once and kept on the object, so later accesses skip the lookup."""
 
     def __getattr__(self, name):
         if name not in SIGNATURES:
             raise AttributeError(name)
-        if SIGNATURES[name][1] is I and name not in ("sx_version", "sx_mlp_param_count", "sx_mlp_bf16_count",
-                                                     "sx_jacobi_sweep_variants", "sx_jacobi_sweep_packed_forms",
-                                                     "sx_jacobi_sweep_default_variant",
-                                                     "sx_contact_pairs_project_variants",
-                                                     "sx_contact_pairs_project_variant_pipelined",
-                                                     "sx_batched_substep_variants",
-                                                     "sx_batched_substep_variant_cluster"):
-            return lambda *a: _call(name, *a)
-        return getattr(load(), name)
+        L = load()
+        fn = getattr(L, name)
+        if SIGNATURES[name][1] is I and name not in _VALUES:
+            raw = fn
+
+            def fn(*args):
+                rc = raw(*args)
+                if rc != SX_OK:
+                    raise SxError(name, rc, L.sx_last_error().decode(errors="replace"))
+                return rc
+
+        setattr(self, name, fn)
+        return fn
 
 
 sx = _Calls()

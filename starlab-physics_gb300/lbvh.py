@@ -95,12 +95,14 @@ class LBVH_CELL:
                              ptr(self.num_faces), ptr(self.node_min4), ptr(self.node_max4), ptr(self.face_rec8),
                              ptr(self.grid8), ptr(self.workspace), self.workspace.numel(), stream_handle())
 
-    def traverse(self, points4, padding: float, cap: int, cand, num, status, n_queries=None):
-        """``traverse_cell_bvh_single`` for boxes ``points4[i] +- padding``."""
+    def traverse(self, points4, padding: float, cap: int, cand, num, status, n_queries=None, stream=None):
+        """``traverse_cell_bvh_single`` for boxes ``points4[i] +- padding`` (on
+        ``stream``, the current one by default)."""
         q = points4.shape[0] if n_queries is None else n_queries
         sx.sx_cell_bvh_traverse(ptr(points4), q, float(padding), ptr(self.grid8), ptr(self.box6),
                                 ptr(self.node_min4), ptr(self.node_max4), ptr(self.prefix_sum_cell),
-                                ptr(self.face_rec8), int(cap), ptr(cand), ptr(num), ptr(status), stream_handle())
+                                ptr(self.face_rec8), int(cap), ptr(cand), ptr(num), ptr(status),
+                                stream_handle(stream))
 
     def traverse_edges(self, edge_indices, n_edges: int, points4, padding: float, cap: int, cand, num, status):
         """``traverse_cell_bvh_single`` for edge boxes: min / max of each edge's

@@ -132,8 +132,11 @@ class Solver:
         # compute_y and the first sweep, the three query sets beside each other
         self.concurrent_broadphase = True
         self._bvh_join = None  # side stream of a BVH build the broad phase must wait for
-        self._bp_streams = ((torch.cuda.Stream(device=mesh_dy.device), torch.cuda.Stream(device=mesh_dy.device))
-                            if torch.device(mesh_dy.device).type == "cuda" else None)
+        self._bp_streams = self._bp_events = None
+        if torch.device(mesh_dy.device).type == "cuda":
+            self._bp_streams = (torch.cuda.Stream(device=mesh_dy.device), torch.cuda.Stream(device=mesh_dy.device))
+            # fork and joins, recorded anew before every wait
+            self._bp_events = tuple(torch.cuda.Event() for _ in range(3))
 
         self.max_num_verts_dy = mesh_dy.num_verts
         self.max_num_edges_dy = mesh_dy.num_edges
@@ -299,27 +302,30 @@ class Solver:
         query set (parallel branches in a captured frame)."""
         m = self.mesh_dy
         cap = self.cache_size
-        cur = torch.cuda.current_stream(self.device)
         side = self.concurrent_broadphase and self.mesh_st is not None and self._bp_streams is not None
+        s1 = s2 = None
         if side:
             s1, s2 = self._bp_streams
-            s1.wait_stream(cur)
-            s2.wait_stream(cur)
+            cur = torch.cuda.current_stream(self.device)
+            fork, join1, join2 = self._bp_events
+            fork.record(cur)
+            s1.wait_event(fork)
+            s2.wait_event(fork)
         if self.mesh_st is not None:
-            with torch.cuda.stream(s1 if side else cur):
-                self.lbvh_st.traverse(m.y4, self.padding, cap, self.vt_st_candidates, self.vt_st_candidates_num,
-                                      self.status)
-            with torch.cuda.stream(s2 if side else cur):
-                self.lbvh_dy.traverse(self.mesh_st.x4, self.padding, cap, self.tv_st_candidates,
-                                      self.tv_st_candidates_num, self.status)
+            self.lbvh_st.traverse(m.y4, self.padding, cap, self.vt_st_candidates, self.vt_st_candidates_num,
+                                  self.status, stream=s1)
+            self.lbvh_dy.traverse(self.mesh_st.x4, self.padding, cap, self.tv_st_candidates,
+                                  self.tv_st_candidates_num, self.status, stream=s2)
         if self.self_collision:
             self.lbvh_dy.traverse(m.y4, self.padding, cap, self.vt_dy_candidates, self.vt_dy_candidates_num,
                                   self.status)
         else:
             self.vt_dy_candidates_num.zero_()
         if side:
-            cur.wait_stream(s1)
-            cur.wait_stream(s2)
+            join1.record(s1)
+            join2.record(s2)
+            cur.wait_event(join1)
+            cur.wait_event(join2)
         if self.enable_edge_edge:
             ee = self._ensure_ee()
             cap = self.cache_size
