@@ -284,6 +284,9 @@ int sx_face_morton(const float* fmin4, const float* fmax4, int n_faces, const fl
 size_t sx_radix_sort_workspace_bytes(int n);
 int sx_radix_sort_pairs(unsigned* keys, int* vals, int n, int bits, void* ws, size_t ws_bytes, void* stream);
 
+/* sx_radix_sort_pairs by the key bits first_bit .. first_bit + bits - 1 alone. */
+int sx_radix_sort_pairs_bits(unsigned* keys, int* vals, int n, int first_bit, int bits, void* ws, size_t ws_bytes,
+                             void* stream);
 /* The same sort for callers that cannot allocate device memory when they
  * sort -- e.g. hosts whose device memory belongs to another allocator with a
  * fixed budget, or real-time loops that cannot take the synchronisation a
@@ -335,6 +338,20 @@ int sx_face_bvh_traverse(int n, const float* p4, int n_queries, float padding, c
 int sx_face_bvh_traverse_ordered(int n, const float* p4, int n_queries, float padding, const int* child_a,
                                  const int* child_b, const int* sorted_ids, const float* nmin4, const float* nmax4,
                                  int cap, int* cand, int* num, int* status, const int* order, void* stream);
+
+/* sx_face_bvh_refit_ranges: the same node boxes as sx_face_bvh_refit_tiled on a
+ * well-formed hierarchy (tie = 1), taken as unions over the nodes' ranges of
+ * leaves, and the child records that sx_face_bvh_query reads; aux:
+ * sx_face_bvh_aux_bytes bytes, 16-byte aligned.  sx_face_bvh_query reports the
+ * same candidates in the same order as sx_face_bvh_traverse on that hierarchy,
+ * visiting the queries in the order `order` (NULL: 0 .. n_queries - 1). */
+size_t sx_face_bvh_aux_bytes(int n);
+int sx_face_bvh_refit_ranges(int n, const int* sorted_ids, const float* fmin4, const float* fmax4, const int* range_l,
+                             const int* range_r, const int* parent, float* nmin4, float* nmax4, float* aux,
+                             size_t aux_bytes, void* stream);
+int sx_face_bvh_query(int n, const float* p4, int n_queries, float padding, const int* sorted_ids, const float* nmin4,
+                      const float* nmax4, const float* aux, int cap, int* cand, int* num, int* status,
+                      const int* order, void* stream);
 
 /* ---- narrow phase + contact projection ------------------------------------ */
 

@@ -80,10 +80,14 @@ SIGNATURES = {
     "sx_face_morton": ([P, P, I, P, P, P, P], I),
     "sx_radix_sort_workspace_bytes": ([I], Z),
     "sx_radix_sort_pairs": ([P, P, I, I, P, Z, P], I),
+    "sx_radix_sort_pairs_bits": ([P, P, I, I, I, P, Z, P], I),
     "sx_radix_sort_pairs_noalloc": ([P, P, I, I, P], I),
     "sx_karras_build": ([P, I, I, P, P, P, P, P, P], I),
     "sx_face_bvh_refit": ([I, P, P, P, P, P, P, P, P, P, P, P], I),
     "sx_face_bvh_refit_tiled": ([I, P, P, P, P, P, P, P, P, P, P, P, P, P], I),
+    "sx_face_bvh_aux_bytes": ([I], Z),
+    "sx_face_bvh_refit_ranges": ([I, P, P, P, P, P, P, P, P, P, Z, P], I),
+    "sx_face_bvh_query": ([I, P, I, F, P, P, P, P, I, P, P, P, P, P], I),
     "sx_face_bvh_traverse": ([I, P, I, F, P, P, P, P, P, I, P, P, P, P], I),
     "sx_face_bvh_traverse_ordered": ([I, P, I, F, P, P, P, P, P, I, P, P, P, P, P], I),
     "sx_collision_sweep": ([I, I, P, P, P, P, P, P, F, F, I, P, P, P, P, P, P, P, P, P, P, P, P, P, P], I),

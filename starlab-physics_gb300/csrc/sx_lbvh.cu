@@ -307,8 +307,9 @@ static size_t rs_ws_bytes(int n) {
     return align256(nn * 4) * 2 + align256((size_t)256 * rs_nblocks(n) * 4) + align256(256 * 4);
 }
 
-static int radix_sort(unsigned* keys, int* vals, int n, int bits, void* ws, size_t ws_bytes, cudaStream_t s) {
-    SX_REQUIRE(bits >= 1 && bits <= 32, "radix sort: bits must be in [1, 32]");
+static int radix_sort(unsigned* keys, int* vals, int n, int bits, void* ws, size_t ws_bytes, cudaStream_t s,
+                      int first = 0) {
+    SX_REQUIRE(bits >= 1 && first >= 0 && first + bits <= 32, "radix sort: bits must be in [1, 32]");
     if (n <= 1) return SX_OK;
     SX_REQUIRE(ws && ws_bytes >= rs_ws_bytes(n), "radix sort: workspace too small (%zu < %zu)", ws_bytes,
                rs_ws_bytes(n));
@@ -327,10 +328,10 @@ static int radix_sort(unsigned* keys, int* vals, int n, int bits, void* ws, size
     unsigned* ko = kalt;
     int* vo = valt;
     for (int pass = 0; pass < passes; ++pass) {
-        const int shift = 8 * pass;
-        // the last digit keeps only the key bits below `bits`: keys are ordered
-        // by their low `bits` bits, higher bits ride along unsorted
-        const int width = bits - shift < 8 ? bits - shift : 8;
+        const int shift = first + 8 * pass;
+        // the last digit keeps only the key bits below `first + bits`: the other
+        // bits ride along unsorted
+        const int width = bits - 8 * pass < 8 ? bits - 8 * pass : 8;
         const unsigned dmask = (1u << width) - 1u;
         launch(rs_upsweep, nb, RS_BLOCK, 0, s, ki, n, shift, dmask, hist, nb);
         launch(rs_digit_scan, 256, RS_BLOCK, 0, s, hist, nb, tot);
@@ -886,6 +887,252 @@ __global__ void __launch_bounds__(FR_TILE) face_refit_tiled_kernel(
     }
 }
 
+// ---------------------------------------------------------------------------
+// Refit by ranges, and child records for the queries.
+//
+// Entry e of level k >= 1 is the union of the sorted leaves 8^k e .. 8^k (e + 1)
+// - 1, {min, max} in 32 bytes; a level is padded with empty boxes to whole
+// groups of 8 and the last one is a single group.  A Karras node covers a
+// contiguous range of leaves, so its box is the union of at most 7 + 7 entries
+// per level: no climb, whose last 20-25 levels are two dependent round trips
+// each (101 us for 2^20 leaves, without the records below; this takes 81, for
+// 20 011 leaves 27 -> 11).  Min and max are exact, so the boxes are the
+// climb's bit for bit.
+//
+// Record i holds both children of internal node i, {min, id}, {max, -} each, the
+// id an internal node's index or ~face: a query reads one line per node in one
+// round trip instead of the two child indices and then four boxes from four
+// places.  Every node writes its own half of its parent's record.
+// ---------------------------------------------------------------------------
+constexpr int LV_MAX = 12;  // 8^11 > 2^31
+struct LevelTable {
+    int top;               // level of the single group
+    long long off[LV_MAX]; // first entry of level k >= 1
+    int count[LV_MAX];     // entries of level k without padding
+};
+static LevelTable level_table(int n) {
+    LevelTable t = {};
+    t.count[0] = n;
+    long long at = 0;
+    int k = 0;
+    while (t.count[k] > 8) {
+        t.count[k + 1] = (int)((t.count[k] + 7LL) / 8);
+        t.off[k + 1] = at;
+        at += (t.count[k + 1] + 7LL) / 8 * 8;
+        ++k;
+    }
+    t.top = k;
+    return t;
+}
+static long long level_entries(int n) {
+    const LevelTable t = level_table(n);
+    return t.top == 0 ? 0 : t.off[t.top] + 8;
+}
+__device__ __forceinline__ void put_child(float4* rec, int parent, bool right, V3 a, V3 b, int id) {
+    float4* r = rec + 4 * (size_t)parent + (right ? 2 : 0);
+    r[0] = make_float4(a.x, a.y, a.z, __int_as_float(id));
+    r[1] = make_float4(b.x, b.y, b.z, 0.0f);
+}
+
+__device__ __forceinline__ void join_lanes(V3& a, V3& b, int width) {
+    for (int o = 1; o < width; o <<= 1) {
+        a = vmin(a, V3{__shfl_xor_sync(0xffffffffu, a.x, o), __shfl_xor_sync(0xffffffffu, a.y, o),
+                       __shfl_xor_sync(0xffffffffu, a.z, o)});
+        b = vmax(b, V3{__shfl_xor_sync(0xffffffffu, b.x, o), __shfl_xor_sync(0xffffffffu, b.y, o),
+                       __shfl_xor_sync(0xffffffffu, b.z, o)});
+    }
+}
+__device__ __forceinline__ void put_entry(float4* lv, long long e, V3 a, V3 b) {
+    lv[2 * e] = make_float4(a.x, a.y, a.z, 0.0f);
+    lv[2 * e + 1] = make_float4(b.x, b.y, b.z, 0.0f);
+}
+
+// Leaf boxes in sorted order and levels 1 and 2 (a block covers 256 leaves: 32
+// entries of level 1, 4 of level 2).
+__device__ __forceinline__ void join_box(V3& a, V3& b, float4 lo, float4 hi) {
+    a = vmin(a, mk(lo));
+    b = vmax(b, mk(hi));
+}
+__global__ void __launch_bounds__(256) face_leaves_kernel(int n, const int* __restrict__ sorted_ids,
+                                                          const float4* __restrict__ fmn4,
+                                                          const float4* __restrict__ fmx4,
+                                                          const int* __restrict__ parent,
+                                                          const int* __restrict__ range_l,
+                                                          float4* __restrict__ nmin4, float4* __restrict__ nmax4,
+                                                          float4* __restrict__ lv, float4* __restrict__ rec,
+                                                          LevelTable t) {
+    pdl_entry();
+    const int j = blockIdx.x * 256 + threadIdx.x, lane = threadIdx.x & 31;
+    V3 a{INFINITY, INFINITY, INFINITY}, b{-INFINITY, -INFINITY, -INFINITY};
+    if (j < n) {
+        const int f = sorted_ids[j];
+        const float4 lo = fmn4[f], hi = fmx4[f];
+        nmin4[n - 1 + j] = lo;
+        nmax4[n - 1 + j] = hi;
+        a = mk(lo);
+        b = mk(hi);
+        if (n > 1) {
+            const int p = parent[n - 1 + j];
+            put_child(rec, p, range_l[p] != j, a, b, ~f);
+        }
+    }
+    if (t.top < 1) return;
+    join_lanes(a, b, 8);
+    const int e1 = j >> 3;
+    const bool own = (lane & 7) == 0;
+    if (own && e1 < (t.count[1] + 7) / 8 * 8) put_entry(lv, t.off[1] + e1, a, b);
+    if (t.top < 2) return;
+    __shared__ V3 sa[32], sb[32];
+    if (own) {
+        sa[threadIdx.x >> 3] = a;
+        sb[threadIdx.x >> 3] = b;
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        a = sa[threadIdx.x];
+        b = sb[threadIdx.x];
+        join_lanes(a, b, 8);
+        const int e2 = blockIdx.x * 4 + (lane >> 3);
+        if (own && e2 < (t.count[2] + 7) / 8 * 8) put_entry(lv, t.off[2] + e2, a, b);
+    }
+}
+
+// Level k from level k - 1, 8 lanes per entry, padding included; the last
+// blocks' padding of level k - 1 holds empty boxes already.
+__global__ void __launch_bounds__(256) face_level_kernel(float4* lv, LevelTable t, int k) {
+    pdl_entry();
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x, e = i >> 3;
+    const long long padded = (t.count[k] + 7) / 8 * 8;
+    V3 a{INFINITY, INFINITY, INFINITY}, b{-INFINITY, -INFINITY, -INFINITY};
+    if (i < t.count[k - 1]) {
+        a = mk(lv[2 * (t.off[k - 1] + i)]);
+        b = mk(lv[2 * (t.off[k - 1] + i) + 1]);
+    }
+    join_lanes(a, b, 8);
+    if ((threadIdx.x & 7) == 0 && e < padded) put_entry(lv, t.off[k] + e, a, b);
+}
+
+// Levels k0 .. top in one block.
+__global__ void __launch_bounds__(1024) face_top_levels_kernel(float4* lv, LevelTable t, int k0) {
+    pdl_entry();
+    for (int k = k0; k <= t.top; ++k) {
+        const int padded = (t.count[k] + 7) / 8 * 8;
+        for (int i0 = 0; i0 < 8 * padded; i0 += 1024) {
+            const int i = i0 + threadIdx.x;
+            V3 a{INFINITY, INFINITY, INFINITY}, b{-INFINITY, -INFINITY, -INFINITY};
+            if (i < t.count[k - 1]) {
+                a = mk(lv[2 * (t.off[k - 1] + i)]);
+                b = mk(lv[2 * (t.off[k - 1] + i) + 1]);
+            }
+            join_lanes(a, b, 8);
+            if ((threadIdx.x & 7) == 0 && i < 8 * padded) put_entry(lv, t.off[k] + (i >> 3), a, b);
+        }
+        __syncthreads();
+    }
+}
+
+// Internal node i: the union over its range of leaves.  (Nodes inside a block's
+// 256 leaves taken from shared memory in the leaf kernel instead: 88 against 81
+// us for the whole refit of 2^20 leaves.)
+__global__ void __launch_bounds__(256) face_ranges_kernel(int n, const int* __restrict__ range_l,
+                                                          const int* __restrict__ range_r,
+                                                          const int* __restrict__ parent, float4* nmin4,
+                                                          float4* nmax4, const float4* __restrict__ lv,
+                                                          float4* __restrict__ rec, LevelTable t) {
+    pdl_entry();
+    __shared__ long long off[LV_MAX];
+    if (threadIdx.x < LV_MAX) off[threadIdx.x] = t.off[threadIdx.x];
+    __syncthreads();
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= n - 1) return;
+    const int l = range_l[i], r = range_r[i];
+    V3 a{NAN, NAN, NAN}, b{NAN, NAN, NAN};  // fminf and fmaxf pass over a NaN
+    int lo = l, hi = r + 1;  // [lo, hi)
+    const float4 *mn = nmin4 + (n - 1), *mx = nmax4 + (n - 1);
+    int step = 1;
+    for (int k = 0;; ++k) {
+        const int l1 = k == t.top ? hi : min((lo + 7) & ~7, hi), h0 = max(hi & ~7, l1);
+        for (int e = lo; e < l1; ++e) join_box(a, b, mn[(size_t)e * step], mx[(size_t)e * step]);
+        for (int e = h0; e < hi; ++e) join_box(a, b, mn[(size_t)e * step], mx[(size_t)e * step]);
+        if (l1 >= h0) break;
+        lo = l1 >> 3;
+        hi = h0 >> 3;
+        mn = lv + 2 * off[k + 1];
+        mx = mn + 1;
+        step = 2;
+    }
+    store_box(nmin4, nmax4, i, a, b);
+    if (i > 0) put_child(rec, parent[i], l == i, a, b, i);  // a right child carries its first leaf's index
+}
+
+// face_traverse_kernel over the child records: the same visiting order (right
+// child first), so the same candidates in the same order.  A leaf that is next
+// in that order is reported where its parent is tested, without a push and a pop.
+__global__ void __launch_bounds__(128) face_query_kernel(int n, int Q, const float4* __restrict__ p4, float pad,
+                                                         const int* __restrict__ sorted_ids,
+                                                         const float4* __restrict__ nmin4,
+                                                         const float4* __restrict__ nmax4,
+                                                         const float4* __restrict__ rec, int cap,
+                                                         int* __restrict__ cand, int* __restrict__ num, int* status,
+                                                         const int* __restrict__ order) {
+    pdl_entry();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= Q) return;
+    const int q = order ? order[i] : i;
+    const V3 p = mk(p4[q]);
+    const V3 a{p.x - pad, p.y - pad, p.z - pad}, b{p.x + pad, p.y + pad, p.z + pad};
+    int count = 0, flags = 0;
+    int* out = cand + (size_t)q * cap;
+    auto report = [&](int face) {
+        if (count < cap) out[count] = face;
+        ++count;
+    };
+    int stack[64];
+    int sc = 0;
+    if (n == 1) {
+        if (overlap(a, b, mk(nmin4[0]), mk(nmax4[0]))) report(sorted_ids[0]);
+    } else {
+        int cur = 0;
+        for (long long visits = 0;; ++visits) {
+            if (visits > 2LL * n) {  // each node is visited at most once
+                flags |= SX_STATUS_STACK_OVERFLOW;
+                break;
+            }
+            const float4* r4 = rec + 4 * (size_t)cur;
+            const float4 la = r4[0], lb = r4[1], ra = r4[2], rb = r4[3];
+            bool hl = overlap(a, b, mk(la), mk(lb)), hr = overlap(a, b, mk(ra), mk(rb));
+            const int l = __float_as_int(la.w), r = __float_as_int(ra.w);
+            if (hr && r < 0) {
+                report(~r);
+                hr = false;
+            }
+            if (hl && l < 0 && !hr) {
+                report(~l);
+                hl = false;
+            }
+            if (hr) {
+                if (hl) {
+                    if (sc < 64) stack[sc++] = l; else flags |= SX_STATUS_STACK_OVERFLOW;
+                }
+                cur = r;
+            } else if (hl) {
+                cur = l;
+            } else {
+                cur = -1;
+                while (sc > 0) {
+                    cur = stack[--sc];
+                    if (cur >= 0) break;
+                    report(~cur);
+                }
+                if (cur < 0) break;
+            }
+        }
+    }
+    num[q] = count;
+    if (count > cap) flags |= SX_STATUS_CAND_OVERFLOW;
+    if (flags) atomicOr(status, flags);
+}
+
 __global__ void __launch_bounds__(128) face_traverse_kernel(int n, int Q, const float4* __restrict__ p4, float pad,
                                                             const int* __restrict__ child_a,
                                                             const int* __restrict__ child_b,
@@ -959,6 +1206,14 @@ extern "C" int sx_radix_sort_pairs(unsigned* keys, int* vals, int n, int bits, v
     if (n <= 1) return SX_OK;
     SX_REQUIRE(keys && vals, "sx_radix_sort_pairs: null pointer");
     return radix_sort(keys, vals, n, bits, ws, ws_bytes, as_stream(stream));
+}
+
+extern "C" int sx_radix_sort_pairs_bits(unsigned* keys, int* vals, int n, int first_bit, int bits, void* ws,
+                                        size_t ws_bytes, void* stream) {
+    SX_REQUIRE(n >= 0, "sx_radix_sort_pairs_bits: n < 0");
+    if (n <= 1) return SX_OK;
+    SX_REQUIRE(keys && vals, "sx_radix_sort_pairs_bits: null pointer");
+    return radix_sort(keys, vals, n, bits, ws, ws_bytes, as_stream(stream), first_bit);
 }
 
 // ---------------------------------------------------------------------------
@@ -1155,6 +1410,49 @@ extern "C" int sx_face_bvh_refit_tiled(int n, const int* sorted_ids, const float
            (const float4*)fmin4, (const float4*)fmax4, child_a, child_b, parent, range_l, range_r, (float4*)nmin4,
            (float4*)nmax4, flags, status);
     return check_launch("face_refit_tiled_kernel");
+}
+
+// aux: [level entries, 32 bytes each][n - 1 child records of 64 bytes]
+extern "C" size_t sx_face_bvh_aux_bytes(int n) {
+    return n < 1 ? 0 : (size_t)level_entries(n) * 32 + (size_t)n * 64;
+}
+
+extern "C" int sx_face_bvh_refit_ranges(int n, const int* sorted_ids, const float* fmin4, const float* fmax4,
+                                        const int* range_l, const int* range_r, const int* parent, float* nmin4,
+                                        float* nmax4, float* aux, size_t aux_bytes, void* stream) {
+    SX_REQUIRE(n >= 1, "sx_face_bvh_refit_ranges: n must be >= 1");
+    SX_REQUIRE(sorted_ids && fmin4 && fmax4 && nmin4 && nmax4 && aux && (n == 1 || (range_l && range_r && parent)),
+               "sx_face_bvh_refit_ranges: null pointer");
+    SX_REQUIRE(((uintptr_t)aux & 15) == 0 && aux_bytes >= sx_face_bvh_aux_bytes(n),
+               "sx_face_bvh_refit_ranges: aux must be 16-byte aligned and sx_face_bvh_aux_bytes long");
+    cudaStream_t s = as_stream(stream);
+    const LevelTable t = level_table(n);
+    float4 *lv = (float4*)aux, *rec = lv + 2 * level_entries(n);
+    // blocks up to the padded end of level 1 (2), so that the padding gets written
+    const long long cover =
+        t.top < 1 ? n : t.top < 2 ? (t.count[1] + 7LL) / 8 * 64 : (t.count[2] + 7LL) / 8 * 512;
+    launch(face_leaves_kernel, grid_for(cover, 256), 256, 0, s, n, sorted_ids, (const float4*)fmin4,
+           (const float4*)fmax4, parent, range_l, (float4*)nmin4, (float4*)nmax4, lv, rec, t);
+    int k = 3;
+    for (; k <= t.top && t.count[k - 1] > 4096; ++k)
+        launch(face_level_kernel, grid_for((t.count[k] + 7LL) / 8 * 64, 256), 256, 0, s, lv, t, k);
+    if (k <= t.top) launch(face_top_levels_kernel, 1, 1024, 0, s, lv, t, k);
+    if (n > 1)
+        launch(face_ranges_kernel, grid_for(n - 1, 256), 256, 0, s, n, range_l, range_r, parent, (float4*)nmin4,
+               (float4*)nmax4, (const float4*)lv, rec, t);
+    return check_launch("sx_face_bvh_refit_ranges");
+}
+
+extern "C" int sx_face_bvh_query(int n, const float* p4, int n_queries, float padding, const int* sorted_ids,
+                                 const float* nmin4, const float* nmax4, const float* aux, int cap, int* cand,
+                                 int* num, int* status, const int* order, void* stream) {
+    SX_REQUIRE(n >= 1 && n_queries >= 0 && cap >= 1, "sx_face_bvh_query: bad sizes");
+    if (n_queries == 0) return SX_OK;
+    SX_REQUIRE(p4 && sorted_ids && nmin4 && nmax4 && aux && cand && num && status, "sx_face_bvh_query: null pointer");
+    launch(face_query_kernel, grid_for(n_queries, 128), 128, 0, as_stream(stream), n, n_queries, (const float4*)p4,
+           padding, sorted_ids, (const float4*)nmin4, (const float4*)nmax4,
+           (const float4*)aux + 2 * level_entries(n), cap, cand, num, status, order);
+    return check_launch("face_query_kernel");
 }
 
 extern "C" int sx_face_bvh_traverse(int n, const float* p4, int n_queries, float padding, const int* child_a,
