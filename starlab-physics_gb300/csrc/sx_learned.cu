@@ -19,6 +19,7 @@
 #include <cuda_bf16.h>
 
 #include "sx_common.cuh"
+#include "sx_exact.cuh"
 
 namespace sx {
 
@@ -34,8 +35,11 @@ __device__ __forceinline__ unsigned short f2bf(float f) {
     return __bfloat16_as_ushort(__float2bfloat16_rn(f));
 }
 __device__ __forceinline__ float bf2f(unsigned short u) { return __bfloat162float(__ushort_as_bfloat16(u)); }
+// one packed conversion: the scalar ones run on the special-function unit
 __device__ __forceinline__ unsigned pack_bf2(float lo, float hi) {
-    return (unsigned)f2bf(lo) | ((unsigned)f2bf(hi) << 16);
+    unsigned d;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
+    return d;
 }
 
 // D += A(16x16, row) * B(16x8, col), BF16 inputs, FP32 accumulate.
@@ -54,9 +58,15 @@ __device__ __forceinline__ void ldsm_x4_trans(unsigned (&r)[4], const void* p) {
                  : "r"(a));
 }
 
-__device__ __forceinline__ float silu(float z) { return z / (1.0f + expf(-z)); }
+// z / (1 + exp(-z)) and the derivative s + z s (1 - s), s = 1 / (1 + exp(-z)),
+// with correctly rounded quotients (straight-line, sx_exact.cuh; the exponent is
+// capped where s is below 2^-99 and of no consequence).
+__device__ __forceinline__ float silu(float z) {
+    const float d = 1.0f + expf(fminf(-z, 69.0f));
+    return div_rn(z, d, rcp_rn(d));
+}
 __device__ __forceinline__ float silu_grad(float z) {
-    const float s = 1.0f / (1.0f + expf(-z));
+    const float s = rcp_rn(1.0f + expf(fminf(-z, 69.0f)));
     return s + z * (s * (1.0f - s));
 }
 
@@ -196,40 +206,40 @@ __global__ void warm_select_kernel(int V, const double* __restrict__ res_warm, c
 // ---------------------------------------------------------------------------
 // MLP tiles.  A warp owns 16 rows.  Shared weights (BF16, rows padded so that
 // the fragment loads are bank-conflict free):
-//   W1s[64][40] (n, k), W2s[64][72] (n, k), W3s[8][72] (n, k),
-//   W2t[64][72] (k, n) and W3t[64][24] (k, n) for the backward data path.
+//   W1s[64][40] (n, k), W2s[64][72] (n, k), W3s[8][72] (n, k);
+// the backward data path reads W2 and W3 transposed by ldmatrix.trans.
 // ---------------------------------------------------------------------------
-constexpr int S1 = 40, S2 = 72, S3 = 72, S2T = 72, S3T = 24;
+constexpr int S1 = 40, S2 = 72, S3 = 72;
 
 struct MlpSmem {
-    unsigned short W1[kHid * S1];
-    unsigned short W2[kHid * S2];
-    unsigned short W3[kOut * S3];
+    alignas(16) unsigned short W1[kHid * S1];
+    alignas(16) unsigned short W2[kHid * S2];
+    alignas(16) unsigned short W3[kOut * S3];
     float b1[kHid], b2[kHid], b3[kOut];
 };
-struct MlpSmemT {
-    unsigned short W2t[kHid * S2T];
-    unsigned short W3t[kHid * S3T];
-};
-
+// rows of K values to rows of the padded stride, 16 bytes at a time where the
+// source allows it
+__device__ __forceinline__ void stage_rows(unsigned short* dst, int stride, const unsigned short* __restrict__ src,
+                                           int rows, int K, bool wide) {
+    if (wide) {
+        for (int i = threadIdx.x; i < rows * (K / 8); i += blockDim.x) {
+            const int n = i / (K / 8), k = i % (K / 8) * 8;
+            *reinterpret_cast<uint4*>(dst + n * stride + k) = *reinterpret_cast<const uint4*>(src + n * K + k);
+        }
+    } else {
+        for (int i = threadIdx.x; i < rows * K; i += blockDim.x) dst[i / K * stride + i % K] = src[i];
+    }
+}
 __device__ void stage_weights(MlpSmem& s, const unsigned short* __restrict__ w16, const float* __restrict__ p32) {
-    for (int i = threadIdx.x; i < kHid * kFeat; i += blockDim.x) s.W1[(i / kFeat) * S1 + i % kFeat] = w16[qW1 + i];
-    for (int i = threadIdx.x; i < kHid * kHid; i += blockDim.x) s.W2[(i / kHid) * S2 + i % kHid] = w16[qW2 + i];
-    for (int i = threadIdx.x; i < kOut * kHid; i += blockDim.x) s.W3[(i / kHid) * S3 + i % kHid] = w16[qW3 + i];
+    const bool wide = (reinterpret_cast<uintptr_t>(w16) & 15) == 0;
+    stage_rows(s.W1, S1, w16 + qW1, kHid, kFeat, wide);
+    stage_rows(s.W2, S2, w16 + qW2, kHid, kHid, wide);
+    stage_rows(s.W3, S3, w16 + qW3, kOut, kHid, wide);
     for (int i = threadIdx.x; i < kHid; i += blockDim.x) {
         s.b1[i] = p32[ob1 + i];
         s.b2[i] = p32[ob2 + i];
     }
     if (threadIdx.x < kOut) s.b3[threadIdx.x] = p32[ob3 + threadIdx.x];
-}
-
-__device__ void stage_weights_t(MlpSmemT& t, const unsigned short* __restrict__ w16) {
-    // W2t[k = in][n = out] = W2[n][k]; W3t[k = hidden][n = out] = W3[n][k]
-    for (int i = threadIdx.x; i < kHid * kHid; i += blockDim.x) t.W2t[(i % kHid) * S2T + i / kHid] = w16[qW2 + i];
-    for (int i = threadIdx.x; i < kHid * S3T; i += blockDim.x) {
-        const int k = i / S3T, n = i % S3T;
-        t.W3t[i] = n < kOut ? w16[qW3 + n * kHid + k] : (unsigned short)0;
-    }
 }
 
 __device__ __forceinline__ unsigned lds32(const unsigned short* p) { return *reinterpret_cast<const unsigned*>(p); }
@@ -241,8 +251,11 @@ struct Frag64 {
     float c[8][4];
 };
 
+// keep(layer, ks, a): the activations of hidden layer 1 or 2 as A fragments
+// (rows g, g + 8 of columns 16 ks + 2 tig, then the same 8 columns on).
+template <typename Keep>
 __device__ __forceinline__ void tile_forward(const MlpSmem& s, const unsigned (&ax)[2][4], Frag64& z1, Frag64& z2,
-                                             float (&o)[4]) {
+                                             float (&o)[4], Keep keep) {
     const int lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -263,6 +276,7 @@ __device__ __forceinline__ void tile_forward(const MlpSmem& s, const unsigned (&
         ah[ks][1] = pack_bf2(silu(z1.c[2 * ks][2]), silu(z1.c[2 * ks][3]));
         ah[ks][2] = pack_bf2(silu(z1.c[2 * ks + 1][0]), silu(z1.c[2 * ks + 1][1]));
         ah[ks][3] = pack_bf2(silu(z1.c[2 * ks + 1][2]), silu(z1.c[2 * ks + 1][3]));
+        keep(1, ks, ah[ks]);
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -282,6 +296,7 @@ __device__ __forceinline__ void tile_forward(const MlpSmem& s, const unsigned (&
         ah[ks][1] = pack_bf2(silu(z2.c[2 * ks][2]), silu(z2.c[2 * ks][3]));
         ah[ks][2] = pack_bf2(silu(z2.c[2 * ks + 1][0]), silu(z2.c[2 * ks + 1][1]));
         ah[ks][3] = pack_bf2(silu(z2.c[2 * ks + 1][2]), silu(z2.c[2 * ks + 1][3]));
+        keep(2, ks, ah[ks]);
     }
     o[0] = s.b3[2 * tig]; o[1] = s.b3[2 * tig + 1]; o[2] = o[0]; o[3] = o[1];
 #pragma unroll
@@ -323,7 +338,7 @@ __global__ void __launch_bounds__(MLP_BLOCK) mlp_forward_kernel(int V, const uns
         load_x_frag(feat, ra, rb, ax);
         Frag64 z1, z2;
         float o[4];
-        tile_forward(s, ax, z1, z2, o);
+        tile_forward(s, ax, z1, z2, o, [](int, int, const unsigned(&)[4]) {});
         if (tig < 2) {
             if (ra >= 0) *reinterpret_cast<float2*>(out4 + 4 * (size_t)ra + 2 * tig) = make_float2(o[0], o[1]);
             if (rb >= 0) *reinterpret_cast<float2*>(out4 + 4 * (size_t)rb + 2 * tig) = make_float2(o[2], o[3]);
@@ -341,24 +356,39 @@ __global__ void __launch_bounds__(MLP_BLOCK) mlp_forward_kernel(int V, const uns
 // thread 0 issues tcgen05.mma (kind::f16, BF16 x BF16 -> FP32) into tensor
 // memory, whose completion tcgen05.commit signals on an mbarrier; each warp
 // then reads its 32 rows of the accumulator with tcgen05.ld, adds the bias,
-// applies SiLU, and writes the next layer's BF16 operand.  Layer 3 is N = 16
-// (W3's 8 rows and 8 zero rows); 128 tensor-memory columns per CTA (D1 at 0,
-// D2 at 64, D3 at 0 once D1 is read).  Every wait is bounded (1 s of global time);
-// a wait that gives up sets SX_STATUS_WAIT_TIMEOUT, waits once more (bounded)
-// for the MMAs in flight, frees the tensor memory and ends the kernel.
+// applies SiLU, and writes the next layer's BF16 operand over the last one.
+// Layer 3 is N = 16 (W3's 8 rows and 8 zero rows); one accumulator of 64
+// tensor-memory columns per CTA serves all three layers, each read before the
+// next overwrites it.
+//
+// The special-function unit sets the floor: 128 tanh a row, 16 a clock and SM, 26
+// us for 10^6 rows.  So nothing else may run on it (the scalar float to BF16
+// conversion does; the packed one does not: 77 -> 53 us), and the CTAs of an SM
+// have to keep it fed through each other's waits: one block barrier per layer,
+// the next tile's features loaded a tile ahead, packed two-wide float operations,
+// and waits on the mbarrier's own suspended try_wait.  10^6 rows take 52 us, 8 of
+// them before the first tile's end (97 with two block barriers per layer, a
+// global timer read in every thread's wait, no prefetch and scalar conversions).
+// 4, 5 or 6 CTAs per SM give 53, 52 and 54 us; ex2 and half a reciprocal in the
+// place of tanh 59; plain loads of a row by its own two threads are faster than
+// coalesced ones regrouped in shared memory (52 against 55).
+//
+// Every wait is bounded (TC_TRIES tries, each suspended for up to 10 us); one that
+// gives up sets SX_STATUS_WAIT_TIMEOUT, waits once more (bounded) for the MMAs
+// in flight, frees the tensor memory and ends the kernel.
 // ---------------------------------------------------------------------------
 constexpr int TC_ROWS = 128;
 constexpr int TC_THREADS = 256;  // warp w reads tensor-memory lanes 32 (w % 4).., columns half w / 4
-constexpr int TC_TMEM_COLS = 128;  // D1 at column 0, D2 at 64, D3 at 0 (D1 is read by then)
-constexpr int TC_PAD_SMEM = 12 * 1024;  // with the 39.5 KB static: 4 CTAs per SM fit, 5 do not
+constexpr int TC_TMEM_COLS = 64;   // every layer's accumulator: the last one has been read by then
+constexpr int TC_PER_SM = 5;       // CTAs: 48 registers a thread, 31 KB of shared memory
 
 struct TcSmem {
-    alignas(128) unsigned short A1[TC_ROWS * kFeat];
-    alignas(128) unsigned short A2[TC_ROWS * kHid];
+    alignas(128) unsigned short A[TC_ROWS * kHid];  // features, then hidden activations
     alignas(128) unsigned short B1[kHid * kFeat];
     alignas(128) unsigned short B2[kHid * kHid];
     alignas(128) unsigned short B3[16 * kHid];
-    float b1[kHid], b2[kHid], b3[16];
+    alignas(16) float b1[kHid], b2[kHid];
+    float b3[16];
     alignas(8) unsigned long long bar;
     unsigned tmem_base;
 };
@@ -392,32 +422,22 @@ __device__ __forceinline__ void umma_commit(unsigned bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                  : "memory");
 }
-__device__ __forceinline__ bool mbar_test(unsigned bar, unsigned parity) {
+constexpr int TC_TRIES = 1 << 18;
+// a try suspends the thread until the phase completes or the hint (ns) is over
+__device__ __forceinline__ bool mbar_try(unsigned bar, unsigned parity) {
     unsigned done;
     asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}\n"
         : "=r"(done)
-        : "r"(bar), "r"(parity)
+        : "r"(bar), "r"(parity), "r"(10000u)
         : "memory");
     return done != 0u;
 }
-__device__ __forceinline__ unsigned long long global_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-__device__ bool mbar_wait_bounded(unsigned bar, unsigned parity) {
-    const unsigned long long t0 = global_ns();
-    while (!mbar_test(bar, parity))
-        if (global_ns() - t0 > 1000000000ull) return false;
-    return true;
-}
-__device__ __forceinline__ void tmem_ld32(unsigned taddr, unsigned (&r)[32]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-                 : "r"(taddr)
-                 : "memory");
+__device__ __forceinline__ bool mbar_wait_bounded(unsigned bar, unsigned parity) {
+    for (int k = 0; k < TC_TRIES; ++k)
+        if (mbar_try(bar, parity)) return true;
+    return false;
 }
 __device__ __forceinline__ void tmem_ld16(unsigned taddr, unsigned (&r)[16]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
@@ -425,44 +445,94 @@ __device__ __forceinline__ void tmem_ld16(unsigned taddr, unsigned (&r)[16]) {
                  : "r"(taddr)
                  : "memory");
 }
+__device__ __forceinline__ void tmem_ld4(unsigned taddr, unsigned (&r)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(taddr)
+                 : "memory");
+}
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// Packed float pairs: the same rounding as two scalar operations.
+#define SX_F32X2(name, op)                                                                                    \
+    __device__ __forceinline__ float2 name(float2 a, float2 b) {                                              \
+        float2 d;                                                                                             \
+        asm("{\n\t.reg .b64 x, y, w;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t" op                \
+            " w, x, y;\n\tmov.b64 {%0, %1}, w;\n\t}"                                                         \
+            : "=f"(d.x), "=f"(d.y)                                                                            \
+            : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));                                                        \
+        return d;                                                                                             \
+    }
+SX_F32X2(add2, "add.rn.f32x2")
+SX_F32X2(mul2, "mul.rn.f32x2")
+#undef SX_F32X2
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{\n\t.reg .b64 x, y, z, w;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
+        "fma.rn.f32x2 w, x, y, z;\n\tmov.b64 {%0, %1}, w;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
 // SiLU through the hardware tanh: z * sigmoid(z) = h + h * tanh(h) with
 // h = z / 2, one special-function instruction instead of an exponential and a
-// reciprocal (the epilogue's special-function unit was its limit).  The
-// tensor-core path's hidden activations are rounded to BF16, far coarser than
-// tanh.approx's error.
+// reciprocal.  The tensor-core path's hidden activations are rounded to BF16, far
+// coarser than tanh.approx's error.
 __device__ __forceinline__ float tanh_hw(float x) {
     float y;
     asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ float silu_fast(float z) {
-    const float h = 0.5f * z;
-    return __fmaf_rn(h, tanh_hw(h), h);
+__device__ __forceinline__ float2 silu2(float2 z) {
+    const float2 h = mul2(z, make_float2(0.5f, 0.5f));
+    return fma2(h, make_float2(tanh_hw(h.x), tanh_hw(h.y)), h);
 }
 
 // 32 accumulator columns of this thread's row (at taddr) + bias -> SiLU ->
-// BF16 columns [c0, c0 + 32) of row `row` of A2
-__device__ __forceinline__ void tc_hidden_half(unsigned taddr, const float* bias, unsigned short* A2, int row, int c0) {
-    unsigned r[32];
-    tmem_ld32(taddr, r);
-    tmem_wait_ld();
+// BF16 columns [c0, c0 + 32) of row `row` of A; 16 at a time, which keeps the
+// kernel at 40 registers
+__device__ __forceinline__ void tc_hidden_half(unsigned taddr, const float* bias, unsigned short* A, int row, int c0) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        uint4 v;
-        unsigned* pv = reinterpret_cast<unsigned*>(&v);
+    for (int p = 0; p < 2; ++p) {
+        unsigned r[16];
+        tmem_ld16(taddr + 16 * p, r);
+        const float2* b2 = reinterpret_cast<const float2*>(bias + c0 + 16 * p);
+        tmem_wait_ld();
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int c = 8 * q + 2 * e;
-            pv[e] = pack_bf2(silu_fast(__uint_as_float(r[c]) + bias[c0 + c]),
-                             silu_fast(__uint_as_float(r[c + 1]) + bias[c0 + c + 1]));
+        for (int q = 0; q < 2; ++q) {
+            uint4 v;
+            unsigned* pv = reinterpret_cast<unsigned*>(&v);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int c = 8 * q + 2 * e;
+                const float2 y = silu2(add2(make_float2(__uint_as_float(r[c]), __uint_as_float(r[c + 1])), b2[c / 2]));
+                pv[e] = pack_bf2(y.x, y.y);
+            }
+            *reinterpret_cast<uint4*>(A + canon(row, c0 + 16 * p + 8 * q, kHid)) = v;
         }
-        *reinterpret_cast<uint4*>(A2 + canon(row, c0 + 8 * q, kHid)) = v;
     }
 }
 
-__global__ void __launch_bounds__(TC_THREADS, 1) mlp_forward_tc_kernel(int V, const unsigned short* __restrict__ feat,
+// 8 consecutive k of row n of a weight matrix -> its 16 bytes of the canonical layout
+__device__ __forceinline__ void stage_canon(unsigned short* dst, const unsigned short* __restrict__ src, int rows,
+                                            int zero_from, int K, bool wide) {
+    for (int i = threadIdx.x; i < rows * (K / 8); i += TC_THREADS) {
+        const int n = i / (K / 8), k = i % (K / 8) * 8;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (n < zero_from) {
+            if (wide) {
+                v = *reinterpret_cast<const uint4*>(src + n * K + k);
+            } else {
+                unsigned short* h = reinterpret_cast<unsigned short*>(&v);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) h[j] = src[n * K + k + j];
+            }
+        }
+        *reinterpret_cast<uint4*>(dst + canon(n, k, K)) = v;
+    }
+}
+
+__global__ void __launch_bounds__(TC_THREADS, TC_PER_SM) mlp_forward_tc_kernel(int V, const unsigned short* __restrict__ feat,
                                                                     const unsigned short* __restrict__ w16,
                                                                     const float* __restrict__ p32,
                                                                     float* __restrict__ out4, int* status) {
@@ -471,12 +541,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) mlp_forward_tc_kernel(int V, co
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int quad = warp & 3, half = warp >> 2;
     const int trow = 32 * quad + lane;  // this thread's row within a tile
-    for (int i = tid; i < kHid * kFeat; i += TC_THREADS) s.B1[canon(i / kFeat, i % kFeat, kFeat)] = w16[qW1 + i];
-    for (int i = tid; i < kHid * kHid; i += TC_THREADS) s.B2[canon(i / kHid, i % kHid, kHid)] = w16[qW2 + i];
-    for (int i = tid; i < 16 * kHid; i += TC_THREADS) {
-        const int n = i / kHid, k = i % kHid;
-        s.B3[canon(n, k, kHid)] = n < kOut ? w16[qW3 + n * kHid + k] : (unsigned short)0;
-    }
+    const bool wide = (reinterpret_cast<uintptr_t>(w16) & 15) == 0;
+    stage_canon(s.B1, w16 + qW1, kHid, kHid, kFeat, wide);
+    stage_canon(s.B2, w16 + qW2, kHid, kHid, kHid, wide);
+    stage_canon(s.B3, w16 + qW3, 16, kOut, kHid, wide);
     for (int i = tid; i < kHid; i += TC_THREADS) {
         s.b1[i] = p32[ob1 + i];
         s.b2[i] = p32[ob2 + i];
@@ -499,78 +567,85 @@ __global__ void __launch_bounds__(TC_THREADS, 1) mlp_forward_tc_kernel(int V, co
     const unsigned long long dB1 = umma_sdesc(smem_u32(s.B1), 128, 512);
     const unsigned long long dB2 = umma_sdesc(smem_u32(s.B2), 128, 1024);
     const unsigned long long dB3 = umma_sdesc(smem_u32(s.B3), 128, 1024);
-    const unsigned long long dA1 = umma_sdesc(smem_u32(s.A1), 128, 512);
-    const unsigned long long dA2 = umma_sdesc(smem_u32(s.A2), 128, 1024);
+    const unsigned long long dA1 = umma_sdesc(smem_u32(s.A), 128, 512);
+    const unsigned long long dA2 = umma_sdesc(smem_u32(s.A), 128, 1024);
     constexpr unsigned id64 = umma_idesc_bf16(TC_ROWS, kHid), id16 = umma_idesc_bf16(TC_ROWS, 16);
     unsigned phase = 0;
     bool ok = true;
-    const int ntiles = (V + TC_ROWS - 1) / TC_ROWS;
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int row = tile * TC_ROWS + trow;
-        // layer 1: features (BF16, 32 columns; half a row per thread) -> A1
-        uint4 f[2];
+    const long long ntiles = ((long long)V + TC_ROWS - 1) / TC_ROWS;
+    // half a row of features (16 BF16) per thread
+    uint4 f[2];
+    auto load_features = [&](long long tile) {
+        const long long row = tile * TC_ROWS + trow;
 #pragma unroll
         for (int j = 0; j < 2; ++j)
-            f[j] = row < V ? __ldg(reinterpret_cast<const uint4*>(feat + (size_t)row * kFeat) + 2 * half + j)
-                           : make_uint4(0, 0, 0, 0);
-#pragma unroll
-        for (int j = 0; j < 2; ++j) *reinterpret_cast<uint4*>(s.A1 + canon(trow, 16 * half + 8 * j, kFeat)) = f[j];
+            f[j] = tile < ntiles && row < V
+                       ? __ldg(reinterpret_cast<const uint4*>(feat + (size_t)row * kFeat) + 2 * half + j)
+                       : make_uint4(0, 0, 0, 0);
+    };
+    // this thread's shared-memory stores and tensor-memory loads are done: one
+    // barrier, and thread 0 issues the next layer; false when a wait gave up
+    auto publish = [&]() {
         fence_async_smem();
         tc_fence_before();
-        __syncthreads();
+        return __syncthreads_and(ok) != 0;
+    };
+    load_features(blockIdx.x);
+    for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) *reinterpret_cast<uint4*>(s.A + canon(trow, 16 * half + 8 * j, kFeat)) = f[j];
+        // (the last tile's layer-3 accumulator, where D1 goes, has been read
+        // before this barrier)
+        if (!publish()) break;
         if (tid == 0) {
             tc_fence_after();
 #pragma unroll
             for (int ks = 0; ks < kFeat / 16; ++ks) umma_bf16(tbase, dA1 + 16 * ks, dB1 + 16 * ks, id64, ks);
             umma_commit(bar);
         }
-        ok = __syncthreads_and(mbar_wait_bounded(bar, phase));
-        if (!ok) break;
+        load_features(tile + gridDim.x);
+        ok = mbar_wait_bounded(bar, phase);
         phase ^= 1u;
         tc_fence_after();
-        tc_hidden_half(tbase + lane_row + 32 * half, s.b1, s.A2, trow, 32 * half);
-        // layer 2
-        fence_async_smem();
-        tc_fence_before();
-        __syncthreads();
+        tc_hidden_half(tbase + lane_row + 32 * half, s.b1, s.A, trow, 32 * half);
+        if (!publish()) break;
         if (tid == 0) {
             tc_fence_after();
 #pragma unroll
-            for (int ks = 0; ks < kHid / 16; ++ks) umma_bf16(tbase + 64, dA2 + 16 * ks, dB2 + 16 * ks, id64, ks);
+            for (int ks = 0; ks < kHid / 16; ++ks) umma_bf16(tbase, dA2 + 16 * ks, dB2 + 16 * ks, id64, ks);
             umma_commit(bar);
         }
-        ok = __syncthreads_and(mbar_wait_bounded(bar, phase));
-        if (!ok) break;
+        ok = mbar_wait_bounded(bar, phase);
         phase ^= 1u;
         tc_fence_after();
-        tc_hidden_half(tbase + lane_row + 64 + 32 * half, s.b2, s.A2, trow, 32 * half);  // layer 2 is done with A2
-        // layer 3 (N = 16)
-        fence_async_smem();
-        tc_fence_before();
-        __syncthreads();
+        tc_hidden_half(tbase + lane_row + 32 * half, s.b2, s.A, trow, 32 * half);  // layer 2 is done with A2
+        if (!publish()) break;
         if (tid == 0) {
             tc_fence_after();
 #pragma unroll
             for (int ks = 0; ks < kHid / 16; ++ks) umma_bf16(tbase, dA2 + 16 * ks, dB3 + 16 * ks, id16, ks);
             umma_commit(bar);
         }
-        ok = __syncthreads_and(mbar_wait_bounded(bar, phase));
-        if (!ok) break;
+        ok = mbar_wait_bounded(bar, phase);
         phase ^= 1u;
         tc_fence_after();
-        unsigned r[16];
-        tmem_ld16(tbase + lane_row, r);
-        tmem_wait_ld();
-        if (half == 0 && row < V)
-            *reinterpret_cast<float4*>(out4 + 4 * (size_t)row) =
-                make_float4(__uint_as_float(r[0]) + s.b3[0], __uint_as_float(r[1]) + s.b3[1],
-                            __uint_as_float(r[2]) + s.b3[2], __uint_as_float(r[3]) + s.b3[3]);
-        tc_fence_before();
-        __syncthreads();  // every row read before the next tile's MMAs reuse the accumulators
+        if (half == 0) {
+            unsigned r[4];
+            tmem_ld4(tbase + lane_row, r);
+            tmem_wait_ld();
+            const long long row = tile * TC_ROWS + trow;
+            if (row < V)
+                *reinterpret_cast<float4*>(out4 + 4 * (size_t)row) =
+                    make_float4(__uint_as_float(r[0]) + s.b3[0], __uint_as_float(r[1]) + s.b3[1],
+                                __uint_as_float(r[2]) + s.b3[2], __uint_as_float(r[3]) + s.b3[3]);
+        }
     }
+    // a wait that gave up: the last layer's MMAs may be in flight, once more
+    // within the bound
+    ok = __syncthreads_and(ok) != 0;
     if (!ok) {
         if (tid == 0) atomicOr(status, SX_STATUS_WAIT_TIMEOUT);
-        mbar_wait_bounded(bar, phase);  // the MMAs in flight, once more within the bound
+        mbar_wait_bounded(bar, phase ^ 1u);
     }
     tc_fence_before();
     __syncthreads();
@@ -581,28 +656,37 @@ __global__ void __launch_bounds__(TC_THREADS, 1) mlp_forward_tc_kernel(int V, co
 }
 
 // ---------------------------------------------------------------------------
-// Training, part 1: forward + backward data path of a minibatch.  Rows are
-// idx[i] into the sample arrays (feat, target4 = (t, mask)).  Loss =
-// sum over rows and the 3 outputs of mask * (o - t)^2 / n_valid.  Writes per
-// row: H1, H2, dZ1, dZ2 (BF16, 64 each) and dO (BF16, 16, columns 3..15 zero),
-// and per warp: partial loss and bias gradients (FP32, in row order within the
-// warp, then summed over lanes in a fixed tree).
+// Training, part 1: forward, backward and weight gradients of a minibatch.  Rows
+// are idx[i] into the sample arrays (feat, target4 = (t, mask)).  Loss = sum over
+// rows and the 3 outputs of mask * (o - t)^2 / n_valid.
+//
+// A block takes tiles of 64 rows, a warp 16 of them: forward and backward data
+// path on its own rows with activations in registers, everything the weight
+// gradients need (X, H1, H2, dZ1, dZ2, dO, BF16) to shared memory; then dW1 =
+// dZ1^T X, dW2 = dZ2^T H1 and dW3 = dO^T H2 over the tile (A and B fragments by
+// ldmatrix.trans), warp w owning output rows 16 w .. of dW1 and dW2 and columns 16
+// w .. of dW3, accumulated in registers over the block's tiles.  One partial of
+// all parameters and the loss per block.
+//
+// The rows are few (65 536 are 1 024 tiles, 3.4 per block), so latency bounds it:
+// weights are staged 16 bytes at a time and only once, the next tile's features
+// load a tile ahead, and nothing returns to global memory in between.  (As two
+// kernels, with transposed weight copies staged value by value, activations and
+// gradients through global memory and bias partials per warp: 66 + 40 us, and 23
+// for the reduction over 4 096 warps' partials.)
 // ---------------------------------------------------------------------------
-struct TrainBuf {
-    unsigned short* h1;
-    unsigned short* h2;
-    unsigned short* dz1;
-    unsigned short* dz2;
-    unsigned short* dout;  // [M][16]
-    float* wpart;          // [nwarps][1 + 64 + 64 + 8]: loss, db1, db2, db3
-};
-constexpr int kWpart = 1 + kHid + kHid + kOut;
+constexpr int TR_ROWS = 64, TR_PER_SM = 2;
+constexpr int SL = 72, SX = 40, SD = 24;  // padded row strides (BF16) of 64, 32 and 16 columns
+constexpr int kBias = 1 + kHid + kHid + kOut;  // loss, db1, db2, db3
+constexpr int kPart = kParams + 1;             // a block's partial: the parameters in order, then the loss
 
-__device__ __forceinline__ void store_c_bf16(unsigned short* base, int ra, int rb, int ld, int col,
-                                             const float (&c)[4]) {
-    if (ra >= 0) *reinterpret_cast<unsigned*>(base + (size_t)ra * ld + col) = pack_bf2(c[0], c[1]);
-    if (rb >= 0) *reinterpret_cast<unsigned*>(base + (size_t)rb * ld + col) = pack_bf2(c[2], c[3]);
-}
+struct TrainSmem {
+    MlpSmem w;
+    alignas(16) unsigned short X[TR_ROWS * SX];
+    alignas(16) unsigned short H1[TR_ROWS * SL], H2[TR_ROWS * SL], D1[TR_ROWS * SL], D2[TR_ROWS * SL];
+    alignas(16) unsigned short DO[TR_ROWS * SD];  // columns 8 .. 15 zero
+    float bias[MLP_BLOCK / 32][kBias];
+};
 
 // sum over the 8 row groups g of a C-fragment column pair (lanes with equal tig)
 __device__ __forceinline__ float colsum(float v) {
@@ -612,145 +696,44 @@ __device__ __forceinline__ float colsum(float v) {
     return v;
 }
 
-__global__ void __launch_bounds__(MLP_BLOCK) mlp_train_fwd_bwd_kernel(int M, const int* __restrict__ idx,
-                                                                      const unsigned short* __restrict__ feat,
-                                                                      const float4* __restrict__ target4,
-                                                                      float inv_valid,
-                                                                      const unsigned short* __restrict__ w16,
-                                                                      const float* __restrict__ p32, TrainBuf tb) {
+__global__ void __launch_bounds__(MLP_BLOCK, TR_PER_SM) mlp_train_kernel(int M, const int* __restrict__ idx,
+                                                                         const unsigned short* __restrict__ feat,
+                                                                         const float4* __restrict__ target4,
+                                                                         float inv_valid,
+                                                                         const unsigned short* __restrict__ w16,
+                                                                         const float* __restrict__ p32,
+                                                                         float* __restrict__ part) {
     pdl_entry();
-    __shared__ MlpSmem s;
-    __shared__ MlpSmemT st;
-    stage_weights(s, w16, p32);
-    stage_weights_t(st, w16);
-    __syncthreads();
-    const int lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
-    float loss = 0.0f, db1[8][2], db2[8][2], db3[2];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) db1[j][0] = db1[j][1] = db2[j][0] = db2[j][1] = 0.0f;
-    db3[0] = db3[1] = 0.0f;
-    for (int r0 = warp * 16; r0 < M; r0 += nwarps * 16) {
-        const int ra = r0 + g < M ? r0 + g : -1, rb = r0 + g + 8 < M ? r0 + g + 8 : -1;
-        const int sa = ra >= 0 ? idx[ra] : -1, sb = rb >= 0 ? idx[rb] : -1;
-        unsigned ax[2][4];
-        load_x_frag(feat, sa, sb, ax);
-        Frag64 z1, z2;
-        float o[4];
-        tile_forward(s, ax, z1, z2, o);
-        // dO (C layout: rows g, g+8; columns 2tig, 2tig+1)
-        float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        if (tig < 2) {
-            const float4 ta = sa >= 0 ? target4[sa] : make_float4(0.f, 0.f, 0.f, 0.f);
-            const float4 tb4 = sb >= 0 ? target4[sb] : make_float4(0.f, 0.f, 0.f, 0.f);
-            const float tta[4] = {ta.x, ta.y, ta.z, 0.0f}, ttb[4] = {tb4.x, tb4.y, tb4.z, 0.0f};
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const int col = 2 * tig + u;
-                if (col < 3) {
-                    const float ea = ta.w * (o[u] - tta[col]), eb = tb4.w * (o[2 + u] - ttb[col]);
-                    loss = loss + (ea * (o[u] - tta[col]) + eb * (o[2 + u] - ttb[col]));
-                    d[u] = (2.0f * inv_valid) * ea;
-                    d[2 + u] = (2.0f * inv_valid) * eb;
-                }
-            }
-        }
-        // dH2 = dO W3 (K = 16, columns 8..15 of dO are zero)
-        unsigned ad[4] = {pack_bf2(d[0], d[1]), pack_bf2(d[2], d[3]), 0u, 0u};
-        Frag64 dz;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            dz.c[j][0] = dz.c[j][1] = dz.c[j][2] = dz.c[j][3] = 0.0f;
-            const unsigned short* w = st.W3t + (8 * j + g) * S3T + 2 * tig;
-            mma16816(dz.c[j], ad, lds32(w), lds32(w + 8));
-        }
-        // dZ2 = dH2 * silu'(Z2); H2 = silu(Z2); H1 = silu(Z1)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            float h[4], h1[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                dz.c[j][u] = dz.c[j][u] * silu_grad(z2.c[j][u]);
-                h[u] = silu(z2.c[j][u]);
-                h1[u] = silu(z1.c[j][u]);
-            }
-            store_c_bf16(tb.h2, ra, rb, kHid, 8 * j + 2 * tig, h);
-            store_c_bf16(tb.h1, ra, rb, kHid, 8 * j + 2 * tig, h1);
-            store_c_bf16(tb.dz2, ra, rb, kHid, 8 * j + 2 * tig, dz.c[j]);
-            db2[j][0] += dz.c[j][0] + dz.c[j][2];
-            db2[j][1] += dz.c[j][1] + dz.c[j][3];
-        }
-        store_c_bf16(tb.dout, ra, rb, 16, 2 * tig, d);
-        if (ra >= 0) *reinterpret_cast<unsigned*>(tb.dout + (size_t)ra * 16 + 8 + 2 * tig) = 0u;
-        if (rb >= 0) *reinterpret_cast<unsigned*>(tb.dout + (size_t)rb * 16 + 8 + 2 * tig) = 0u;
-        db3[0] += d[0] + d[2];
-        db3[1] += d[1] + d[3];
-        // dH1 = dZ2 W2, dZ1 = dH1 * silu'(Z1)
-        unsigned az[4][4];
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks) {
-            az[ks][0] = pack_bf2(dz.c[2 * ks][0], dz.c[2 * ks][1]);
-            az[ks][1] = pack_bf2(dz.c[2 * ks][2], dz.c[2 * ks][3]);
-            az[ks][2] = pack_bf2(dz.c[2 * ks + 1][0], dz.c[2 * ks + 1][1]);
-            az[ks][3] = pack_bf2(dz.c[2 * ks + 1][2], dz.c[2 * ks + 1][3]);
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-            for (int ks = 0; ks < 4; ++ks) {
-                const unsigned short* w = st.W2t + (8 * j + g) * S2T + 16 * ks + 2 * tig;
-                mma16816(c, az[ks], lds32(w), lds32(w + 8));
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) c[u] = c[u] * silu_grad(z1.c[j][u]);
-            store_c_bf16(tb.dz1, ra, rb, kHid, 8 * j + 2 * tig, c);
-            db1[j][0] += c[0] + c[2];
-            db1[j][1] += c[1] + c[3];
-        }
-    }
-    // per-warp partials: loss and bias gradients, summed over the row groups
-    float* wp = tb.wpart + (size_t)warp * kWpart;
-    float l = loss;
-    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    if (lane == 0) wp[0] = l;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const float a0 = colsum(db1[j][0]), a1 = colsum(db1[j][1]);
-        const float c0 = colsum(db2[j][0]), c1 = colsum(db2[j][1]);
-        if (g == 0) {
-            wp[1 + 8 * j + 2 * tig] = a0;
-            wp[1 + 8 * j + 2 * tig + 1] = a1;
-            wp[1 + kHid + 8 * j + 2 * tig] = c0;
-            wp[1 + kHid + 8 * j + 2 * tig + 1] = c1;
-        }
-    }
-    const float e0 = colsum(db3[0]), e1 = colsum(db3[1]);
-    if (g == 0) {
-        wp[1 + 2 * kHid + 2 * tig] = e0;
-        wp[1 + 2 * kHid + 2 * tig + 1] = e1;
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Training, part 2: weight gradients dW1 = dZ1^T X, dW2 = dZ2^T H1,
-// dW3 = dO^T H2 over this block's rows (64-row tiles staged in shared memory,
-// A = dZ^T and B = H fragments by ldmatrix.trans), one partial per block.
-// Warp w owns output rows 16w..16w+15 of dW1 and dW2 and columns 16w..16w+15
-// of dW3.
-// ---------------------------------------------------------------------------
-constexpr int WG_ROWS = 64, SL = 72;  // tile rows; padded row stride (BF16)
-constexpr int kWgrad = kHid * kFeat + kHid * kHid + kOut * kHid;
-
-__global__ void __launch_bounds__(MLP_BLOCK) mlp_wgrad_kernel(int M, int rows_per_block,
-                                                              const int* __restrict__ idx,
-                                                              const unsigned short* __restrict__ feat,
-                                                              TrainBuf tb, float* __restrict__ bpart) {
-    pdl_entry();
-    __shared__ __align__(16) unsigned short X[WG_ROWS * SL], H1[WG_ROWS * SL], H2[WG_ROWS * SL],
-        D1[WG_ROWS * SL], D2[WG_ROWS * SL], DO[WG_ROWS * SL];
+    extern __shared__ uint4 smem_raw[];
+    TrainSmem& s = *reinterpret_cast<TrainSmem*>(smem_raw);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, tig = lane & 3;
     const int q = lane >> 3, r8 = lane & 7;
+    // the warp's 16 feature rows of a tile: 64 pieces of 16 bytes, two a lane
+    auto piece = [&](int j) { return lane + 32 * j; };
+    auto load_idx = [&](long long tile, int (&id)[2]) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const long long row = tile * TR_ROWS + 16 * w + (piece(j) >> 2);
+            id[j] = row < M ? idx[row] : -1;
+        }
+    };
+    auto load_x = [&](const int (&id)[2], uint4 (&x)[2]) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+            x[j] = id[j] >= 0 ? *reinterpret_cast<const uint4*>(feat + (size_t)id[j] * kFeat + (piece(j) & 3) * 8)
+                              : make_uint4(0u, 0u, 0u, 0u);
+    };
+    const long long ntiles = ((long long)M + TR_ROWS - 1) / TR_ROWS;
+    int id[2], next[2];
+    uint4 x[2];
+    load_idx(blockIdx.x, id);
+    load_idx(blockIdx.x + gridDim.x, next);
+    stage_weights(s.w, w16, p32);
+    for (int i = threadIdx.x; i < TR_ROWS; i += MLP_BLOCK)
+        *reinterpret_cast<uint4*>(s.DO + i * SD + 8) = make_uint4(0u, 0u, 0u, 0u);
+    load_x(id, x);
+    __syncthreads();
+
     float a1[4][4], a2[8][4], a3[2][4];
 #pragma unroll
     for (int j = 0; j < 8; ++j) a2[j][0] = a2[j][1] = a2[j][2] = a2[j][3] = 0.0f;
@@ -758,92 +741,209 @@ __global__ void __launch_bounds__(MLP_BLOCK) mlp_wgrad_kernel(int M, int rows_pe
     for (int j = 0; j < 4; ++j) a1[j][0] = a1[j][1] = a1[j][2] = a1[j][3] = 0.0f;
 #pragma unroll
     for (int j = 0; j < 2; ++j) a3[j][0] = a3[j][1] = a3[j][2] = a3[j][3] = 0.0f;
-    const int rbeg = blockIdx.x * rows_per_block, rend = min(M, rbeg + rows_per_block);
-    for (int t0 = rbeg; t0 < rend; t0 += WG_ROWS) {
-        __syncthreads();
-        // stage 64 rows (zero past the end): 8 BF16 = 16 bytes per copy
-        for (int i = threadIdx.x; i < WG_ROWS * 8; i += blockDim.x) {
-            const int r = i >> 3, c8 = (i & 7) * 8, row = t0 + r;
-            const bool ok = row < rend;
-            const uint4 z = make_uint4(0u, 0u, 0u, 0u);
-            *reinterpret_cast<uint4*>(H1 + r * SL + c8) = ok ? *reinterpret_cast<const uint4*>(tb.h1 + (size_t)row * kHid + c8) : z;
-            *reinterpret_cast<uint4*>(H2 + r * SL + c8) = ok ? *reinterpret_cast<const uint4*>(tb.h2 + (size_t)row * kHid + c8) : z;
-            *reinterpret_cast<uint4*>(D1 + r * SL + c8) = ok ? *reinterpret_cast<const uint4*>(tb.dz1 + (size_t)row * kHid + c8) : z;
-            *reinterpret_cast<uint4*>(D2 + r * SL + c8) = ok ? *reinterpret_cast<const uint4*>(tb.dz2 + (size_t)row * kHid + c8) : z;
-            if (c8 < kFeat)
-                *reinterpret_cast<uint4*>(X + r * SL + c8) =
-                    ok ? *reinterpret_cast<const uint4*>(feat + (size_t)idx[row] * kFeat + c8) : z;
-            if (c8 < 16)
-                *reinterpret_cast<uint4*>(DO + r * SL + c8) = ok ? *reinterpret_cast<const uint4*>(tb.dout + (size_t)row * 16 + c8) : z;
+    float loss = 0.0f, db1[8][2], db2[8][2], db3[2];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) db1[j][0] = db1[j][1] = db2[j][0] = db2[j][1] = 0.0f;
+    db3[0] = db3[1] = 0.0f;
+    const int ra = 16 * w + g, rb = ra + 8;  // this lane's rows of the tile
+    auto put = [](unsigned short* p, unsigned v) { *reinterpret_cast<unsigned*>(p) = v; };
+
+    for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const int sa = __shfl_sync(0xffffffffu, id[0], 4 * g), sb = __shfl_sync(0xffffffffu, id[1], 4 * g);
+        float4 ta = make_float4(0.f, 0.f, 0.f, 0.f), tb = ta;
+        if (tig < 2) {
+            if (sa >= 0) ta = target4[sa];
+            if (sb >= 0) tb = target4[sb];
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+            *reinterpret_cast<uint4*>(s.X + (16 * w + (piece(j) >> 2)) * SX + (piece(j) & 3) * 8) = x[j];
+        __syncwarp();
+        id[0] = next[0];
+        id[1] = next[1];
+        load_x(id, x);
+        load_idx(tile + 2LL * gridDim.x, next);
+        unsigned ax[2][4];
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) {
+            const int c = 16 * ks + 2 * tig;
+            ax[ks][0] = lds32(s.X + ra * SX + c);
+            ax[ks][1] = lds32(s.X + rb * SX + c);
+            ax[ks][2] = lds32(s.X + ra * SX + c + 8);
+            ax[ks][3] = lds32(s.X + rb * SX + c + 8);
+        }
+        Frag64 z1, z2;
+        float o[4];
+        tile_forward(s.w, ax, z1, z2, o, [&](int layer, int ks, const unsigned(&a)[4]) {
+            unsigned short* h = layer == 1 ? s.H1 : s.H2;
+            const int c = 16 * ks + 2 * tig;
+            put(h + ra * SL + c, a[0]);
+            put(h + rb * SL + c, a[1]);
+            put(h + ra * SL + c + 8, a[2]);
+            put(h + rb * SL + c + 8, a[3]);
+        });
+        // dO (C layout: rows g, g+8; columns 2tig, 2tig+1)
+        float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if (tig < 2) {
+            const float tta[4] = {ta.x, ta.y, ta.z, 0.0f}, ttb[4] = {tb.x, tb.y, tb.z, 0.0f};
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int col = 2 * tig + u;
+                if (col < 3) {
+                    const float ea = ta.w * (o[u] - tta[col]), eb = tb.w * (o[2 + u] - ttb[col]);
+                    loss = loss + (ea * (o[u] - tta[col]) + eb * (o[2 + u] - ttb[col]));
+                    d[u] = (2.0f * inv_valid) * ea;
+                    d[2 + u] = (2.0f * inv_valid) * eb;
+                }
+            }
+        }
+        db3[0] += d[0] + d[2];
+        db3[1] += d[1] + d[3];
+        // dH2 = dO W3 (K = 16, columns 8..15 of dO are zero), dZ2 = dH2 * silu'(Z2)
+        const unsigned ad[4] = {pack_bf2(d[0], d[1]), pack_bf2(d[2], d[3]), 0u, 0u};
+        put(s.DO + ra * SD + 2 * tig, ad[0]);
+        put(s.DO + rb * SD + 2 * tig, ad[1]);
+        unsigned az[4][4];
+#pragma unroll
+        for (int jq = 0; jq < 2; ++jq) {
+            unsigned B[4];  // W3 rows 0..7 (k), columns 8 j .. of j = 4 jq .. 4 jq + 3
+            ldsm_x4_trans(B, s.w.W3 + r8 * S3 + 8 * (4 * jq + q));
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int j = 4 * jq + i;
+                float dz[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                mma16816(dz, ad, B[i], 0u);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) dz[u] = dz[u] * silu_grad(z2.c[j][u]);
+                db2[j][0] += dz[0] + dz[2];
+                db2[j][1] += dz[1] + dz[3];
+                const unsigned lo = pack_bf2(dz[0], dz[1]), hi = pack_bf2(dz[2], dz[3]);
+                az[j / 2][2 * (j & 1)] = lo;
+                az[j / 2][2 * (j & 1) + 1] = hi;
+                put(s.D2 + ra * SL + 8 * j + 2 * tig, lo);
+                put(s.D2 + rb * SL + 8 * j + 2 * tig, hi);
+            }
+        }
+        // dH1 = dZ2 W2, dZ1 = dH1 * silu'(Z1)
+#pragma unroll
+        for (int jp = 0; jp < 4; ++jp) {
+            float c[2][4] = {{0.0f, 0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f, 0.0f}};
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks) {
+                unsigned B[4];  // W2 rows 16 ks .. (k), columns 16 jp ..: (k, n) (k+8, n) (k, n+8) (k+8, n+8)
+                ldsm_x4_trans(B, s.w.W2 + (16 * ks + (q & 1) * 8 + r8) * S2 + 16 * jp + (q >> 1) * 8);
+                mma16816(c[0], az[ks], B[0], B[1]);
+                mma16816(c[1], az[ks], B[2], B[3]);
+            }
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int j = 2 * jp + i;
+#pragma unroll
+                for (int u = 0; u < 4; ++u) c[i][u] = c[i][u] * silu_grad(z1.c[j][u]);
+                db1[j][0] += c[i][0] + c[i][2];
+                db1[j][1] += c[i][1] + c[i][3];
+                put(s.D1 + ra * SL + 8 * j + 2 * tig, pack_bf2(c[i][0], c[i][1]));
+                put(s.D1 + rb * SL + 8 * j + 2 * tig, pack_bf2(c[i][2], c[i][3]));
+            }
         }
         __syncthreads();
 #pragma unroll
-        for (int ks = 0; ks < WG_ROWS / 16; ++ks) {
+        for (int ks = 0; ks < TR_ROWS / 16; ++ks) {
             const int m0 = 16 * ks;
             // A = D^T rows o0 = 16w .. 16w+15 (matrices: (m0,o0) (m0,o0+8) (m0+8,o0) (m0+8,o0+8))
             const int am = m0 + (q >> 1) * 8 + r8, ao = 16 * w + (q & 1) * 8;
             unsigned A2[4], A1[4];
-            ldsm_x4_trans(A2, D2 + am * SL + ao);
-            ldsm_x4_trans(A1, D1 + am * SL + ao);
+            ldsm_x4_trans(A2, s.D2 + am * SL + ao);
+            ldsm_x4_trans(A1, s.D1 + am * SL + ao);
             // B fragments for two n-tiles per load: matrices (m0,n0) (m0+8,n0) (m0,n0+8) (m0+8,n0+8)
             const int bm = m0 + (q & 1) * 8 + r8, bn = (q >> 1) * 8;
 #pragma unroll
             for (int jp = 0; jp < 4; ++jp) {
                 unsigned B[4];
-                ldsm_x4_trans(B, H1 + bm * SL + 16 * jp + bn);
+                ldsm_x4_trans(B, s.H1 + bm * SL + 16 * jp + bn);
                 mma16816(a2[2 * jp], A2, B[0], B[1]);
                 mma16816(a2[2 * jp + 1], A2, B[2], B[3]);
             }
 #pragma unroll
             for (int jp = 0; jp < 2; ++jp) {
                 unsigned B[4];
-                ldsm_x4_trans(B, X + bm * SL + 16 * jp + bn);
+                ldsm_x4_trans(B, s.X + bm * SX + 16 * jp + bn);
                 mma16816(a1[2 * jp], A1, B[0], B[1]);
                 mma16816(a1[2 * jp + 1], A1, B[2], B[3]);
             }
             // dW3: A = dO^T (16 rows, 8 used), B = H2 columns 16w .. 16w+15
             unsigned A3[4], B3[4];
-            ldsm_x4_trans(A3, DO + am * SL + (q & 1) * 8);
-            ldsm_x4_trans(B3, H2 + bm * SL + 16 * w + bn);
+            ldsm_x4_trans(A3, s.DO + am * SD + (q & 1) * 8);
+            ldsm_x4_trans(B3, s.H2 + bm * SL + 16 * w + bn);
             mma16816(a3[0], A3, B3[0], B3[1]);
             mma16816(a3[1], A3, B3[2], B3[3]);
         }
+        __syncthreads();
     }
-    // write this block's partial (C layout: rows g, g+8; columns 2tig, 2tig+1)
-    float* bp = bpart + (size_t)blockIdx.x * kWgrad;
+    // bias gradients and loss: over the lanes, then over the warps in order
+    float* wb = s.bias[w];
+    for (int off = 16; off > 0; off >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, off);
+    if (lane == 0) wb[0] = loss;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const float u0 = colsum(db1[j][0]), u1 = colsum(db1[j][1]);
+        const float v0 = colsum(db2[j][0]), v1 = colsum(db2[j][1]);
+        if (g == 0) {
+            wb[1 + 8 * j + 2 * tig] = u0;
+            wb[1 + 8 * j + 2 * tig + 1] = u1;
+            wb[1 + kHid + 8 * j + 2 * tig] = v0;
+            wb[1 + kHid + 8 * j + 2 * tig + 1] = v1;
+        }
+    }
+    const float e0 = colsum(db3[0]), e1 = colsum(db3[1]);
+    if (g == 0) {
+        wb[1 + 2 * kHid + 2 * tig] = e0;
+        wb[1 + 2 * kHid + 2 * tig + 1] = e1;
+    }
+    __syncthreads();
+    float* bp = part + (size_t)blockIdx.x * kPart;
+    for (int i = threadIdx.x; i < kBias; i += MLP_BLOCK) {
+        float t = s.bias[0][i];
+#pragma unroll
+        for (int k = 1; k < MLP_BLOCK / 32; ++k) t += s.bias[k][i];
+        const int at = i == 0            ? kParams
+                       : i < 1 + kHid     ? ob1 + i - 1
+                       : i < 1 + 2 * kHid ? ob2 + i - 1 - kHid
+                                          : ob3 + i - 1 - 2 * kHid;
+        bp[at] = t;
+    }
+    // weight gradients (C layout: rows g, g+8; columns 2tig, 2tig+1)
     const int o_lo = 16 * w + g, o_hi = o_lo + 8;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         const int c = 8 * j + 2 * tig;
-        bp[o_lo * kFeat + c] = a1[j][0];
-        bp[o_lo * kFeat + c + 1] = a1[j][1];
-        bp[o_hi * kFeat + c] = a1[j][2];
-        bp[o_hi * kFeat + c + 1] = a1[j][3];
+        bp[oW1 + o_lo * kFeat + c] = a1[j][0];
+        bp[oW1 + o_lo * kFeat + c + 1] = a1[j][1];
+        bp[oW1 + o_hi * kFeat + c] = a1[j][2];
+        bp[oW1 + o_hi * kFeat + c + 1] = a1[j][3];
     }
-    float* bp2 = bp + kHid * kFeat;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
         const int c = 8 * j + 2 * tig;
-        bp2[o_lo * kHid + c] = a2[j][0];
-        bp2[o_lo * kHid + c + 1] = a2[j][1];
-        bp2[o_hi * kHid + c] = a2[j][2];
-        bp2[o_hi * kHid + c + 1] = a2[j][3];
+        bp[oW2 + o_lo * kHid + c] = a2[j][0];
+        bp[oW2 + o_lo * kHid + c + 1] = a2[j][1];
+        bp[oW2 + o_hi * kHid + c] = a2[j][2];
+        bp[oW2 + o_hi * kHid + c + 1] = a2[j][3];
     }
-    float* bp3 = bp2 + kHid * kHid;
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
         const int c = 16 * w + 8 * j + 2 * tig;
         if (g < kOut) {
-            bp3[g * kHid + c] = a3[j][0];
-            bp3[g * kHid + c + 1] = a3[j][1];
+            bp[oW3 + g * kHid + c] = a3[j][0];
+            bp[oW3 + g * kHid + c + 1] = a3[j][1];
         }
     }
 }
 
 // ---------------------------------------------------------------------------
-// Training, part 3: sum the block and warp partials in a fixed order into
-// grad; stats[0] = loss (sum over the warps' partials).
-// Part 4: Adam on the FP32 master weights, refreshing the BF16 copy.
+// Training, part 2: sum the blocks' partials in a fixed order into grad;
+// stats[0] = loss.
+// Part 3: Adam on the FP32 master weights, refreshing the BF16 copy.
 // Structurally zero parameters (W1 columns >= 24, W3/b3 rows >= 3) stay zero.
 // ---------------------------------------------------------------------------
 constexpr int RD_GROUPS = 16;  // partial groups per parameter column in mlp_reduce_kernel
@@ -851,41 +951,25 @@ constexpr int RD_GROUPS = 16;  // partial groups per parameter column in mlp_red
 // Block = 32 parameter columns x RD_GROUPS groups: group y sums partials
 // y, y + RD_GROUPS, ... of its column (coalesced across the columns), then
 // the groups are added in order -- a fixed order, so the sums are
-// deterministic.  Column -1 is the loss.
-__global__ void __launch_bounds__(32 * RD_GROUPS) mlp_reduce_kernel(int nblocks, const float* __restrict__ bpart,
-                                                                   int nwarps, const float* __restrict__ wpart,
+// deterministic.
+__global__ void __launch_bounds__(32 * RD_GROUPS) mlp_reduce_kernel(int nblocks, const float* __restrict__ part,
                                                                    float* __restrict__ grad,
                                                                    float* __restrict__ stats) {
     pdl_entry();
-    __shared__ float part[RD_GROUPS][33];
+    __shared__ float sums[RD_GROUPS][33];
     const int tx = threadIdx.x & 31, gy = threadIdx.x >> 5;
-    const int i = blockIdx.x * 32 + tx - 1;
-    const float* base = wpart;
-    size_t stride = kWpart;
-    int count = 0;
-    if (i == -1) {
-        count = nwarps;
-    } else if (i < ob1) {
-        base = bpart + (i - oW1), stride = kWgrad, count = nblocks;
-    } else if (i < oW2) {
-        base = wpart + 1 + (i - ob1), count = nwarps;
-    } else if (i < ob2) {
-        base = bpart + kHid * kFeat + (i - oW2), stride = kWgrad, count = nblocks;
-    } else if (i < oW3) {
-        base = wpart + 1 + kHid + (i - ob2), count = nwarps;
-    } else if (i < ob3) {
-        base = bpart + kHid * kFeat + kHid * kHid + (i - oW3), stride = kWgrad, count = nblocks;
-    } else if (i < kParams) {
-        base = wpart + 1 + 2 * kHid + (i - ob3), count = nwarps;
-    }
+    const int i = blockIdx.x * 32 + tx;
     float sum = 0.0f;
-    for (int k = gy; k < count; k += RD_GROUPS) sum += base[(size_t)k * stride];
-    part[gy][tx] = sum;
+    if (i < kPart) {
+#pragma unroll 8
+        for (int k = gy; k < nblocks; k += RD_GROUPS) sum += part[(size_t)k * kPart + i];
+    }
+    sums[gy][tx] = sum;
     __syncthreads();
-    if (gy == 0 && i < kParams) {
-        float t = part[0][tx];
-        for (int y = 1; y < RD_GROUPS; ++y) t += part[y][tx];
-        if (i < 0)
+    if (gy == 0 && i < kPart) {
+        float t = sums[0][tx];
+        for (int y = 1; y < RD_GROUPS; ++y) t += sums[y][tx];
+        if (i == kParams)
             stats[0] = t;
         else
             grad[i] = t;
@@ -983,20 +1067,14 @@ extern "C" int sx_mlp_forward_tc(const void* feat, int n_rows, const void* w16, 
     SX_REQUIRE(n_rows >= 0, "sx_mlp_forward_tc: n_rows < 0");
     if (n_rows == 0) return SX_OK;
     SX_REQUIRE(feat && w16 && p32 && out4 && status, "sx_mlp_forward_tc: null pointer");
-    const int tiles = (n_rows + TC_ROWS - 1) / TC_ROWS;
+    const long long tiles = ((long long)n_rows + TC_ROWS - 1) / TC_ROWS;
     int dev = 0, sms = 0;
     SX_CUDA(cudaGetDevice(&dev));
     SX_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    // four CTAs per SM share the SM's 512 tensor-memory columns; unused dynamic
-    // shared memory keeps a fifth from becoming resident and waiting in
-    // tcgen05.alloc for a column range
-    static bool attr = false;
-    if (!attr) {
-        SX_CUDA(cudaFuncSetAttribute(mlp_forward_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_PAD_SMEM));
-        attr = true;
-    }
-    const int blocks = tiles < 4 * sms ? tiles : 4 * sms;
-    launch(mlp_forward_tc_kernel, blocks, TC_THREADS, TC_PAD_SMEM, as_stream(stream), n_rows,
+    // at most 7 CTAs fit an SM's shared memory, whose tensor memory holds 8: no
+    // CTA waits in tcgen05.alloc
+    const long long most = (long long)TC_PER_SM * sms;
+    launch(mlp_forward_tc_kernel, (int)(tiles < most ? tiles : most), TC_THREADS, 0, as_stream(stream), n_rows,
            (const unsigned short*)feat, (const unsigned short*)w16, p32, out4, status);
     return check_launch("mlp_forward_tc_kernel");
 }
@@ -1014,64 +1092,27 @@ extern "C" int sx_mlp_forward(const void* feat, int n_rows, const void* w16, con
     return check_launch("mlp_forward_kernel");
 }
 
-// Training workspace: per row 4x64 + 16 BF16, per warp kWpart floats, per
-// weight-gradient block kWgrad floats, then the gradient (kParams floats).
-static void train_shape(int M, int* fb_blocks, int* nwarps, int* wg_blocks, int* rows_per_block) {
-    const int tiles = (M + 15) / 16;
-    int b = (tiles + MLP_BLOCK / 32 - 1) / (MLP_BLOCK / 32);
-    if (b > 152 * 8) b = 152 * 8;
-    *fb_blocks = b;
-    *nwarps = b * (MLP_BLOCK / 32);
-    // about two blocks per SM, whole 64-row tiles each
-    const int rpb = ((M + 152 * 2 - 1) / (152 * 2) + WG_ROWS - 1) / WG_ROWS * WG_ROWS;
-    const int wg = (M + rpb - 1) / rpb;
-    *wg_blocks = wg;
-    *rows_per_block = rpb;
-}
-
-struct TrainWs {
-    TrainBuf tb;
-    float* bpart;
-    float* grad;
-    int fb, nw, wg, rpb;
-};
-
-static TrainWs train_ws(void* ws, int n_rows) {
-    TrainWs w;
-    train_shape(n_rows, &w.fb, &w.nw, &w.wg, &w.rpb);
-    char* p = (char*)ws;
-    const size_t rows = (size_t)n_rows;
-    w.tb.h1 = (unsigned short*)p;
-    w.tb.h2 = w.tb.h1 + rows * kHid;
-    w.tb.dz1 = w.tb.h2 + rows * kHid;
-    w.tb.dz2 = w.tb.dz1 + rows * kHid;
-    w.tb.dout = w.tb.dz2 + rows * kHid;
-    w.tb.wpart = (float*)(p + rows * (4 * kHid + 16) * 2);
-    w.bpart = w.tb.wpart + (size_t)w.nw * kWpart;
-    w.grad = w.bpart + (size_t)w.wg * kWgrad;
-    return w;
+// Training workspace: a partial of kPart floats per block, then the gradient.
+static int train_blocks(int M) {
+    const long long tiles = ((long long)M + TR_ROWS - 1) / TR_ROWS, most = 152LL * TR_PER_SM;
+    return (int)(tiles < most ? tiles : most);
 }
 
 extern "C" size_t sx_mlp_train_workspace_bytes(int max_rows) {
-    int fb, nw, wg, rpb;
-    const int M = max_rows > 0 ? max_rows : 1;
-    train_shape(M, &fb, &nw, &wg, &rpb);
-    return (size_t)M * (4 * kHid + 16) * 2 + (size_t)nw * kWpart * 4 + (size_t)wg * kWgrad * 4 +
-           (size_t)kParams * 4 + 256;
+    return ((size_t)train_blocks(max_rows > 0 ? max_rows : 1) * kPart + kParams) * 4 + 256;
 }
 
-static int mlp_grad_launches(const TrainWs& w, const void* feat, const float* target4, const int* idx, int n_rows,
+static int mlp_grad_launches(float* part, const void* feat, const float* target4, const int* idx, int n_rows,
                              int n_valid, const void* w16, const float* p32, float* grad, float* stats,
                              cudaStream_t s) {
-    launch(mlp_train_fwd_bwd_kernel, w.fb, MLP_BLOCK, 0, s, n_rows, idx, (const unsigned short*)feat,
-           (const float4*)target4, 1.0f / (float)n_valid, (const unsigned short*)w16, p32, w.tb);
-    int rc = check_launch("mlp_train_fwd_bwd_kernel");
+    SX_CUDA(cudaFuncSetAttribute(mlp_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(TrainSmem)));
+    const int blocks = train_blocks(n_rows);
+    launch(mlp_train_kernel, blocks, MLP_BLOCK, sizeof(TrainSmem), s, n_rows, idx, (const unsigned short*)feat,
+           (const float4*)target4, 1.0f / (float)n_valid, (const unsigned short*)w16, p32, part);
+    int rc = check_launch("mlp_train_kernel");
     if (rc) return rc;
-    launch(mlp_wgrad_kernel, w.wg, MLP_BLOCK, 0, s, n_rows, w.rpb, idx, (const unsigned short*)feat, w.tb, w.bpart);
-    rc = check_launch("mlp_wgrad_kernel");
-    if (rc) return rc;
-    launch(mlp_reduce_kernel, (kParams + 1 + 31) / 32, 32 * RD_GROUPS, 0, s, w.wg, (const float*)w.bpart, w.nw,
-           (const float*)w.tb.wpart, grad, stats);
+    launch(mlp_reduce_kernel, (kPart + 31) / 32, 32 * RD_GROUPS, 0, s, blocks, (const float*)part, grad, stats);
     return check_launch("mlp_reduce_kernel");
 }
 
@@ -1081,8 +1122,7 @@ extern "C" int sx_mlp_gradients(const void* feat, const float* target4, const in
     SX_REQUIRE(n_rows > 0 && n_valid > 0, "sx_mlp_gradients: bad sizes");
     SX_REQUIRE(feat && target4 && idx && w16 && p32 && grad && stats && ws, "sx_mlp_gradients: null pointer");
     SX_REQUIRE(ws_bytes >= sx_mlp_train_workspace_bytes(n_rows), "sx_mlp_gradients: workspace too small");
-    const TrainWs w = train_ws(ws, n_rows);
-    return mlp_grad_launches(w, feat, target4, idx, n_rows, n_valid, w16, p32, grad, stats, as_stream(stream));
+    return mlp_grad_launches((float*)ws, feat, target4, idx, n_rows, n_valid, w16, p32, grad, stats, as_stream(stream));
 }
 
 extern "C" int sx_mlp_train_step(const void* feat, const float* target4, const int* idx, int n_rows, int n_valid,
@@ -1093,12 +1133,12 @@ extern "C" int sx_mlp_train_step(const void* feat, const float* target4, const i
     SX_REQUIRE(feat && target4 && idx && w16 && p32 && adam_m && adam_v && stats && ws,
                "sx_mlp_train_step: null pointer");
     SX_REQUIRE(ws_bytes >= sx_mlp_train_workspace_bytes(n_rows), "sx_mlp_train_step: workspace too small");
-    const TrainWs w = train_ws(ws, n_rows);
     cudaStream_t s = as_stream(stream);
-    int rc = mlp_grad_launches(w, feat, target4, idx, n_rows, n_valid, w16, p32, w.grad, stats, s);
+    float* grad = (float*)ws + (size_t)train_blocks(n_rows) * kPart;
+    int rc = mlp_grad_launches((float*)ws, feat, target4, idx, n_rows, n_valid, w16, p32, grad, stats, s);
     if (rc) return rc;
     const float bc1 = 1.0f - powf(beta1, (float)step), bc2 = 1.0f - powf(beta2, (float)step);
-    launch(mlp_adam_kernel, grid_for(kParams, 256), 256, 0, s, (const float*)w.grad, p32, adam_m, adam_v,
+    launch(mlp_adam_kernel, grid_for(kParams, 256), 256, 0, s, (const float*)grad, p32, adam_m, adam_v,
            (unsigned short*)w16, lr, beta1, beta2, eps, bc1, bc2);
     return check_launch("mlp_adam_kernel");
 }
