@@ -122,6 +122,19 @@ int sx_jacobi_sweep_packed_forms(void);
 int sx_jacobi_sweep_packed_v(const float* x4, const float* y_in4, float* y_out4, const float* fixed,
                              const int* adj_ptr, const short* nbr16, const unsigned* rest32, int n_verts,
                              float k_spring, float k_bend, int bend_on_y, int form, int fast, void* stream);
+/* sx_jacobi_sweep_mode / sx_jacobi_sweep_packed_v that also raise, for each
+ * block of 32 vertices, moved[block] to the largest squared distance of an output
+ * position from ref4 (as float bits, which order like the values), for
+ * sx_contact_pairs_project_headed, where the heads of the pair list are in use.
+ * pair_counts: the last 256 bytes of the list's workspace.  All three NULL: the
+ * plain sweep. */
+int sx_jacobi_sweep_tracked(const float* x4, const float* y_in4, float* y_out4, const float* fixed, const int* adj_ptr,
+                            const int* adj, int n_verts, float k_spring, float k_bend, int bend_on_y, int variant,
+                            int fast, const float* ref4, unsigned* moved, const int* pair_counts, void* stream);
+int sx_jacobi_sweep_packed_tracked(const float* x4, const float* y_in4, float* y_out4, const float* fixed,
+                                   const int* adj_ptr, const short* nbr16, const unsigned* rest32, int n_verts,
+                                   float k_spring, float k_bend, int bend_on_y, int form, int fast, const float* ref4,
+                                   unsigned* moved, const int* pair_counts, void* stream);
 
 /* solve_sewing_constraints_x (XPBD.py:425-441) + update_dx over sewn vertex
  * pairs (zero rest length, k = compliance argument of the reference):
@@ -413,6 +426,26 @@ int sx_contact_pairs_project_v(int n_dy, int n_st, const int* pairs, const void*
                                const float* xs4, const float* fixed, const float* m_inv, float dHat, float compliance,
                                float cull_d2, long long* dx_fix, int* nc, int* status, const int* conv, int iter,
                                int variant, void* stream);
+int sx_contact_pairs_project_default_variant(void);
+/* Heads of the vertex-vs-cloth pairs: per chunk of 32 consecutive pairs of the
+ * list, a bound on the motion of its vertices below which none of its pairs can
+ * come within cull_d2 (a margin above dHat), and the blocks of 32 vertices they
+ * lie in.  sx_contact_pairs_heads writes them for the positions y4, which it also
+ * copies to ref4, and clears moved ((n_dy + 31) / 32 words); with fewer than
+ * min_pairs such pairs it writes none.  Afterwards every change of the positions
+ * must end in a tracked sweep (sx_jacobi_sweep_tracked with this ref4 and moved)
+ * before sx_contact_pairs_project_headed, which then passes over the chunks that
+ * cannot have come into reach: the same sums as sx_contact_pairs_project_v.  A
+ * new list (sx_contact_pairs_build) drops the heads.  heads:
+ * sx_contact_pairs_heads_bytes bytes, 16-byte aligned. */
+size_t sx_contact_pairs_heads_bytes(int n_dy, int cap);
+int sx_contact_pairs_heads(int n_dy, int n_st, int cap, const int* pairs, void* ws, const float* y4, float cull_d2,
+                           int min_pairs, float* ref4, unsigned* moved, int* heads, size_t heads_bytes, void* stream);
+int sx_contact_pairs_project_headed(int n_dy, int n_st, const int* pairs, const void* ws, const float* y4,
+                                    const float* xs4, const float* fixed, const float* m_inv, float dHat,
+                                    float compliance, float cull_d2, long long* dx_fix, int* nc, int* status,
+                                    const int* conv, int iter, int variant, const int* heads, const unsigned* moved,
+                                    void* stream);
 int sx_contact_apply(int n_dy, float* y4, const float* fixed, long long* dx_fix, int* nc, const int* conv, int iter,
                      void* stream);
 

@@ -55,6 +55,8 @@ SIGNATURES = {
     "sx_set_programmatic_launch": ([I], I),
     "sx_jacobi_sweep_v": ([P, P, P, P, P, P, I, F, F, I, I, P], I),
     "sx_jacobi_sweep_mode": ([P, P, P, P, P, P, I, F, F, I, I, I, P], I),
+    "sx_jacobi_sweep_tracked": ([P, P, P, P, P, P, I, F, F, I, I, I, P, P, P, P], I),
+    "sx_jacobi_sweep_packed_tracked": ([P, P, P, P, P, P, P, I, F, F, I, I, I, P, P, P, P], I),
     "sx_velocity_update": ([P, P, P, P, I, F, F, P], I),
     "sx_compute_velocity": ([P, P, P, P, I, F, F, P], I),
     "sx_update_x": ([P, P, I, F, P], I),
@@ -99,6 +101,10 @@ SIGNATURES = {
     "sx_contact_pairs_project_variant_pipelined": ([I], I),
     "sx_contact_pairs_project_variant_info": ([I, P, P], I),
     "sx_contact_pairs_project_v": ([I, I, P, P, P, P, P, P, F, F, F, P, P, P, P, I, I, P], I),
+    "sx_contact_pairs_project_headed": ([I, I, P, P, P, P, P, P, F, F, F, P, P, P, P, I, I, P, P, P], I),
+    "sx_contact_pairs_project_default_variant": ([], I),
+    "sx_contact_pairs_heads_bytes": ([I, I], Z),
+    "sx_contact_pairs_heads": ([I, I, I, P, P, P, F, I, P, P, P, Z, P], I),
     "sx_contact_apply": ([I, P, P, P, P, P, I, P], I),
     "sx_batched_substep_variants": ([], I),
     "sx_batched_substep_variant_cluster": ([I], I),
@@ -201,7 +207,7 @@ def stream_handle(stream=None) -> int:
 # entry points whose int result is a value, not a status
 _VALUES = ("sx_version", "sx_mlp_param_count", "sx_mlp_bf16_count", "sx_jacobi_sweep_variants",
            "sx_jacobi_sweep_packed_forms", "sx_jacobi_sweep_default_variant", "sx_contact_pairs_project_variants",
-           "sx_contact_pairs_project_variant_pipelined", "sx_batched_substep_variants",
+           "sx_contact_pairs_project_default_variant", "sx_contact_pairs_project_variant_pipelined", "sx_batched_substep_variants",
            "sx_batched_substep_variant_cluster")
 
 

@@ -143,7 +143,9 @@ inline int tile_grid(K kernel, int n_verts) {
 // form but not bit-identical to it; validated against the oracle at the
 // position and residual tolerance of the substep instead.
 // STREAM: adjacency entries read with the evict-first policy (AdjInt2Stream).
-template <bool CHECK, int G = 2, int BLOCK = SW_BLOCK, bool BY = false, bool FAST = false, bool STREAM = false>
+// TRACK: keep the vertices' motion (SweepTrack).
+template <bool CHECK, int G = 2, int BLOCK = SW_BLOCK, bool BY = false, bool FAST = false, bool STREAM = false,
+          bool TRACK = false>
 __global__ void __launch_bounds__(BLOCK) jacobi_sweep_kernel(int V, const float4* __restrict__ x4,
                                                                 const float4* __restrict__ yin,
                                                                 float4* __restrict__ yout,
@@ -151,7 +153,7 @@ __global__ void __launch_bounds__(BLOCK) jacobi_sweep_kernel(int V, const float4
                                                                 const int* __restrict__ ptr,
                                                                 const int2* __restrict__ adj, float ks, float kb,
                                                                 int bend_y, const int* conv, int iter,
-                                                                double* __restrict__ partial) {
+                                                                double* __restrict__ partial, SweepTrack track) {
     pdl_entry();
     if (iteration_skipped(conv, iter)) return;  // grid-uniform
     static_assert(!CHECK || BLOCK == SW_BLOCK, "residual partials are per SW_BLOCK tile");
@@ -159,13 +161,18 @@ __global__ void __launch_bounds__(BLOCK) jacobi_sweep_kernel(int V, const float4
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const int v = tile * BLOCK + threadIdx.x;
     float c2 = 0.0f;  // sum of C^2 over this vertex's entries (CHECK)
-    if (v < V) {
+    const bool valid = v < V;
+    const int tracked = track_on<TRACK>(track);
+    float4 out = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (valid) {
         if (STREAM)
-            yout[v] = sweep_vertex_src<G, BY, FAST, CHECK, true>(v, x4, yin, fixed, __ldg(ptr + v), __ldg(ptr + v + 1),
-                                                                 AdjInt2Stream{adj}, ks, kb, bend_y, &c2);
+            out = sweep_vertex_src<G, BY, FAST, CHECK, true>(v, x4, yin, fixed, __ldg(ptr + v), __ldg(ptr + v + 1),
+                                                             AdjInt2Stream{adj}, ks, kb, bend_y, &c2);
         else
-            yout[v] = sweep_vertex<G, BY, FAST, CHECK, true>(v, x4, yin, fixed, ptr, adj, ks, kb, bend_y, &c2);
+            out = sweep_vertex<G, BY, FAST, CHECK, true>(v, x4, yin, fixed, ptr, adj, ks, kb, bend_y, &c2);
+        yout[v] = out;
     }
+    track_motion<TRACK>(track, tracked, v, valid, out);
     if (CHECK) block_residual_partial(c2, partial, tile);
     }
 }
@@ -174,7 +181,7 @@ __global__ void __launch_bounds__(BLOCK) jacobi_sweep_kernel(int V, const float4
 // leave the SMs short of warps (65 536 vertices are 13 warps per SM), L times
 // the threads and a shorter chain of dependent loads per thread; the same
 // sums in the same order, so bit-identical to jacobi_sweep_kernel.
-template <int L, int G, int BLOCK, bool BY = false, bool FAST = false>
+template <int L, int G, int BLOCK, bool BY = false, bool FAST = false, bool TRACK = false>
 __global__ void __launch_bounds__(BLOCK) jacobi_sweep_lanes_kernel(int V, const float4* __restrict__ x4,
                                                                       const float4* __restrict__ yin,
                                                                       float4* __restrict__ yout,
@@ -182,7 +189,7 @@ __global__ void __launch_bounds__(BLOCK) jacobi_sweep_lanes_kernel(int V, const 
                                                                       const int* __restrict__ ptr,
                                                                       const int2* __restrict__ adj, float ks,
                                                                       float kb, int bend_y, const int* conv, int iter,
-                                                                      double* __restrict__ partial) {
+                                                                      double* __restrict__ partial, SweepTrack track) {
     pdl_entry();
     if (iteration_skipped(conv, iter)) return;  // grid-uniform
     const long long t = (long long)blockIdx.x * BLOCK + threadIdx.x;
@@ -193,8 +200,10 @@ __global__ void __launch_bounds__(BLOCK) jacobi_sweep_lanes_kernel(int V, const 
         b = __ldg(ptr + v);
         e = __ldg(ptr + v + 1);
     }
+    const int tracked = track_on<TRACK>(track);
     const float4 out = sweep_vertex_lanes<L, G, BY, FAST, true>(v, valid, x4, yin, fixed, b, e, adj, ks, kb, bend_y);
     if (valid && (threadIdx.x & (L - 1)) == 0) yout[v] = out;
+    track_motion<TRACK>(track, tracked, v, valid, out);
 }
 
 // ---------------------------------------------------------------------------
@@ -432,7 +441,8 @@ extern "C" int sx_jacobi_sweep(const float* x4, const float* y_in4, float* y_out
     SX_REQUIRE(y_in4 != y_out4, "sx_jacobi_sweep: y_in4 and y_out4 must not alias");
     launch(bend_on_y ? jacobi_sweep_kernel<false, 2, SW_BLOCK, true> : jacobi_sweep_kernel<false>, sweep_blocks(n_verts),
            SW_BLOCK, 0, as_stream(stream), n_verts, (const float4*)x4, (const float4*)y_in4, (float4*)y_out4, fixed,
-           adj_ptr, (const int2*)adj, k_spring, k_bend, bend_on_y ? 1 : 0, (const int*)nullptr, 0, (double*)nullptr);
+           adj_ptr, (const int2*)adj, k_spring, k_bend, bend_on_y ? 1 : 0, (const int*)nullptr, 0, (double*)nullptr,
+           SweepTrack{});
     return check_launch("jacobi_sweep_kernel");
 }
 
@@ -441,22 +451,34 @@ extern "C" int sx_jacobi_sweep(const float* x4, const float* y_in4, float* y_out
 // read with the streaming cache policy.  All give bit-identical results.
 namespace sx {
 using SweepKernel = void (*)(int, const float4*, const float4*, float4*, const float*, const int*, const int2*, float,
-                            float, int, const int*, int, double*);
+                            float, int, const int*, int, double*, SweepTrack);
 struct SweepVariant {
     int g, block, lanes, stream;
     SweepKernel kern, kern_y;  // bending on x or y chosen at run time / bending on y
     SweepKernel fast, fast_y;  // the FAST arithmetic
+    SweepKernel track, track_y, track_fast, track_fast_y;  // the same four, keeping the vertices' motion
 };
 #define SX_SWEEP_VARIANT(G, B)                                                                                  \
     {G, B, 1, 0, jacobi_sweep_kernel<false, G, B>, jacobi_sweep_kernel<false, G, B, true>,                     \
-     jacobi_sweep_kernel<false, G, B, false, true>, jacobi_sweep_kernel<false, G, B, true, true>}
+     jacobi_sweep_kernel<false, G, B, false, true>, jacobi_sweep_kernel<false, G, B, true, true>,               \
+     jacobi_sweep_kernel<false, G, B, false, false, false, true>,                                               \
+     jacobi_sweep_kernel<false, G, B, true, false, false, true>,                                                \
+     jacobi_sweep_kernel<false, G, B, false, true, false, true>,                                                \
+     jacobi_sweep_kernel<false, G, B, true, true, false, true>}
 #define SX_SWEEP_LANES(L, G, B)                                                                                 \
     {G, B, L, 0, jacobi_sweep_lanes_kernel<L, G, B>, jacobi_sweep_lanes_kernel<L, G, B, true>,                 \
-     jacobi_sweep_lanes_kernel<L, G, B, false, true>, jacobi_sweep_lanes_kernel<L, G, B, true, true>}
+     jacobi_sweep_lanes_kernel<L, G, B, false, true>, jacobi_sweep_lanes_kernel<L, G, B, true, true>,           \
+     jacobi_sweep_lanes_kernel<L, G, B, false, false, true>,                                                    \
+     jacobi_sweep_lanes_kernel<L, G, B, true, false, true>,                                                     \
+     jacobi_sweep_lanes_kernel<L, G, B, false, true, true>, jacobi_sweep_lanes_kernel<L, G, B, true, true, true>}
 #define SX_SWEEP_STREAM(G, B)                                                                                   \
     {G, B, 1, 1, jacobi_sweep_kernel<false, G, B, false, false, true>,                                         \
      jacobi_sweep_kernel<false, G, B, true, false, true>, jacobi_sweep_kernel<false, G, B, false, true, true>,   \
-     jacobi_sweep_kernel<false, G, B, true, true, true>}
+     jacobi_sweep_kernel<false, G, B, true, true, true>,                                                        \
+     jacobi_sweep_kernel<false, G, B, false, false, true, true>,                                                \
+     jacobi_sweep_kernel<false, G, B, true, false, true, true>,                                                 \
+     jacobi_sweep_kernel<false, G, B, false, true, true, true>,                                                 \
+     jacobi_sweep_kernel<false, G, B, true, true, true, true>}
 static const SweepVariant kSweepVariants[] = {
     SX_SWEEP_VARIANT(2, 256), SX_SWEEP_VARIANT(1, 256), SX_SWEEP_VARIANT(4, 256), SX_SWEEP_VARIANT(2, 128),
     SX_SWEEP_VARIANT(2, 512), SX_SWEEP_VARIANT(4, 128), SX_SWEEP_VARIANT(1, 128), SX_SWEEP_VARIANT(3, 256),
@@ -511,20 +533,34 @@ extern "C" int sx_jacobi_sweep_v(const float* x4, const float* y_in4, float* y_o
                                 0, stream);
 }
 
-extern "C" int sx_jacobi_sweep_mode(const float* x4, const float* y_in4, float* y_out4, const float* fixed,
-                                    const int* adj_ptr, const int* adj, int n_verts, float k_spring, float k_bend,
-                                    int bend_on_y, int variant, int fast, void* stream) {
+extern "C" int sx_jacobi_sweep_tracked(const float* x4, const float* y_in4, float* y_out4, const float* fixed,
+                                       const int* adj_ptr, const int* adj, int n_verts, float k_spring, float k_bend,
+                                       int bend_on_y, int variant, int fast, const float* ref4, unsigned* moved,
+                                       const int* pair_counts, void* stream) {
     SX_REQUIRE(n_verts >= 0, "sx_jacobi_sweep_v: n_verts < 0");
     SX_REQUIRE(variant >= 0 && variant < kNumSweepVariants, "sx_jacobi_sweep_v: bad variant");
     if (n_verts == 0) return SX_OK;
     SX_REQUIRE(x4 && y_in4 && y_out4 && fixed && adj_ptr && adj, "sx_jacobi_sweep_v: null pointer");
     SX_REQUIRE(y_in4 != y_out4, "sx_jacobi_sweep_v: y_in4 and y_out4 must not alias");
+    SX_REQUIRE(!ref4 == !moved && !ref4 == !pair_counts,
+               "sx_jacobi_sweep_tracked: ref4, moved and pair_counts go together");
     const SweepVariant& sv = kSweepVariants[variant];
-    const SweepKernel k = fast ? (bend_on_y ? sv.fast_y : sv.fast) : (bend_on_y ? sv.kern_y : sv.kern);
+    const SweepKernel k = ref4   ? (fast ? (bend_on_y ? sv.track_fast_y : sv.track_fast)
+                                         : (bend_on_y ? sv.track_y : sv.track))
+                          : fast ? (bend_on_y ? sv.fast_y : sv.fast)
+                                 : (bend_on_y ? sv.kern_y : sv.kern);
     launch(k, grid_for((long long)n_verts * sv.lanes, sv.block), sv.block, 0, as_stream(stream), n_verts, (const float4*)x4,
            (const float4*)y_in4, (float4*)y_out4, fixed, adj_ptr, (const int2*)adj, k_spring, k_bend,
-           bend_on_y ? 1 : 0, (const int*)nullptr, 0, (double*)nullptr);
+           bend_on_y ? 1 : 0, (const int*)nullptr, 0, (double*)nullptr,
+           SweepTrack{(const float4*)ref4, moved, pair_counts});
     return check_launch("jacobi_sweep_kernel");
+}
+
+extern "C" int sx_jacobi_sweep_mode(const float* x4, const float* y_in4, float* y_out4, const float* fixed,
+                                    const int* adj_ptr, const int* adj, int n_verts, float k_spring, float k_bend,
+                                    int bend_on_y, int variant, int fast, void* stream) {
+    return sx_jacobi_sweep_tracked(x4, y_in4, y_out4, fixed, adj_ptr, adj, n_verts, k_spring, k_bend, bend_on_y,
+                                   variant, fast, nullptr, nullptr, nullptr, stream);
 }
 
 // ---------------------------------------------------------------------------
@@ -540,7 +576,7 @@ extern "C" int sx_jacobi_sweep_mode(const float* x4, const float* y_in4, float* 
 namespace sx {
 constexpr int kStagedCap = 4096;  // entries per block: 16 KB rest bits + 8 KB offsets
 
-template <int BLOCK, bool BY, bool FAST>
+template <int BLOCK, bool BY, bool FAST, bool TRACK>
 __global__ void __launch_bounds__(BLOCK) jacobi_sweep_staged_kernel(int V, const float4* __restrict__ x4,
                                                                        const float4* __restrict__ yin,
                                                                        float4* __restrict__ yout,
@@ -548,7 +584,8 @@ __global__ void __launch_bounds__(BLOCK) jacobi_sweep_staged_kernel(int V, const
                                                                        const int* __restrict__ ptr,
                                                                        const short* __restrict__ nbr16,
                                                                        const unsigned* __restrict__ rest32,
-                                                                       float ks, float kb, int bend_y) {
+                                                                       float ks, float kb, int bend_y,
+                                                                       SweepTrack track) {
     __shared__ __align__(16) unsigned s_rest[kStagedCap];
     __shared__ __align__(16) short s_nbr[kStagedCap];
     pdl_entry();
@@ -570,16 +607,19 @@ __global__ void __launch_bounds__(BLOCK) jacobi_sweep_staged_kernel(int V, const
         }
         __syncthreads();
         const int v = v0 + threadIdx.x;
-        if (v < V) {
+        const bool valid = v < V;
+        const int tracked = track_on<TRACK>(track);
+        float4 out = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (valid) {
             const int b = __ldg(ptr + v), e = __ldg(ptr + v + 1);
             float c2 = 0.0f;
-            yout[v] = staged ? sweep_vertex_src<2, BY, FAST, false, true>(v, x4, yin, fixed, b, e,
-                                                                          AdjPacked{s_nbr, s_rest, a0}, ks, kb,
-                                                                          bend_y, &c2)
-                             : sweep_vertex_src<2, BY, FAST, false, true>(v, x4, yin, fixed, b, e,
-                                                                          AdjPacked{nbr16, rest32, 0}, ks, kb,
-                                                                          bend_y, &c2);
+            out = staged ? sweep_vertex_src<2, BY, FAST, false, true>(v, x4, yin, fixed, b, e,
+                                                                      AdjPacked{s_nbr, s_rest, a0}, ks, kb, bend_y, &c2)
+                         : sweep_vertex_src<2, BY, FAST, false, true>(v, x4, yin, fixed, b, e,
+                                                                      AdjPacked{nbr16, rest32, 0}, ks, kb, bend_y, &c2);
+            yout[v] = out;
         }
+        track_motion<TRACK>(track, tracked, v, valid, out);
         __syncthreads();
     }
 }
@@ -588,7 +628,7 @@ __global__ void __launch_bounds__(BLOCK) jacobi_sweep_staged_kernel(int V, const
 // thread, G entries' loads issued together: 6 bytes per entry (two loads)
 // instead of the int2 entry's 8 and none of the staging's barriers.  Same
 // projection code, so bit-identical.
-template <int G, int BLOCK, bool BY, bool FAST>
+template <int G, int BLOCK, bool BY, bool FAST, bool TRACK>
 __global__ void __launch_bounds__(BLOCK) jacobi_sweep_packed_kernel(int V, const float4* __restrict__ x4,
                                                                        const float4* __restrict__ yin,
                                                                        float4* __restrict__ yout,
@@ -596,28 +636,42 @@ __global__ void __launch_bounds__(BLOCK) jacobi_sweep_packed_kernel(int V, const
                                                                        const int* __restrict__ ptr,
                                                                        const short* __restrict__ nbr16,
                                                                        const unsigned* __restrict__ rest32,
-                                                                       float ks, float kb, int bend_y) {
+                                                                       float ks, float kb, int bend_y,
+                                                                       SweepTrack track) {
     pdl_entry();
     const int v = blockIdx.x * BLOCK + threadIdx.x;
-    if (v >= V) return;
-    float c2 = 0.0f;
-    yout[v] = sweep_vertex_src<G, BY, FAST, false, true>(v, x4, yin, fixed, __ldg(ptr + v), __ldg(ptr + v + 1),
+    const bool valid = v < V;
+    const int tracked = track_on<TRACK>(track);
+    float4 out = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (valid) {
+        float c2 = 0.0f;
+        out = sweep_vertex_src<G, BY, FAST, false, true>(v, x4, yin, fixed, __ldg(ptr + v), __ldg(ptr + v + 1),
                                                          AdjPackedGlobal{nbr16, rest32}, ks, kb, bend_y, &c2);
+        yout[v] = out;
+    }
+    track_motion<TRACK>(track, tracked, v, valid, out);
 }
 
 // Forms of the packed sweep: 0 staged (sx_jacobi_sweep_packed), then the
 // direct kernel in several (entries per load batch, threads per block).
 using PackedKernel = void (*)(int, const float4*, const float4*, float4*, const float*, const int*, const short*,
-                              const unsigned*, float, float, int);
+                              const unsigned*, float, float, int, SweepTrack);
 struct PackedForm {
     int g, block;
-    PackedKernel kern, kern_y, fast, fast_y;
+    PackedKernel kern, kern_y, fast, fast_y, track, track_y, track_fast, track_fast_y;
 };
 #define SX_PACKED_FORM(G, B)                                                                                    \
-    {G, B, jacobi_sweep_packed_kernel<G, B, false, false>, jacobi_sweep_packed_kernel<G, B, true, false>,       \
-     jacobi_sweep_packed_kernel<G, B, false, true>, jacobi_sweep_packed_kernel<G, B, true, true>}
+    {G, B, jacobi_sweep_packed_kernel<G, B, false, false, false>,                                               \
+     jacobi_sweep_packed_kernel<G, B, true, false, false>, jacobi_sweep_packed_kernel<G, B, false, true, false>, \
+     jacobi_sweep_packed_kernel<G, B, true, true, false>, jacobi_sweep_packed_kernel<G, B, false, false, true>, \
+     jacobi_sweep_packed_kernel<G, B, true, false, true>, jacobi_sweep_packed_kernel<G, B, false, true, true>,  \
+     jacobi_sweep_packed_kernel<G, B, true, true, true>}
 static const PackedForm kPackedForms[] = {
-    {0, SW_BLOCK, nullptr, nullptr, nullptr, nullptr},  // staged: sx_jacobi_sweep_packed
+    {0, SW_BLOCK, jacobi_sweep_staged_kernel<SW_BLOCK, false, false, false>,
+     jacobi_sweep_staged_kernel<SW_BLOCK, true, false, false>, jacobi_sweep_staged_kernel<SW_BLOCK, false, true, false>,
+     jacobi_sweep_staged_kernel<SW_BLOCK, true, true, false>, jacobi_sweep_staged_kernel<SW_BLOCK, false, false, true>,
+     jacobi_sweep_staged_kernel<SW_BLOCK, true, false, true>, jacobi_sweep_staged_kernel<SW_BLOCK, false, true, true>,
+     jacobi_sweep_staged_kernel<SW_BLOCK, true, true, true>},  // staged: sx_jacobi_sweep_packed
     SX_PACKED_FORM(4, 256), SX_PACKED_FORM(2, 256), SX_PACKED_FORM(6, 256), SX_PACKED_FORM(4, 128),
     SX_PACKED_FORM(3, 512),
 };
@@ -625,44 +679,44 @@ static const PackedForm kPackedForms[] = {
 constexpr int kNumPackedForms = sizeof(kPackedForms) / sizeof(kPackedForms[0]);
 }  // namespace sx
 
+extern "C" int sx_jacobi_sweep_packed_tracked(const float* x4, const float* y_in4, float* y_out4, const float* fixed,
+                                              const int* adj_ptr, const short* nbr16, const unsigned* rest32,
+                                              int n_verts, float k_spring, float k_bend, int bend_on_y, int form,
+                                              int fast, const float* ref4, unsigned* moved, const int* pair_counts,
+                                              void* stream) {
+    SX_REQUIRE(form >= 0 && form < kNumPackedForms, "sx_jacobi_sweep_packed_v: bad form");
+    SX_REQUIRE(n_verts >= 0, "sx_jacobi_sweep_packed_v: n_verts < 0");
+    if (n_verts == 0) return SX_OK;
+    SX_REQUIRE(x4 && y_in4 && y_out4 && fixed && adj_ptr && nbr16 && rest32, "sx_jacobi_sweep_packed_v: null pointer");
+    SX_REQUIRE(y_in4 != y_out4, "sx_jacobi_sweep_packed_v: y_in4 and y_out4 must not alias");
+    SX_REQUIRE(!ref4 == !moved && !ref4 == !pair_counts,
+               "sx_jacobi_sweep_packed_tracked: ref4, moved and pair_counts go together");
+    SX_REQUIRE(form != 0 || (((uintptr_t)nbr16 & 15) == 0 && ((uintptr_t)rest32 & 15) == 0),
+               "sx_jacobi_sweep_packed: nbr16 and rest32 must be 16-byte aligned");
+    const PackedForm& pf = kPackedForms[form];
+    const PackedKernel k = ref4   ? (fast ? (bend_on_y ? pf.track_fast_y : pf.track_fast)
+                                          : (bend_on_y ? pf.track_y : pf.track))
+                           : fast ? (bend_on_y ? pf.fast_y : pf.fast)
+                                  : (bend_on_y ? pf.kern_y : pf.kern);
+    launch(k, grid_for(n_verts, pf.block), pf.block, 0, as_stream(stream), n_verts, (const float4*)x4,
+           (const float4*)y_in4, (float4*)y_out4, fixed, adj_ptr, nbr16, rest32, k_spring, k_bend, bend_on_y ? 1 : 0,
+           SweepTrack{(const float4*)ref4, moved, pair_counts});
+    return check_launch("jacobi_sweep_packed_kernel");
+}
+
 extern "C" int sx_jacobi_sweep_packed(const float* x4, const float* y_in4, float* y_out4, const float* fixed,
                                       const int* adj_ptr, const short* nbr16, const unsigned* rest32, int n_verts,
                                       float k_spring, float k_bend, int bend_on_y, int fast, void* stream) {
-    SX_REQUIRE(n_verts >= 0, "sx_jacobi_sweep_packed: n_verts < 0");
-    if (n_verts == 0) return SX_OK;
-    SX_REQUIRE(x4 && y_in4 && y_out4 && fixed && adj_ptr && nbr16 && rest32, "sx_jacobi_sweep_packed: null pointer");
-    SX_REQUIRE(y_in4 != y_out4, "sx_jacobi_sweep_packed: y_in4 and y_out4 must not alias");
-    SX_REQUIRE(((uintptr_t)nbr16 & 15) == 0 && ((uintptr_t)rest32 & 15) == 0,
-               "sx_jacobi_sweep_packed: nbr16 and rest32 must be 16-byte aligned");
-    using K = void (*)(int, const float4*, const float4*, float4*, const float*, const int*, const short*,
-                       const unsigned*, float, float, int);
-    const K k = fast ? (bend_on_y ? jacobi_sweep_staged_kernel<SW_BLOCK, true, true>
-                                  : jacobi_sweep_staged_kernel<SW_BLOCK, false, true>)
-                     : (bend_on_y ? jacobi_sweep_staged_kernel<SW_BLOCK, true, false>
-                                  : jacobi_sweep_staged_kernel<SW_BLOCK, false, false>);
-    launch(k, sweep_blocks(n_verts), SW_BLOCK, 0, as_stream(stream), n_verts, (const float4*)x4,
-           (const float4*)y_in4, (float4*)y_out4, fixed, adj_ptr, nbr16, rest32, k_spring, k_bend,
-           bend_on_y ? 1 : 0);
-    return check_launch("jacobi_sweep_staged_kernel");
+    return sx_jacobi_sweep_packed_tracked(x4, y_in4, y_out4, fixed, adj_ptr, nbr16, rest32, n_verts, k_spring, k_bend,
+                                          bend_on_y, 0, fast, nullptr, nullptr, nullptr, stream);
 }
 
 extern "C" int sx_jacobi_sweep_packed_v(const float* x4, const float* y_in4, float* y_out4, const float* fixed,
                                         const int* adj_ptr, const short* nbr16, const unsigned* rest32, int n_verts,
                                         float k_spring, float k_bend, int bend_on_y, int form, int fast,
                                         void* stream) {
-    SX_REQUIRE(form >= 0 && form < kNumPackedForms, "sx_jacobi_sweep_packed_v: bad form");
-    if (form == 0)
-        return sx_jacobi_sweep_packed(x4, y_in4, y_out4, fixed, adj_ptr, nbr16, rest32, n_verts, k_spring, k_bend,
-                                      bend_on_y, fast, stream);
-    SX_REQUIRE(n_verts >= 0, "sx_jacobi_sweep_packed_v: n_verts < 0");
-    if (n_verts == 0) return SX_OK;
-    SX_REQUIRE(x4 && y_in4 && y_out4 && fixed && adj_ptr && nbr16 && rest32, "sx_jacobi_sweep_packed_v: null pointer");
-    SX_REQUIRE(y_in4 != y_out4, "sx_jacobi_sweep_packed_v: y_in4 and y_out4 must not alias");
-    const PackedForm& pf = kPackedForms[form];
-    const PackedKernel k = fast ? (bend_on_y ? pf.fast_y : pf.fast) : (bend_on_y ? pf.kern_y : pf.kern);
-    launch(k, grid_for(n_verts, pf.block), pf.block, 0, as_stream(stream), n_verts, (const float4*)x4,
-           (const float4*)y_in4, (float4*)y_out4, fixed, adj_ptr, nbr16, rest32, k_spring, k_bend, bend_on_y ? 1 : 0);
-    return check_launch("jacobi_sweep_packed_kernel");
+    return sx_jacobi_sweep_packed_tracked(x4, y_in4, y_out4, fixed, adj_ptr, nbr16, rest32, n_verts, k_spring, k_bend,
+                                          bend_on_y, form, fast, nullptr, nullptr, nullptr, stream);
 }
 
 extern "C" int sx_jacobi_sweep_packed_forms(void) { return kNumPackedForms; }
@@ -1016,7 +1070,7 @@ extern "C" int sx_jacobi_sweep_checked_mode(const float* x4, const float* y_in4,
                              : jacobi_sweep_kernel<true, 2, SW_BLOCK, true>;
         launch(kc, gate ? tile_grid(kc, n_verts) : sweep_blocks(n_verts), SW_BLOCK, 0, s, n_verts,
                (const float4*)x4, (const float4*)y_in4, (float4*)y_out4, fixed, adj_ptr, (const int2*)adj, k_spring,
-               k_bend, 1, gate, iter, (double*)ws);
+               k_bend, 1, gate, iter, (double*)ws, SweepTrack{});
         int rc = check_launch("jacobi_sweep_kernel");
         if (rc) return rc;
         return residual_finish(n_verts, adj_ptr, ws, res3, conv, iter, tol, ref3, loop, n_iter, s);
@@ -1025,7 +1079,7 @@ extern "C" int sx_jacobi_sweep_checked_mode(const float* x4, const float* y_in4,
                          : jacobi_sweep_kernel<false, 2, SW_BLOCK, true>;
     launch(kp, gate ? tile_grid(kp, n_verts) : sweep_blocks(n_verts), SW_BLOCK, 0, s, n_verts,
            (const float4*)x4, (const float4*)y_in4, (float4*)y_out4, fixed, adj_ptr, (const int2*)adj, k_spring,
-           k_bend, 1, gate, iter, (double*)nullptr);
+           k_bend, 1, gate, iter, (double*)nullptr, SweepTrack{});
     return check_launch("jacobi_sweep_kernel");
 }
 

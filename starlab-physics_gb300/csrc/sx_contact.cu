@@ -553,8 +553,8 @@ __global__ void __launch_bounds__(128) collision_project_kernel(
 // without the faces __vt_dy skips (incident ones); every iteration then runs
 // one thread per pair.  The per-pair arithmetic is the same code as above and
 // accumulation is order independent, so the result equals the per-query walk.
-// Workspace: block totals, then meta[4] = {end of vt_st pairs, end of vt_dy
-// pairs, total pairs, unused}.
+// Workspace: block totals, then meta[6] = {end of vt_st pairs, end of vt_dy
+// pairs, total pairs, heads in use, heads with a bound, blocks that wrote them}.
 // ---------------------------------------------------------------------------
 constexpr int PB = 256;
 
@@ -649,7 +649,12 @@ __global__ void __launch_bounds__(PB) pairs_fill_kernel(int Vd, int Vs, int cap,
     const int off = block_off[blockIdx.x] + block_excl_scan(c, &tot);
     if (q == Vd) meta[0] = off;
     if (q == 2 * Vd) meta[1] = off;
-    if (q == Q) meta[2] = off;
+    if (q == Q) {
+        meta[2] = off;
+        meta[3] = 0;  // no heads of this list yet, none of them useful
+        meta[4] = 0;
+        meta[5] = 0;
+    }
     if (q >= Q || c == 0) return;
     int k = off;
     if (q < Vd) {
@@ -773,6 +778,147 @@ __device__ __forceinline__ void pair_points(const PairCtx& c, int t, int4 pr, V3
     x[3] = mk(tri[pr.w]);
 }
 
+// ---------------------------------------------------------------------------
+// Skipping the vertex-vs-cloth pairs that cannot have come into reach.
+//
+// Nearly all of those pairs are a vertex and a triangle of its own sheet a few
+// edges away: never in contact, and in every iteration tested again, which is
+// what a contact sweep over a large sheet costs.  Vertices move little within a
+// substep, so once per substep (sx_contact_pairs_heads, after the first
+// iteration) each chunk of 32 consecutive pairs gets a head: a motion mu below
+// which none of its pairs can come into reach, and the blocks of 32 vertices its
+// pairs touch.  The sweeps keep, per block, the largest squared displacement since
+// then (SweepTrack), and a projection given the heads passes over every chunk all
+// of whose blocks moved at most mu.  The chunk's other pairs are tested as ever.
+//
+// mu of a pair: with a lower bound D on its distance (the box's, and the gap
+// along the separating axes of sat_far, rounding subtracted as there) and c =
+// sqrt(cull_d2), motions of at most mu = (D - c) / 2 of its four vertices keep
+// the point farther than c from the triangle.  That a region's distance is at
+// least the true one needs a classifiable triangle (see classifiable), so mu is
+// also at most an eighth of the triangle's least altitude h, and the triangle has
+// to satisfy |n|^2 min|e|^4 > 1e-26 and |n|^2 max|e|^4 < 1e26: edges then change
+// by at most h / 4 <= a quarter of themselves and |n| by at most 9/16 of itself,
+// so the two products stay within factors 0.06 and 6 of what they were, inside
+// classifiable's 1e-30 and 1e30.  A skipped pair is therefore one that adds
+// nothing, and the sums are the same bit for bit.
+//
+// Head: 16 words, {mu^2 or -1, up to 15 blocks (the first repeated)}; -1 when a
+// pair has no such mu or the chunk touches more blocks (a mesh whose numbering
+// has no locality: its chunks are tested as before).
+// ---------------------------------------------------------------------------
+constexpr int HEAD_WORDS = 16;
+
+__device__ __forceinline__ float axis_gap(V3 m, V3 da, V3 db, V3 dc, float l1) {
+    const float mm = dot(m, m);
+    const float sa = dot(da, m), sb = dot(db, m), sc = dot(dc, m);
+    const float gap = fmaxf(fminf(fminf(sa, sb), sc), -fmaxf(fmaxf(sa, sb), sc)) - 1e-6f * (l1 * l1n(m));
+    return mm > 1e-30f ? gap * rsqrtf(mm) : 0.0f;
+}
+// -1: none
+__device__ __forceinline__ float pair_reach_motion(V3 p, V3 a, V3 b, V3 c, float cull) {
+    const V3 da = sub(a, p), db = sub(b, p), dc = sub(c, p);
+    const float l1 = fmaxf(fmaxf(l1n(da), l1n(db)), l1n(dc));
+    const V3 eab = sub(db, da), ebc = sub(dc, db), eca = sub(da, dc);
+    const V3 n = cross(eab, sub(dc, da));
+    const float nn = dot(n, n);
+    const float l0 = dot(eab, eab), l2 = dot(ebc, ebc), l3 = dot(eca, eca);
+    const float lo = fminf(fminf(l0, l2), l3), hi = fmaxf(fmaxf(l0, l2), l3);
+    float d = sqrtf(box_d2(p, a, b, c));
+    d = fmaxf(d, axis_gap(n, da, db, dc, l1));
+    d = fmaxf(d, axis_gap(cross(eab, n), da, db, dc, l1));
+    d = fmaxf(d, axis_gap(cross(ebc, n), da, db, dc, l1));
+    d = fmaxf(d, axis_gap(cross(eca, n), da, db, dc, l1));
+    // (a NaN in p is its block's motion in every tracked sweep)
+    const float mu = fminf(0.499f * (d * 0.9999f - cull * 1.0001f), 0.12f * sqrtf(nn / hi));
+    return mu > 0.0f && (nn * lo) * lo > 1e-26f && (nn * hi) * hi < 1e26f ? mu : -1.0f;
+}
+
+// meta[4] counts the heads with a mu, meta[5] the blocks that have added theirs;
+// the last one puts the heads to use, meta[3] = 1, when more than half have one.
+// With fewer than min_pairs vertex-vs-cloth pairs the projection costs less than
+// this, and the heads stay unwritten.
+__global__ void __launch_bounds__(256) pairs_heads_kernel(int V, int* meta, const int4* __restrict__ pairs,
+                                                          const float4* __restrict__ y4, float cull_d2, int min_pairs,
+                                                          float4* __restrict__ ref, unsigned* __restrict__ moved,
+                                                          int* __restrict__ heads) {
+    pdl_entry();
+    const int first = meta[0], last = meta[1];
+    const bool on = last - first >= min_pairs && cull_d2 > 0.0f;
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+    if (!on) {
+        if (tid == 0) meta[3] = 0;
+        return;
+    }
+    for (int v = tid; v < V; v += nt) {
+        ref[v] = y4[v];
+        if ((v & 31) == 0) moved[v >> 5] = 0u;
+    }
+    const int lane = threadIdx.x & 31;
+    const float cull = sqrtf(cull_d2);
+    const int nchunks = (last - first + 31) / 32;
+    int useful = 0;
+    for (int c = tid >> 5; c < nchunks; c += nt >> 5) {
+        const int t = first + 32 * c + lane;
+        const bool valid = t < last;
+        int b[4] = {0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff};
+        float mu = INFINITY;
+        if (valid) {
+            const int4 pr = pairs[t];
+            mu = pair_reach_motion(mk(y4[pr.x]), mk(y4[pr.y]), mk(y4[pr.z]), mk(y4[pr.w]), cull);
+            b[0] = pr.x >> 5;
+            b[1] = pr.y >> 5;
+            b[2] = pr.z >> 5;
+            b[3] = pr.w >> 5;
+        }
+        int word = 0;
+        if (__all_sync(0xffffffffu, mu > 0.0f)) {
+            const float least = __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(mu)));
+            // the distinct blocks in ascending order, block k to lane k + 1
+            int prev = -1, n = 0;
+            for (;; ++n) {
+                int next = 0x7fffffff;
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (b[k] > prev) next = min(next, b[k]);
+                next = __reduce_min_sync(0xffffffffu, next);
+                if (next == 0x7fffffff || n == HEAD_WORDS - 1) {
+                    if (next != 0x7fffffff) n = HEAD_WORDS;  // too many
+                    break;
+                }
+                if (lane == n + 1) word = next;
+                prev = next;
+            }
+            const int one = __shfl_sync(0xffffffffu, word, 1);
+            if (lane > n) word = one;
+            if (lane == 0) {
+                word = __float_as_int(n == HEAD_WORDS ? -1.0f : (least * least) * 0.999f);
+                if (n != HEAD_WORDS) ++useful;
+            }
+        } else if (lane == 0) {
+            word = __float_as_int(-1.0f);
+        }
+        if (lane < HEAD_WORDS) heads[(size_t)c * HEAD_WORDS + lane] = word;
+    }
+    if (useful) atomicAdd(meta + 4, useful);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(meta + 5, 1) == (int)gridDim.x - 1)
+        meta[3] = 2 * atomicAdd(meta + 4, 0) > nchunks ? 1 : 0;
+}
+// whether a chunk has to be tested
+__device__ __forceinline__ bool head_moved(const int* __restrict__ heads, const unsigned* __restrict__ moved, int c) {
+    const int4* h = reinterpret_cast<const int4*>(heads + (size_t)c * HEAD_WORDS);
+    const int4 q0 = h[0], q1 = h[1], q2 = h[2], q3 = h[3];
+    const float mu2 = __int_as_float(q0.x);
+    if (!(mu2 > 0.0f)) return true;
+    const int id[15] = {q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w, q2.x, q2.y, q2.z, q2.w, q3.x, q3.y, q3.z, q3.w};
+    unsigned m = 0u;
+#pragma unroll
+    for (int k = 0; k < 15; ++k) m = max(m, moved[id[k]]);
+    return !(__uint_as_float(m) <= mu2);
+}
+
 constexpr int PP_BLOCK = 256;
 
 // With the cull on, most pairs end at the box test, most of the rest at the
@@ -794,42 +940,39 @@ constexpr int PP_BLOCK = 256;
 // above, with the next step's pair records loaded while the current step's
 // positions are gathered, so that a warp waits on one round trip per step
 // instead of two.
-template <int U, int MINB, bool PIPE>
-__global__ void __launch_bounds__(PP_BLOCK, MINB) pairs_project_kernel(const int* __restrict__ meta,
-                                                                       const int4* __restrict__ pairs,
-                                                                       const float4* __restrict__ y4,
-                                                                       const float4* __restrict__ xs4,
-                                                                       const float* __restrict__ fixed,
-                                                                       const float* __restrict__ m_inv, float dHat,
-                                                                       float compliance, float cull_d2, long long* dx,
-                                                                       int* nc, int* status, const int* conv,
-                                                                       int iter) {
-    pdl_entry();
-    if (iteration_skipped(conv, iter)) return;
-    const PairCtx c{pairs, y4, xs4, fixed, m_inv, dHat, compliance, dx, nc, meta[0], meta[1]};
-    const int P = meta[2], st_end = c.st_end, dy_end = c.dy_end;
+//
+// HEADED: a warp first looks at the heads of its chunks, 32 of them together
+// (chunks gw, gw + nw, ...: neighbours, which move together, lie on different
+// warps), and takes only those that moved, or all of them where the heads are not
+// in use (a body with both loops spills and costs such a list 0.3 us).
+template <int U, bool PIPE, bool HEADED>
+__device__ __forceinline__ void pairs_project_body(const PairCtx& c, int P, bool in_use, float cull_d2, int* s1, int* s2,
+                                                   int* status, const int* __restrict__ heads,
+                                                   const unsigned* __restrict__ moved) {
+    const int4* __restrict__ pairs = c.pairs;
+    const float4* __restrict__ y4 = c.y4;
+    const int st_end = c.st_end, dy_end = c.dy_end;
     const bool cull = cull_d2 > 0.0f;  // without it every pair is classified
-    __shared__ int box_stack[PP_BLOCK / 32][32 * U + 32];
-    __shared__ int sat_stack[PP_BLOCK / 32][64];
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
-    int* s1 = box_stack[threadIdx.x >> 5];
-    int* s2 = sat_stack[threadIdx.x >> 5];
     int n1 = 0, n2 = 0;  // warp-uniform
     int bad = 0;
     const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
-    const bool split = PIPE && cull;
+    const bool split = HEADED || (PIPE && cull);
     const int first = split ? st_end : 0, last = split ? dy_end : P, chunk = cull ? 32 * U : 32;
     // the obstacle kinds go to the last warps, which have the fewest chunks
     const int H = split ? st_end + (P - dy_end) : 0;
-    int h0 = (nw - 1 - gw) * 32, base = first + gw * chunk;
+    int h0 = (nw - 1 - gw) * 32, base = HEADED ? last : first + gw * chunk;
     auto push = [&](int* s, int& n, int t, bool keep) {
         const unsigned m = __ballot_sync(0xffffffffu, keep);
         if (keep) s[n + __popc(m & below)] = t;
         n += __popc(m);
     };
+    const int nchunks = HEADED ? (dy_end - st_end + 31) / 32 : 0;
+    int c0 = gw;  // the first chunk of the next look
+    unsigned todo = 0u;
     int4 nx[U];
-    if (split) {
+    if (split && !HEADED) {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const int t = base + 32 * u + lane;
@@ -853,7 +996,7 @@ __global__ void __launch_bounds__(PP_BLOCK, MINB) pairs_project_kernel(const int
             // fill the second stack to at least 32 entries, or to what is left
             bool more = true;
             while (n2 < 32 && more) {
-                if (n1 >= 32 || (n1 > 0 && base >= last)) {
+                if (n1 >= 32 || (n1 > 0 && base >= last && (!HEADED || (todo == 0u && c0 >= nchunks)))) {
                     // the top of s1 through the separating-axis test onto s2
                     const int cnt = n1 < 32 ? n1 : 32;
                     const int q = lane < cnt ? s1[n1 - cnt + lane] : -1;
@@ -865,37 +1008,49 @@ __global__ void __launch_bounds__(PP_BLOCK, MINB) pairs_project_kernel(const int
                     }
                     n1 -= cnt;
                     push(s2, n2, q, keep);
-                } else if (base < last) {
-                    if (!cull) {
-                        push(s2, n2, base + lane, base + lane < last);
-                    } else {
-                        V3 z[U][4];
+                } else if (HEADED && c0 < nchunks && todo == 0u) {
+                    const int ch = c0 + lane * nw;
+                    todo = __ballot_sync(0xffffffffu, ch < nchunks && (!in_use || head_moved(heads, moved, ch)));
+                    c0 += 32 * nw;
+                } else if (!cull && base < last) {
+                    push(s2, n2, base + lane, base + lane < last);
+                    base += nw * chunk;
+                } else if ((HEADED && todo != 0u) || base < last) {
+                    // the next U x 32 pairs (with heads: U moved chunks)
+                    int q[U];
+                    V3 z[U][4];
 #pragma unroll
-                        for (int u = 0; u < U; ++u) {
-                            const int q = base + 32 * u + lane;
-                            if (PIPE) {
-                                z[u][0] = mk(y4[nx[u].x]);
-                                z[u][1] = mk(y4[nx[u].y]);
-                                z[u][2] = mk(y4[nx[u].z]);
-                                z[u][3] = mk(y4[nx[u].w]);
-                            } else if (q < last) {
-                                pair_points(c, q, pairs[q], z[u]);
-                            }
-                        }
-                        if (PIPE) {
-#pragma unroll
-                            for (int u = 0; u < U; ++u) {
-                                const int q = base + nw * chunk + 32 * u + lane;
-                                nx[u] = q < last ? pairs[q] : make_int4(0, 0, 0, 0);
-                            }
-                        }
-#pragma unroll
-                        for (int u = 0; u < U; ++u) {
-                            const int q = base + 32 * u + lane;
-                            push(s1, n1, q, q < last && !box_far(z[u][0], z[u][1], z[u][2], z[u][3], cull_d2));
+                    for (int u = 0; u < U; ++u) {
+                        q[u] = base + 32 * u + lane;
+                        if (HEADED) {
+                            q[u] = dy_end;
+                            if (todo != 0u) q[u] = st_end + 32 * (c0 + (__ffs(todo) - 33) * nw) + lane;
+                            todo &= todo - 1u;
+                            nx[u] = q[u] < dy_end ? pairs[q[u]] : make_int4(0, 0, 0, 0);
                         }
                     }
-                    base += nw * chunk;
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        if (PIPE) {
+                            z[u][0] = mk(y4[nx[u].x]);
+                            z[u][1] = mk(y4[nx[u].y]);
+                            z[u][2] = mk(y4[nx[u].z]);
+                            z[u][3] = mk(y4[nx[u].w]);
+                        } else if (q[u] < last) {
+                            pair_points(c, q[u], pairs[q[u]], z[u]);
+                        }
+                    }
+                    if (PIPE && !HEADED) {
+#pragma unroll
+                        for (int u = 0; u < U; ++u) {
+                            const int t = base + nw * chunk + 32 * u + lane;
+                            nx[u] = t < last ? pairs[t] : make_int4(0, 0, 0, 0);
+                        }
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+                        push(s1, n1, q[u], q[u] < last && !box_far(z[u][0], z[u][1], z[u][2], z[u][3], cull_d2));
+                    if (!HEADED) base += nw * chunk;
                 } else {
                     more = false;
                 }
@@ -912,10 +1067,32 @@ __global__ void __launch_bounds__(PP_BLOCK, MINB) pairs_project_kernel(const int
             __syncwarp();
         }
         if (t >= 0)
-            pair_project(t < st_end ? VT_ST : t < dy_end ? VT_DY : TV_ST, pr, x, fixed, m_inv, dHat, compliance, dx,
-                         nc, &bad);
+            pair_project(t < st_end ? VT_ST : t < dy_end ? VT_DY : TV_ST, pr, x, c.fixed, c.m_inv, c.dHat,
+                         c.compliance, c.dx, c.nc, &bad);
     }
     if (bad) atomicOr(status, SX_STATUS_FIXED_RANGE);
+}
+
+template <int U, int MINB, bool PIPE, bool HEADED>
+__global__ void __launch_bounds__(PP_BLOCK, MINB) pairs_project_kernel(const int* __restrict__ meta,
+                                                                       const int4* __restrict__ pairs,
+                                                                       const float4* __restrict__ y4,
+                                                                       const float4* __restrict__ xs4,
+                                                                       const float* __restrict__ fixed,
+                                                                       const float* __restrict__ m_inv, float dHat,
+                                                                       float compliance, float cull_d2, long long* dx,
+                                                                       int* nc, int* status, const int* conv,
+                                                                       int iter, const int* __restrict__ heads,
+                                                                       const unsigned* __restrict__ moved) {
+    pdl_entry();
+    if (iteration_skipped(conv, iter)) return;
+    const PairCtx c{pairs, y4, xs4, fixed, m_inv, dHat, compliance, dx, nc, meta[0], meta[1]};
+    __shared__ int box_stack[PP_BLOCK / 32][32 * U + 32];
+    __shared__ int sat_stack[PP_BLOCK / 32][64];
+    int* s1 = box_stack[threadIdx.x >> 5];
+    int* s2 = sat_stack[threadIdx.x >> 5];
+    pairs_project_body<U, PIPE, HEADED>(c, meta[2], HEADED && heads_in_use(meta) != 0, cull_d2, s1, s2, status, heads,
+                                        moved);
 }
 
 // update_dx (XPBD.py:384-387) from the fixed-point accumulators; clears them.
@@ -2005,14 +2182,17 @@ static int sm_count() {
 // narrow phase and FP64 fixed point the same launches took 7.8 / 9.8 / 19.0.
 struct PairsProjectVariant {
     int unroll, blocks_per_sm, pipelined;
-    decltype(&pairs_project_kernel<1, 4, false>) kern;
+    decltype(&pairs_project_kernel<1, 4, false, false>) kern, headed;
 };
+#define SX_PAIRS_VARIANT(U, B, MINB, PIPE)                                                             \
+    {U, B, PIPE ? 1 : 0, pairs_project_kernel<U, MINB, PIPE, false>,                                    \
+     pairs_project_kernel<U, MINB, PIPE, PIPE>}  // the stacked form tests every pair
 static const PairsProjectVariant kPairsProjectVariants[] = {
-    {2, 3, 0, pairs_project_kernel<2, 3, false>}, {1, 4, 0, pairs_project_kernel<1, 4, false>},
-    {2, 6, 0, pairs_project_kernel<2, 3, false>}, {4, 2, 0, pairs_project_kernel<4, 2, false>},
-    {2, 3, 1, pairs_project_kernel<2, 3, true>},  {1, 4, 1, pairs_project_kernel<1, 4, true>},
-    {2, 4, 1, pairs_project_kernel<2, 4, true>},
+    SX_PAIRS_VARIANT(2, 3, 3, false), SX_PAIRS_VARIANT(1, 4, 4, false), SX_PAIRS_VARIANT(2, 6, 3, false),
+    SX_PAIRS_VARIANT(4, 2, 2, false), SX_PAIRS_VARIANT(2, 3, 3, true),  SX_PAIRS_VARIANT(1, 4, 4, true),
+    SX_PAIRS_VARIANT(2, 4, 4, true),
 };
+#undef SX_PAIRS_VARIANT
 constexpr int kNumPairsProjectVariants = sizeof(kPairsProjectVariants) / sizeof(kPairsProjectVariants[0]);
 constexpr int kPairsProjectDefault = 4;
 
@@ -2032,22 +2212,34 @@ extern "C" int sx_contact_pairs_project_variant_pipelined(int variant) {
     return kPairsProjectVariants[variant].pipelined;
 }
 
-extern "C" int sx_contact_pairs_project_v(int n_dy, int n_st, const int* pairs, const void* ws, const float* y4,
-                                          const float* xs4, const float* fixed, const float* m_inv, float dHat,
-                                          float compliance, float cull_d2, long long* dx_fix, int* nc, int* status,
-                                          const int* conv, int iter, int variant, void* stream) {
+extern "C" int sx_contact_pairs_project_headed(int n_dy, int n_st, const int* pairs, const void* ws, const float* y4,
+                                               const float* xs4, const float* fixed, const float* m_inv, float dHat,
+                                               float compliance, float cull_d2, long long* dx_fix, int* nc,
+                                               int* status, const int* conv, int iter, int variant, const int* heads,
+                                               const unsigned* moved, void* stream) {
     SX_REQUIRE(variant >= 0 && variant < kNumPairsProjectVariants, "sx_contact_pairs_project_v: bad variant");
     SX_REQUIRE(n_dy >= 0 && n_st >= 0, "sx_contact_pairs_project: bad sizes");
     if (n_dy == 0) return SX_OK;
     SX_REQUIRE(pairs && ws && y4 && fixed && m_inv && dx_fix && nc && status,
                "sx_contact_pairs_project: null pointer");
     SX_REQUIRE(n_st == 0 || xs4, "sx_contact_pairs_project: null static positions");
+    SX_REQUIRE(!heads == !moved && ((uintptr_t)heads & 15) == 0,
+               "sx_contact_pairs_project_headed: heads (16-byte aligned) and moved go together");
     PairsWs w = pairs_ws(const_cast<void*>(ws), n_dy, n_st);
     const PairsProjectVariant& pv = kPairsProjectVariants[variant];
-    launch(pv.kern, sm_count() * pv.blocks_per_sm, PP_BLOCK, 0, as_stream(stream), (const int*)w.meta,
+    launch(heads ? pv.headed : pv.kern, sm_count() * pv.blocks_per_sm, PP_BLOCK, 0, as_stream(stream),
+           (const int*)w.meta,
            (const int4*)pairs, (const float4*)y4, (const float4*)xs4, fixed, m_inv, dHat, compliance, cull_d2, dx_fix,
-           nc, status, conv, iter);
+           nc, status, conv, iter, heads, moved);
     return check_launch("pairs_project_kernel");
+}
+
+extern "C" int sx_contact_pairs_project_v(int n_dy, int n_st, const int* pairs, const void* ws, const float* y4,
+                                          const float* xs4, const float* fixed, const float* m_inv, float dHat,
+                                          float compliance, float cull_d2, long long* dx_fix, int* nc, int* status,
+                                          const int* conv, int iter, int variant, void* stream) {
+    return sx_contact_pairs_project_headed(n_dy, n_st, pairs, ws, y4, xs4, fixed, m_inv, dHat, compliance, cull_d2,
+                                           dx_fix, nc, status, conv, iter, variant, nullptr, nullptr, stream);
 }
 
 extern "C" int sx_contact_pairs_project(int n_dy, int n_st, const int* pairs, const void* ws, const float* y4,
@@ -2056,6 +2248,27 @@ extern "C" int sx_contact_pairs_project(int n_dy, int n_st, const int* pairs, co
                                         const int* conv, int iter, void* stream) {
     return sx_contact_pairs_project_v(n_dy, n_st, pairs, ws, y4, xs4, fixed, m_inv, dHat, compliance, cull_d2, dx_fix,
                                       nc, status, conv, iter, kPairsProjectDefault, stream);
+}
+
+extern "C" int sx_contact_pairs_project_default_variant(void) { return kPairsProjectDefault; }
+
+extern "C" size_t sx_contact_pairs_heads_bytes(int n_dy, int cap) {
+    if (n_dy < 0 || cap < 1) return 0;
+    return ((size_t)n_dy * cap + 31) / 32 * HEAD_WORDS * sizeof(int) + 16;
+}
+
+extern "C" int sx_contact_pairs_heads(int n_dy, int n_st, int cap, const int* pairs, void* ws, const float* y4,
+                                      float cull_d2, int min_pairs, float* ref4, unsigned* moved, int* heads,
+                                      size_t heads_bytes, void* stream) {
+    SX_REQUIRE(n_dy >= 0 && n_st >= 0 && cap >= 1, "sx_contact_pairs_heads: bad sizes");
+    if (n_dy == 0) return SX_OK;
+    SX_REQUIRE(pairs && ws && y4 && ref4 && moved && heads, "sx_contact_pairs_heads: null pointer");
+    SX_REQUIRE(((uintptr_t)heads & 15) == 0 && heads_bytes >= sx_contact_pairs_heads_bytes(n_dy, cap),
+               "sx_contact_pairs_heads: heads must be 16-byte aligned and sx_contact_pairs_heads_bytes long");
+    PairsWs w = pairs_ws(ws, n_dy, n_st);
+    launch(pairs_heads_kernel, resident_blocks(pairs_heads_kernel, 256), 256, 0, as_stream(stream), n_dy, w.meta,
+           (const int4*)pairs, (const float4*)y4, cull_d2, min_pairs, (float4*)ref4, moved, heads);
+    return check_launch("pairs_heads_kernel");
 }
 
 extern "C" int sx_contact_apply(int n_dy, float* y4, const float* fixed, long long* dx_fix, int* nc, const int* conv,

@@ -341,4 +341,35 @@ __device__ __forceinline__ float4 sweep_vertex(int v, const float4* __restrict__
                                                       AdjInt2{adj}, ks, kb, bend_y, c2);
 }
 
+// Motion of the vertices since a reference: the largest squared displacement of
+// each block of 32 vertices, as float bits in moved[], raised by every tracked
+// sweep.  The vertices of a warp lie in one block; every lane of the warp calls
+// it.  A template flag, not a test of ref: the 4-lane sweep of a 64 x 64 sheet is
+// short enough for the test alone to cost it 0.25 of its 4.4 us.  Sweeps of a
+// list whose heads stand unused track nothing.
+struct SweepTrack {
+    const float4* ref;
+    unsigned* moved;
+    const int* meta;
+};
+// whether the heads of a pair list (its meta words) are in use
+__device__ __forceinline__ int heads_in_use(const int* meta) { return meta[3]; }
+// on: read before the sweep's loads and needed after them
+template <bool TRACK>
+__device__ __forceinline__ int track_on(const SweepTrack& t) {
+    return TRACK ? heads_in_use(t.meta) : 0;
+}
+template <bool TRACK>
+__device__ __forceinline__ void track_motion(const SweepTrack& t, int on, int v, bool valid, float4 out) {
+    if (!TRACK || on == 0) return;
+    unsigned d2 = 0u;
+    if (valid) {
+        const float4 ref = __ldg(t.ref + v);
+        const float dx = out.x - ref.x, dy = out.y - ref.y, dz = out.z - ref.z;
+        d2 = __float_as_uint((dx * dx + dy * dy) + dz * dz);  // a NaN is the largest
+    }
+    const unsigned m = __reduce_max_sync(0xffffffffu, d2);
+    if ((threadIdx.x & 31) == 0 && m != 0u) atomicMax(t.moved + (v >> 5), m);
+}
+
 }  // namespace sx
