@@ -620,7 +620,7 @@ __device__ __forceinline__ void cell_range(float qa, float qb, float o, float c,
     *i1 = (int)fminf(f1, (float)(kGridRes - 1));
 }
 
-// One warp per query.  The warp walks the (x, y) columns of the query's cell
+// A warp takes one query after the other.  It walks the (x, y) columns of the query's cell
 // range in descending order.  In each column, lane l takes cell z = 31 - l, so
 // that ascending lanes are the reference's descending-z visiting order: the
 // occupied cells' leaf boxes are tested at once, a warp scan lays the faces of
@@ -629,7 +629,19 @@ __device__ __forceinline__ void cell_range(float qa, float qb, float o, float c,
 // ballot places each overlapping face after those of lower lanes, so
 // candidates come out in descending cell order and, within a cell, in sorted
 // face order -- the reference's visiting order -- with every lane busy.
+//
+// Instruction issue bounds it (a thousand a query, 2.3 a cycle and SM, DRAM idle),
+// so: the cell ranges' divisions are done once, an axis a lane; cells that pass
+// with 20 faces or more on average (CT_LONG_CELL; a 256 x 256 sheet has 150) are
+// scanned one after the other, which takes half the instructions per 32 faces of
+// the search for each lane's cell (63 against 77 us, the crossing is flat between
+// 12 and 20); empty runs of columns are left at once; and one resident wave of
+// blocks keeps the occupancy words instead of loading them for every 8 queries.
+// 65 536 queries of a sheet on itself 80.5 -> 63 us, on a sphere 26 -> 18,
+// 4096 on a box of 12 faces 14.7 -> 10.1; 6 blocks an SM (4: 70 us, 8: 62 but 25
+// on the sphere).
 constexpr int CT_BLOCK = 256;
+constexpr int CT_LONG_CELL = 20;
 
 __device__ __forceinline__ int warp_incl_scan(int v, int lane) {
 #pragma unroll
@@ -651,7 +663,7 @@ __device__ __forceinline__ int warp_owner(int incl, int k) {
 // EDGE: query q is the box of edge q (endpoints edges[2q], edges[2q+1] in p4)
 // grown by pad (XPBD.py:221-232), else the box p4[q] +- pad.
 template <bool EDGE>
-__global__ void __launch_bounds__(CT_BLOCK, 4) cell_traverse_kernel(
+__global__ void __launch_bounds__(CT_BLOCK, 6) cell_traverse_kernel(
     int Q, const float4* __restrict__ p4, float pad, const float* __restrict__ grid8, const float* __restrict__ box6,
     const float4* __restrict__ nmin4, const float4* __restrict__ nmax4, const int* __restrict__ prefix,
     const float4* __restrict__ frec, int cap, int* __restrict__ cand, int* __restrict__ num, int* status,
@@ -662,97 +674,128 @@ __global__ void __launch_bounds__(CT_BLOCK, 4) cell_traverse_kernel(
     const unsigned* gocc = reinterpret_cast<const unsigned*>(grid8) + kGridHeader;
     for (int k = threadIdx.x; k < kGridRes * kGridRes; k += blockDim.x) occ[k] = gocc[k];
     __syncthreads();
-    const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (q >= Q) return;  // warp-uniform
-    V3 a, b;
-    if (EDGE) {
-        const V3 p0 = mk(p4[edges[2 * q]]), p1 = mk(p4[edges[2 * q + 1]]);
-        const V3 lo = vmin(p0, p1), hi = vmax(p0, p1);
-        a = V3{lo.x - pad, lo.y - pad, lo.z - pad};
-        b = V3{hi.x + pad, hi.y + pad, hi.z + pad};
-    } else {
-        const V3 p = mk(p4[q]);
-        a = V3{p.x - pad, p.y - pad, p.z - pad};
-        b = V3{p.x + pad, p.y + pad, p.z + pad};
-    }
-    const V3 pos = scale(0.5f, add(a, b));
-    const V3 cs{grid8[0], grid8[1], grid8[2]}, org{box6[0], box6[1], box6[2]};
-    const int ix = f2i_sat((pos.x - org.x) / cs.x), iy = f2i_sat((pos.y - org.y) / cs.y),
-              iz = f2i_sat((pos.z - org.z) / cs.z);
-    const int cid =
-        (int)((unsigned)ix * (unsigned)(kGridRes * kGridRes) + (unsigned)iy * (unsigned)kGridRes + (unsigned)iz);
-    int count = 0;  // warp-uniform
-    int* out = cand + (size_t)q * cap;
-    if (cid <= kNumCells - 1) {  // the reference's skip rule (lbvh_cell.py:665)
-        int x0, x1, y0, y1, z0, z1;
-        cell_range(a.x, b.x, org.x, cs.x, grid8[3], &x0, &x1);
-        cell_range(a.y, b.y, org.y, cs.y, grid8[4], &y0, &y1);
-        cell_range(a.z, b.z, org.z, cs.z, grid8[5], &z0, &z1);
-        if (z0 <= z1 && x0 <= x1 && y0 <= y1) {
-            const unsigned zmask = (z1 == 31 ? 0xffffffffu : ((1u << (z1 + 1)) - 1u)) & ~((1u << z0) - 1u);
-            const int ny = y1 - y0 + 1, ncol = (x1 - x0 + 1) * ny;
-            // columns in visiting order (x descending, then y descending), 32 at a time
-            for (int c0 = 0; c0 < ncol; c0 += 32) {
-                unsigned cm = 0u;  // this lane's column: occupied cells within the z range
-                if (c0 + lane < ncol) {
-                    const int cc = c0 + lane;
-                    cm = occ[(x1 - cc / ny) * kGridRes + (y1 - cc % ny)] & zmask;
-                }
-                const int cn = __popc(cm);
-                const int cincl = warp_incl_scan(cn, lane);
-                const int ctotal = __shfl_sync(0xffffffffu, cincl, 31);
-                // the occupied cells of these columns end to end (z descending
-                // within a column), 32 at a time: lane k takes the k-th
-                for (int k0 = 0; k0 < ctotal; k0 += 32) {
-                    const int k = k0 + lane;
-                    const int oc = warp_owner(cincl, k);
-                    const unsigned m = __shfl_sync(0xffffffffu, cm, oc);
-                    const int rank = k - (__shfl_sync(0xffffffffu, cincl, oc) - __shfl_sync(0xffffffffu, cn, oc));
-                    int start = 0, n = 0;
-                    if (k < ctotal) {
-                        // position of the rank-th highest set bit of m
-                        int cz = 0;
-#pragma unroll
-                        for (int step = 16; step >= 1; step >>= 1)
-                            if (__popc(m >> (cz + step)) >= rank + 1) cz += step;
-                        const int cc = c0 + oc;
-                        const int i = (x1 - cc / ny) * kGridRes * kGridRes + (y1 - cc % ny) * kGridRes + cz;
-                        const int leaf = i + kNumCells - 1;
-                        if (overlap(a, b, mk(nmin4[leaf]), mk(nmax4[leaf]))) {
-                            start = i == 0 ? 0 : prefix[i - 1];
-                            n = prefix[i] - start;
-                        }
+    const int lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
+    const unsigned below = (1u << lane) - 1u;
+    // lanes 0, 1, 2 (and all further ones, as 2): this lane's axis
+    const int axis = min(lane, 2);
+    const float cell = grid8[axis], reach = grid8[3 + axis], origin = box6[axis];
+    const float* p = reinterpret_cast<const float*>(p4) + axis;
+    for (int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < Q; q += nw) {  // warp-uniform
+        float qa, qb;
+        if (EDGE) {
+            const float p0 = p[4 * (size_t)edges[2 * q]], p1 = p[4 * (size_t)edges[2 * q + 1]];
+            qa = fminf(p0, p1) - pad;
+            qb = fmaxf(p0, p1) + pad;
+        } else {
+            const float p0 = p[4 * (size_t)q];
+            qa = p0 - pad;
+            qb = p0 + pad;
+        }
+        const int ic = f2i_sat((0.5f * (qa + qb) - origin) / cell);
+        int i0, i1;
+        cell_range(qa, qb, origin, cell, reach, &i0, &i1);
+        const int ix = __shfl_sync(0xffffffffu, ic, 0), iy = __shfl_sync(0xffffffffu, ic, 1),
+                  iz = __shfl_sync(0xffffffffu, ic, 2);
+        const V3 a{__shfl_sync(0xffffffffu, qa, 0), __shfl_sync(0xffffffffu, qa, 1), __shfl_sync(0xffffffffu, qa, 2)};
+        const V3 b{__shfl_sync(0xffffffffu, qb, 0), __shfl_sync(0xffffffffu, qb, 1), __shfl_sync(0xffffffffu, qb, 2)};
+        const int cid =
+            (int)((unsigned)ix * (unsigned)(kGridRes * kGridRes) + (unsigned)iy * (unsigned)kGridRes + (unsigned)iz);
+        int count = 0;  // warp-uniform
+        int* out = cand + (size_t)q * cap;
+        if (cid <= kNumCells - 1) {  // the reference's skip rule (lbvh_cell.py:665)
+            const int x0 = __shfl_sync(0xffffffffu, i0, 0), x1 = __shfl_sync(0xffffffffu, i1, 0);
+            const int y0 = __shfl_sync(0xffffffffu, i0, 1), y1 = __shfl_sync(0xffffffffu, i1, 1);
+            const int z0 = __shfl_sync(0xffffffffu, i0, 2), z1 = __shfl_sync(0xffffffffu, i1, 2);
+            if (z0 <= z1 && x0 <= x1 && y0 <= y1) {
+                const unsigned zmask = (z1 == 31 ? 0xffffffffu : ((1u << (z1 + 1)) - 1u)) & ~((1u << z0) - 1u);
+                const int ny = y1 - y0 + 1, ncol = (x1 - x0 + 1) * ny;
+                // columns in visiting order (x descending, then y descending), 32 at a time
+                for (int c0 = 0; c0 < ncol; c0 += 32) {
+                    unsigned cm = 0u;  // this lane's column: occupied cells within the z range
+                    if (c0 + lane < ncol) {
+                        const int cc = c0 + lane;
+                        cm = occ[(x1 - cc / ny) * kGridRes + (y1 - cc % ny)] & zmask;
                     }
-                    const int incl = warp_incl_scan(n, lane);  // faces of the passing cells, in order
-                    const int total = __shfl_sync(0xffffffffu, incl, 31);
-                    for (int f0 = 0; f0 < total; f0 += 32) {
-                        const int f = f0 + lane;
-                        const int lo = warp_owner(incl, f);
-                        const int o_incl = __shfl_sync(0xffffffffu, incl, lo);
-                        const int o_n = __shfl_sync(0xffffffffu, n, lo);
-                        const int o_start = __shfl_sync(0xffffffffu, start, lo);
-                        bool hit = false;
-                        float4 fa = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (f < total) {
-                            const int j = o_start + (f - (o_incl - o_n));
-                            fa = frec[2 * j];
-                            hit = overlap(a, b, mk(fa), mk(frec[2 * j + 1]));
+                    if (!__any_sync(0xffffffffu, cm != 0u)) continue;
+                    const int cn = __popc(cm);
+                    const int cincl = warp_incl_scan(cn, lane);
+                    const int ctotal = __shfl_sync(0xffffffffu, cincl, 31);
+                    // the occupied cells of these columns end to end (z descending
+                    // within a column), 32 at a time: lane k takes the k-th
+                    for (int k0 = 0; k0 < ctotal; k0 += 32) {
+                        const int k = k0 + lane;
+                        const int oc = warp_owner(cincl, k);
+                        const unsigned m = __shfl_sync(0xffffffffu, cm, oc);
+                        const int rank = k - (__shfl_sync(0xffffffffu, cincl, oc) - __shfl_sync(0xffffffffu, cn, oc));
+                        int start = 0, n = 0;
+                        if (k < ctotal) {
+                            // position of the rank-th highest set bit of m
+                            int cz = 0;
+    #pragma unroll
+                            for (int step = 16; step >= 1; step >>= 1)
+                                if (__popc(m >> (cz + step)) >= rank + 1) cz += step;
+                            const int cc = c0 + oc;
+                            const int i = (x1 - cc / ny) * kGridRes * kGridRes + (y1 - cc % ny) * kGridRes + cz;
+                            const int leaf = i + kNumCells - 1;
+                            if (overlap(a, b, mk(nmin4[leaf]), mk(nmax4[leaf]))) {
+                                start = i == 0 ? 0 : prefix[i - 1];
+                                n = prefix[i] - start;
+                            }
                         }
-                        const unsigned hits = __ballot_sync(0xffffffffu, hit);
-                        if (hit) {
-                            const int slot = count + __popc(hits & ((1u << lane) - 1u));
-                            if (slot < cap) out[slot] = __float_as_int(fa.w);
+                        unsigned full = __ballot_sync(0xffffffffu, n > 0);
+                        const int total = __reduce_add_sync(0xffffffffu, n);
+                        if (total >= CT_LONG_CELL * __popc(full)) {
+                            // long cells: one after the other
+                            for (; full != 0u; full &= full - 1u) {
+                                const int l = __ffs(full) - 1;
+                                const int o_start = __shfl_sync(0xffffffffu, start, l);
+                                const int o_n = __shfl_sync(0xffffffffu, n, l);
+                                for (int f0 = 0; f0 < o_n; f0 += 32) {
+                                    bool hit = false;
+                                    float4 fa = make_float4(0.f, 0.f, 0.f, 0.f);
+                                    if (f0 + lane < o_n) {
+                                        fa = frec[2 * (o_start + f0 + lane)];
+                                        hit = overlap(a, b, mk(fa), mk(frec[2 * (o_start + f0 + lane) + 1]));
+                                    }
+                                    const unsigned hits = __ballot_sync(0xffffffffu, hit);
+                                    if (hit) {
+                                        const int slot = count + __popc(hits & below);
+                                        if (slot < cap) out[slot] = __float_as_int(fa.w);
+                                    }
+                                    count += __popc(hits);
+                                }
+                            }
+                            continue;
                         }
-                        count += __popc(hits);
+                        const int incl = warp_incl_scan(n, lane);  // faces of the passing cells, in order
+                        for (int f0 = 0; f0 < total; f0 += 32) {
+                            const int f = f0 + lane;
+                            const int lo = warp_owner(incl, f);
+                            const int o_incl = __shfl_sync(0xffffffffu, incl, lo);
+                            const int o_n = __shfl_sync(0xffffffffu, n, lo);
+                            const int o_start = __shfl_sync(0xffffffffu, start, lo);
+                            bool hit = false;
+                            float4 fa = make_float4(0.f, 0.f, 0.f, 0.f);
+                            if (f < total) {
+                                const int j = o_start + (f - (o_incl - o_n));
+                                fa = frec[2 * j];
+                                hit = overlap(a, b, mk(fa), mk(frec[2 * j + 1]));
+                            }
+                            const unsigned hits = __ballot_sync(0xffffffffu, hit);
+                            if (hit) {
+                                const int slot = count + __popc(hits & below);
+                                if (slot < cap) out[slot] = __float_as_int(fa.w);
+                            }
+                            count += __popc(hits);
+                        }
                     }
                 }
             }
         }
-    }
-    if (lane == 0) {
-        num[q] = count;
-        if (count > cap) atomicOr(status, SX_STATUS_CAND_OVERFLOW);
+        if (lane == 0) {
+            num[q] = count;
+            if (count > cap) atomicOr(status, SX_STATUS_CAND_OVERFLOW);
+        }
     }
 }
 
@@ -1354,6 +1397,13 @@ extern "C" int sx_cell_bvh_build(const float* fmin4, const float* fmax4, int n_f
     return check_launch("cell_top_refit_kernel");
 }
 
+// a warp a query, at most one resident wave of blocks
+template <typename K>
+static int traverse_grid(K kernel, int queries) {
+    const int g = grid_for(32LL * queries, CT_BLOCK), cap = resident_blocks(kernel, CT_BLOCK);
+    return g < cap ? g : cap;
+}
+
 extern "C" int sx_cell_bvh_traverse(const float* p4, int n_queries, float padding, const float* grid8,
                                     const float* origin_box6, const float* nmin4, const float* nmax4,
                                     const int* prefix,
@@ -1364,9 +1414,9 @@ extern "C" int sx_cell_bvh_traverse(const float* p4, int n_queries, float paddin
     SX_REQUIRE(p4 && grid8 && origin_box6 && nmin4 && nmax4 && prefix && face_rec8 &&
                    cand && num && status,
                "sx_cell_bvh_traverse: null pointer");
-    launch(cell_traverse_kernel<false>, grid_for(32LL * n_queries, CT_BLOCK), CT_BLOCK, 0, as_stream(stream),
-           n_queries, (const float4*)p4, padding, grid8, origin_box6, (const float4*)nmin4, (const float4*)nmax4,
-           prefix, (const float4*)face_rec8, cap, cand, num, status, (const int*)nullptr);
+    launch(cell_traverse_kernel<false>, traverse_grid(cell_traverse_kernel<false>, n_queries), CT_BLOCK, 0,
+           as_stream(stream), n_queries, (const float4*)p4, padding, grid8, origin_box6, (const float4*)nmin4,
+           (const float4*)nmax4, prefix, (const float4*)face_rec8, cap, cand, num, status, (const int*)nullptr);
     return check_launch("cell_traverse_kernel");
 }
 
@@ -1379,7 +1429,8 @@ extern "C" int sx_cell_bvh_traverse_edges(const int* edges, int n_edges, const f
     SX_REQUIRE(edges && p4 && grid8 && origin_box6 && nmin4 && nmax4 && prefix && face_rec8 && cand && num &&
                    status,
                "sx_cell_bvh_traverse_edges: null pointer");
-    launch(cell_traverse_kernel<true>, grid_for(32LL * n_edges, CT_BLOCK), CT_BLOCK, 0, as_stream(stream), n_edges,
+    launch(cell_traverse_kernel<true>, traverse_grid(cell_traverse_kernel<true>, n_edges), CT_BLOCK, 0,
+           as_stream(stream), n_edges,
            (const float4*)p4, padding, grid8, origin_box6, (const float4*)nmin4, (const float4*)nmax4, prefix,
            (const float4*)face_rec8, cap, cand, num, status, edges);
     return check_launch("cell_traverse_kernel");
