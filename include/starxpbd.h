@@ -247,8 +247,8 @@ int sx_cell_bvh_init(int* sorted_codes, int* sorted_ids, int* child_a, int* chil
 
 /* LBVH_CELL.build, lbvh_cell.py:637-653: cell size from box6
  * (assign_cell_centers :105-120), faces binned by AABB centre
- * (assign_face_cell_ids :577-586), inclusive scan, stable counting sort
- * (counting_sort_cells :589-598), leaves = row-major cells with
+ * (assign_face_cell_ids :577-586), stably sorted by cell (the order of
+ * counting_sort_cells :589-598), leaves = row-major cells with
  * AABB = centre U faces (assign_leaf_cell_nodes :602-634) and a single-launch
  * bottom-up refit with the rules of compute_cell_node_aabbs :491-522.
  * Outputs: sorted_face_ids[n_faces], prefix[32768] (inclusive),
@@ -262,6 +262,11 @@ int sx_cell_bvh_build(const float* fmin4, const float* fmax4, int n_faces, const
                       const int* child_b, const int* parent, int* sorted_face_ids, int* prefix, int* num_faces,
                       float* nmin4, float* nmax4, float* face_rec8, float* grid8, void* ws, size_t ws_bytes,
                       void* stream);
+/* The same, which also copies box6 to box_out6 (NULL: no copy). */
+int sx_cell_bvh_build_copy(const float* fmin4, const float* fmax4, int n_faces, const float* box6, float* box_out6,
+                           const int* child_a, const int* child_b, const int* parent, int* sorted_face_ids, int* prefix,
+                           int* num_faces, float* nmin4, float* nmax4, float* face_rec8, float* grid8, void* ws,
+                           size_t ws_bytes, void* stream);
 
 /* traverse_cell_bvh_single, lbvh_cell.py:656-714, for query boxes
  * p4[i] +- padding (Solver.broadphase_lbvh, XPBD.py:187-215), over a build's

@@ -102,6 +102,18 @@ __device__ __forceinline__ void pdl_entry() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// Release of this thread's memory operations to the cluster and acquire of the others'.
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ unsigned load_cluster(const unsigned* p, unsigned rank) {
+    unsigned addr = (unsigned)__cvta_generic_to_shared(p), remote, v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(remote) : "memory");
+    return v;
+}
+
 // ---- float3 arithmetic with fixed evaluation order ----------------------------
 struct V3 {
     float x, y, z;

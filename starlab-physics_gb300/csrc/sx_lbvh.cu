@@ -310,17 +310,6 @@ __global__ void __launch_bounds__(RS_BLOCK) rs_scatter(const unsigned* __restric
 constexpr int RC_BLOCK = 1024, RC_WARPS = RC_BLOCK / 32, RC_CLUSTER = 16, RC_MAX_ITEMS = 4;
 constexpr size_t rc_smem(int items) { return (size_t)(RC_WARPS * 256 + 2 * RC_BLOCK * items) * 4; }
 
-// Release of this thread's memory operations to the cluster and acquire of the others'.
-__device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ unsigned load_cluster(const unsigned* p, unsigned rank) {
-    unsigned addr = (unsigned)__cvta_generic_to_shared(p), remote, v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
-    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(remote) : "memory");
-    return v;
-}
 // Exclusive scan of one value per thread over the first 256 threads of the block
 // (the others pass 0 and get the total).
 __device__ __forceinline__ unsigned first256_excl_scan(unsigned v, unsigned* wsum) {
@@ -593,9 +582,9 @@ __global__ void karras_kernel(int n, const unsigned* __restrict__ c, int tie, in
 // ---------------------------------------------------------------------------
 // Cell-grid BVH build (LBVH_CELL.build, lbvh_cell.py:637-653)
 // ---------------------------------------------------------------------------
+// box_out (optional): a copy of box6.
 __global__ void face_cell_kernel(int F, const float4* __restrict__ mn4, const float4* __restrict__ mx4,
-                                 const float* __restrict__ box6, unsigned* keys, int* ids, unsigned* counts,
-                                 float* grid8) {
+                                 const float* box6, float* box_out, unsigned* keys, int* ids, float* grid8) {
     pdl_entry();
     int f = blockIdx.x * blockDim.x + threadIdx.x;
     V3 lo{box6[0], box6[1], box6[2]};
@@ -605,17 +594,36 @@ __global__ void face_cell_kernel(int F, const float4* __restrict__ mn4, const fl
         grid8[1] = cs.y;
         grid8[2] = cs.z;
         grid8[3] = grid8[4] = grid8[5] = 0.0f;  // max leaf overhang, raised by the leaf kernel
-        grid8[6] = grid8[7] = 0.0f;
+        grid8[6] = grid8[7] = 0.0f;             // [7]: the leaf kernel's blocks that are done
     }
+    if (box_out != nullptr && f < 6) box_out[f] = box6[f];
     if (f >= F) return;
     V3 c = scale(0.5f, add(mk(mn4[f]), mk(mx4[f])));
     int ix = min(max(f2i_sat((c.x - lo.x) / cs.x), 0), kGridRes - 1);
     int iy = min(max(f2i_sat((c.y - lo.y) / cs.y), 0), kGridRes - 1);
     int iz = min(max(f2i_sat((c.z - lo.z) / cs.z), 0), kGridRes - 1);
-    int cell = ix * kGridRes * kGridRes + iy * kGridRes + iz;
-    keys[f] = (unsigned)cell;
+    keys[f] = (unsigned)(ix * kGridRes * kGridRes + iy * kGridRes + iz);
     ids[f] = f;
-    atomicAdd(counts + cell, 1u);
+}
+
+// prefix[c] = faces in cells 0 .. c, from the sorted cells: thread i writes the
+// cells from key i - 1 up to key i (to the end for the last), a long run of empty
+// cells with its whole warp.  No counters to clear, raise and scan.
+__global__ void __launch_bounds__(256) cell_bounds_kernel(int F, const unsigned* __restrict__ keys,
+                                                          int* __restrict__ prefix) {
+    pdl_entry();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    int from = 0, to = 0;
+    if (i <= F) {
+        from = i == 0 ? 0 : (int)keys[i - 1];
+        to = i == F ? kNumCells : (int)keys[i];
+    }
+    unsigned runs = __ballot_sync(0xffffffffu, to > from);
+    for (; runs != 0u; runs &= runs - 1u) {
+        const int l = __ffs(runs) - 1;
+        const int end = __shfl_sync(0xffffffffu, to, l), n = i - lane + l;
+        for (int c = __shfl_sync(0xffffffffu, from, l) + lane; c < end; c += 32) prefix[c] = n;
+    }
 }
 
 // Node boxes are float4 pairs; min.w carries the node's face count (int bits)
@@ -673,37 +681,55 @@ __device__ __forceinline__ NodeBox join_nodes(const NodeBox& l, const NodeBox& r
     return o;
 }
 
-// Block = one z-column (cells col*32 .. col*32+31), a warp per cell: 8 warps
-// taking 4 cells each, so that the 1024 columns fit one wave of blocks.
+// Block = one z-column (cells col*32 .. col*32+31); the 1024 columns fit one wave
+// of blocks.  Most of a column's cells are empty: a lane each writes the centre
+// point, and the warps take the cells that hold faces, two batches of 32 faces at
+// once.  The last block to finish fits the 1023 nodes above the columns (sizes 64 ..
+// 32768).  A chain of dependent loads (prefix, face, box) bounds it; a warp that
+// took four cells one after the other went through it four times.  The whole
+// build, with the sums before each cell read off the sorted cells instead of cleared,
+// counted and scanned: 64 x 64 sheet 35.6 -> 26.5 us, 181 x 139 40.2 -> 29.1, 256 x
+// 256 46.9 -> 35.2.
 constexpr int kColumnRefitThreads = 256;
 
 __global__ void __launch_bounds__(kColumnRefitThreads) cell_column_refit_kernel(
     const float* __restrict__ box6, const int* __restrict__ prefix, const int* __restrict__ sorted_face_ids,
-    const float4* __restrict__ fmn4, const float4* __restrict__ fmx4, int* __restrict__ num_faces,
-    float4* __restrict__ nmin4, float4* __restrict__ nmax4, float4* __restrict__ frec, float* grid8) {
+    const float4* __restrict__ fmn4, const float4* __restrict__ fmx4, int* __restrict__ num_faces, float4* nmin4,
+    float4* nmax4, float4* __restrict__ frec, float* grid8) {
     pdl_entry();
     __shared__ NodeBox tree[64];  // [32 + k]: leaf k; [16 + k], [8 + k], ...: levels above
-    __shared__ unsigned ext_bits[3];
+    __shared__ NodeBox top[2 * kColumnRefitThreads];  // the same above the columns, from [256 + k] on
+    __shared__ bool last;
     const int col = blockIdx.x, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (threadIdx.x < 3) ext_bits[threadIdx.x] = 0u;
     const V3 lo{box6[0], box6[1], box6[2]};
     const V3 cs = cell_size_of(box6);
-    __syncthreads();  // ext_bits initialised
-    // warp w takes the column's cells w, w + warps, ... (one warp per cell)
-    for (int z = w; z < kGridRes; z += kColumnRefitThreads / 32) {
-        const int i = col * kGridRes + z;
-        const int rl = i == 0 ? 0 : prefix[i - 1];
-        const int size = prefix[i] - rl;
-        const V3 c = cell_center(i, cs, lo);
+    // every warp: lane z's cell
+    const int i = col * kGridRes + lane;
+    const int rl = i == 0 ? 0 : prefix[i - 1];
+    const int size = prefix[i] - rl;
+    const unsigned occ = __ballot_sync(0xffffffffu, size > 0);
+    if (w == 0 && size == 0) tree[32 + lane] = NodeBox{cell_center(i, cs, lo), cell_center(i, cs, lo), 0};
+    unsigned todo = occ;
+    for (int k = 0; todo != 0u; ++k, todo &= todo - 1u) {
+        if (k % (kColumnRefitThreads / 32) != w) continue;
+        const int z = __ffs(todo) - 1;
+        const int first = __shfl_sync(0xffffffffu, rl, z), n = __shfl_sync(0xffffffffu, size, z);
+        const V3 c = cell_center(col * kGridRes + z, cs, lo);
         V3 a = c, b = c;
-        for (int j = lane; j < size; j += 32) {
-            const int fid = sorted_face_ids[rl + j];
-            const float4 fa = fmn4[fid], fb = fmx4[fid];
-            a = vmin(a, mk(fa));
-            b = vmax(b, mk(fb));
-            frec[2 * (rl + j)] = make_float4(fa.x, fa.y, fa.z, __int_as_float(fid));
-            frec[2 * (rl + j) + 1] = make_float4(fb.x, fb.y, fb.z, 0.0f);
+        for (int j = lane; j < n; j += 64) {
+            const bool two = j + 32 < n;
+            const int f0 = sorted_face_ids[first + j], f1 = two ? sorted_face_ids[first + j + 32] : f0;
+            const float4 a0 = fmn4[f0], b0 = fmx4[f0], a1 = fmn4[f1], b1 = fmx4[f1];
+            a = vmin(vmin(a, mk(a0)), mk(a1));
+            b = vmax(vmax(b, mk(b0)), mk(b1));
+            frec[2 * (first + j)] = make_float4(a0.x, a0.y, a0.z, __int_as_float(f0));
+            frec[2 * (first + j) + 1] = make_float4(b0.x, b0.y, b0.z, 0.0f);
+            if (two) {
+                frec[2 * (first + j + 32)] = make_float4(a1.x, a1.y, a1.z, __int_as_float(f1));
+                frec[2 * (first + j + 32) + 1] = make_float4(b1.x, b1.y, b1.z, 0.0f);
+            }
         }
+        __syncwarp();
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             a = vmin(a, V3{__shfl_xor_sync(0xffffffffu, a.x, o), __shfl_xor_sync(0xffffffffu, a.y, o),
@@ -711,32 +737,28 @@ __global__ void __launch_bounds__(kColumnRefitThreads) cell_column_refit_kernel(
             b = vmax(b, V3{__shfl_xor_sync(0xffffffffu, b.x, o), __shfl_xor_sync(0xffffffffu, b.y, o),
                            __shfl_xor_sync(0xffffffffu, b.z, o)});
         }
-        if (lane == 0) {
-            const int leaf = i + kNumCells - 1;
-            num_faces[leaf] = size;
-            store_box(nmin4, nmax4, leaf, a, b, size);
-            tree[32 + z] = NodeBox{a, b, size};
-            // how far this leaf's box reaches beyond its cell (>= 0), maximised
-            // over the grid: the traversal scans the cells within that reach
-            if (size > 0) {
-                const int x0 = i / (kGridRes * kGridRes), y0 = (i % (kGridRes * kGridRes)) / kGridRes, z0 = z;
-                const float clo[3] = {lo.x + cs.x * (float)x0, lo.y + cs.y * (float)y0, lo.z + cs.z * (float)z0};
-                const float chi[3] = {lo.x + cs.x * (float)(x0 + 1), lo.y + cs.y * (float)(y0 + 1),
-                                      lo.z + cs.z * (float)(z0 + 1)};
-                const float am[3] = {a.x, a.y, a.z}, bm[3] = {b.x, b.y, b.z};
-                for (int k = 0; k < 3; ++k) {
-                    const float ext = fmaxf(fmaxf(clo[k] - am[k], bm[k] - chi[k]), 0.0f);
-                    if (ext > 0.0f) atomicMax(ext_bits + k, __float_as_uint(ext));
-                }
-            }
-        }
+        if (lane == 0) tree[32 + z] = NodeBox{a, b, n};
     }
     __syncthreads();
     if (w == 0) {
+        const NodeBox nb = tree[32 + lane];
+        num_faces[i + kNumCells - 1] = nb.n;
+        store_box(nmin4, nmax4, i + kNumCells - 1, nb.a, nb.b, nb.n);
+        // how far this leaf's box reaches beyond its cell (>= 0), maximised over the
+        // grid: the traversal scans the cells within that reach
+        const int x0 = i / (kGridRes * kGridRes), y0 = (i % (kGridRes * kGridRes)) / kGridRes;
+        const float clo[3] = {lo.x + cs.x * (float)x0, lo.y + cs.y * (float)y0, lo.z + cs.z * (float)lane};
+        const float chi[3] = {lo.x + cs.x * (float)(x0 + 1), lo.y + cs.y * (float)(y0 + 1),
+                              lo.z + cs.z * (float)(lane + 1)};
+        const float am[3] = {nb.a.x, nb.a.y, nb.a.z}, bm[3] = {nb.b.x, nb.b.y, nb.b.z};
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const float ext = nb.n > 0 ? fmaxf(fmaxf(clo[k] - am[k], bm[k] - chi[k]), 0.0f) : 0.0f;
+            const unsigned most = __reduce_max_sync(0xffffffffu, ext > 0.0f ? __float_as_uint(ext) : 0u);
+            if (lane == 0 && most != 0u) atomicMax(reinterpret_cast<unsigned*>(grid8) + 3 + k, most);
+        }
         // occupancy word of the column, and the column's subtree, level by level
-        const unsigned occ = __ballot_sync(0xffffffffu, tree[32 + lane].n > 0);
         if (lane == 0) reinterpret_cast<unsigned*>(grid8)[kGridHeader + col] = occ;
-        if (lane < 3 && ext_bits[lane] != 0u) atomicMax(reinterpret_cast<unsigned*>(grid8) + 3 + lane, ext_bits[lane]);
         for (int half = 16, sz = 2; half >= 1; half >>= 1, sz <<= 1) {
             if (lane < half) {
                 const NodeBox nb = join_nodes(tree[2 * half + 2 * lane], tree[2 * half + 2 * lane + 1]);
@@ -747,37 +769,43 @@ __global__ void __launch_bounds__(kColumnRefitThreads) cell_column_refit_kernel(
             }
             __syncwarp();
         }
-    }
-}
-
-// The 1023 nodes above the columns (sizes 64 .. 32768), one block.
-__global__ void __launch_bounds__(1024) cell_top_refit_kernel(int* __restrict__ num_faces,
-                                                              float4* __restrict__ nmin4,
-                                                              float4* __restrict__ nmax4) {
-    pdl_entry();
-    __shared__ float4 sa[kGridRes * kGridRes], sb[kGridRes * kGridRes];
-    const int t = threadIdx.x;
-    {
-        const int node = cell_node_index(t * kGridRes, kGridRes);
-        sa[t] = nmin4[node];
-        sb[t] = nmax4[node];
+        __threadfence();
+        __syncwarp();
+        if (lane == 0) last = atomicAdd(reinterpret_cast<int*>(grid8) + 7, 1) == (int)gridDim.x - 1;
     }
     __syncthreads();
-    for (int half = kGridRes * kGridRes / 2, sz = 2 * kGridRes; half >= 1; half >>= 1, sz <<= 1) {
-        NodeBox nb;
-        if (t < half) {
-            const float4 la = sa[2 * t], lb = sb[2 * t], ra = sa[2 * t + 1], rb = sb[2 * t + 1];
-            nb = join_nodes(NodeBox{mk(la), mk(lb), __float_as_int(la.w)}, NodeBox{mk(ra), mk(rb), __float_as_int(ra.w)});
-            const int node = cell_node_index(t * sz, sz);
-            num_faces[node] = nb.n;
-            store_box(nmin4, nmax4, node, nb.a, nb.b, nb.n);
-        }
+    if (!last) return;
+    __threadfence();
+    const int t = threadIdx.x;
+    if (t == 0) grid8[7] = 0.0f;
+    // four columns a thread, two levels in registers, the others in shared memory
+    static_assert(4 * kColumnRefitThreads == kGridRes * kGridRes, "four columns a thread");
+    auto put = [&](int l, int size, const NodeBox& nb) {
+        const int node = cell_node_index(l, size);
+        num_faces[node] = nb.n;
+        store_box(nmin4, nmax4, node, nb.a, nb.b, nb.n);
+    };
+    NodeBox c[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int node = cell_node_index((4 * t + k) * kGridRes, kGridRes);
+        const float4 na = __ldcg(nmin4 + node), nb = __ldcg(nmax4 + node);
+        c[k] = NodeBox{mk(na), mk(nb), __float_as_int(na.w)};
+    }
+    c[0] = join_nodes(c[0], c[1]);
+    c[2] = join_nodes(c[2], c[3]);
+    put(4 * t * kGridRes, 2 * kGridRes, c[0]);
+    put((4 * t + 2) * kGridRes, 2 * kGridRes, c[2]);
+    c[0] = join_nodes(c[0], c[2]);
+    put(4 * t * kGridRes, 4 * kGridRes, c[0]);
+    top[kColumnRefitThreads + t] = c[0];
+    for (int half = kColumnRefitThreads / 2, sz = 8 * kGridRes; half >= 1; half >>= 1, sz <<= 1) {
         __syncthreads();
         if (t < half) {
-            sa[t] = make_float4(nb.a.x, nb.a.y, nb.a.z, __int_as_float(nb.n));
-            sb[t] = make_float4(nb.b.x, nb.b.y, nb.b.z, 0.0f);
+            const NodeBox nb = join_nodes(top[2 * (half + t)], top[2 * (half + t) + 1]);
+            top[half + t] = nb;
+            put(t * sz, sz, nb);
         }
-        __syncthreads();
     }
 }
 
@@ -1536,8 +1564,6 @@ extern "C" int sx_cell_bvh_init(int* sorted_codes, int* sorted_ids, int* child_a
     SX_REQUIRE(sorted_codes && sorted_ids && child_a && child_b && range_l && range_r && parent,
                "sx_cell_bvh_init: null pointer");
     SX_REQUIRE(ws && ws_bytes >= sx_cell_bvh_workspace_bytes(0), "sx_cell_bvh_init: workspace too small");
-    const cudaError_t attr = scan_smem_attr();  // for sx_cell_bvh_build's prefix scan
-    if (attr != cudaSuccess) return cuda_status(attr, "cudaFuncSetAttribute(scan_single_block)");
     cudaStream_t s = as_stream(stream);
     launch(cell_morton_kernel, grid_for(kNumCells, 256), 256, 0, s, (unsigned*)sorted_codes, sorted_ids);
     int rc = check_launch("cell_morton_kernel");
@@ -1549,10 +1575,10 @@ extern "C" int sx_cell_bvh_init(int* sorted_codes, int* sorted_ids, int* child_a
     return check_launch("karras_kernel(cells)");
 }
 
-extern "C" int sx_cell_bvh_build(const float* fmin4, const float* fmax4, int n_faces, const float* box6,
-                                 const int* child_a, const int* child_b, const int* parent, int* sorted_face_ids,
-                                 int* prefix, int* num_faces, float* nmin4, float* nmax4, float* face_rec8,
-                                 float* grid8, void* ws, size_t ws_bytes, void* stream) {
+extern "C" int sx_cell_bvh_build_copy(const float* fmin4, const float* fmax4, int n_faces, const float* box6,
+                                      float* box_out6, const int* child_a, const int* child_b, const int* parent,
+                                      int* sorted_face_ids, int* prefix, int* num_faces, float* nmin4, float* nmax4,
+                                      float* face_rec8, float* grid8, void* ws, size_t ws_bytes, void* stream) {
     SX_REQUIRE(n_faces >= 0, "sx_cell_bvh_build: n_faces < 0");
     SX_REQUIRE(box6 && child_a && child_b && parent && prefix && num_faces && nmin4 && nmax4 && grid8,
                "sx_cell_bvh_build: null pointer");
@@ -1564,25 +1590,27 @@ extern "C" int sx_cell_bvh_build(const float* fmin4, const float* fmax4, int n_f
     unsigned* keys = (unsigned*)p;
     p += align256((size_t)(n_faces > 0 ? n_faces : 1) * 4);
     void* rws = p;
-    p += rs_ws_bytes(n_faces);
-    SX_CUDA(cudaMemsetAsync(prefix, 0, sizeof(int) * kNumCells, s));
-    launch(face_cell_kernel, grid_for(n_faces, 256), 256, 0, s, n_faces, (const float4*)fmin4, (const float4*)fmax4,
-           box6, keys, sorted_face_ids, (unsigned*)prefix, grid8);
+    launch(face_cell_kernel, grid_for(n_faces > 0 ? n_faces : 1, 256), 256, 0, s, n_faces, (const float4*)fmin4,
+           (const float4*)fmax4, box6, box_out6, keys, sorted_face_ids, grid8);
     int rc = check_launch("face_cell_kernel");
-    if (rc) return rc;
-    rc = launch_scan_single_block((unsigned*)prefix, kNumCells, 1, s);
     if (rc) return rc;
     if (n_faces > 1) {
         rc = radix_sort(keys, sorted_face_ids, n_faces, 15, rws, rs_ws_bytes(n_faces), s);
         if (rc) return rc;
     }
+    launch(cell_bounds_kernel, grid_for((long long)n_faces + 1, 256), 256, 0, s, n_faces, (const unsigned*)keys, prefix);
     launch(cell_column_refit_kernel, kGridRes * kGridRes, kColumnRefitThreads, 0, s, box6, (const int*)prefix,
            (const int*)sorted_face_ids, (const float4*)fmin4, (const float4*)fmax4, num_faces, (float4*)nmin4,
            (float4*)nmax4, (float4*)face_rec8, grid8);
-    rc = check_launch("cell_column_refit_kernel");
-    if (rc) return rc;
-    launch(cell_top_refit_kernel, 1, 1024, 0, s, num_faces, (float4*)nmin4, (float4*)nmax4);
-    return check_launch("cell_top_refit_kernel");
+    return check_launch("cell_column_refit_kernel");
+}
+
+extern "C" int sx_cell_bvh_build(const float* fmin4, const float* fmax4, int n_faces, const float* box6,
+                                 const int* child_a, const int* child_b, const int* parent, int* sorted_face_ids,
+                                 int* prefix, int* num_faces, float* nmin4, float* nmax4, float* face_rec8,
+                                 float* grid8, void* ws, size_t ws_bytes, void* stream) {
+    return sx_cell_bvh_build_copy(fmin4, fmax4, n_faces, box6, nullptr, child_a, child_b, parent, sorted_face_ids,
+                                  prefix, num_faces, nmin4, nmax4, face_rec8, grid8, ws, ws_bytes, stream);
 }
 
 // a warp a query, at most one resident wave of blocks

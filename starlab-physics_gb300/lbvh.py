@@ -88,12 +88,13 @@ class LBVH_CELL:
         nf = fmn.shape[0]
         if nf != self.num_leafs:
             raise ValueError(f"LBVH_CELL built for {self.num_leafs} faces, got {nf}")
-        self.box6.copy_(_as_box6(aabb_min_g, aabb_max_g, self.device))
+        box6 = _as_box6(aabb_min_g, aabb_max_g, self.device)
         self.face_aabb_min4, self.face_aabb_max4 = fmn, fmx
-        sx.sx_cell_bvh_build(ptr(fmn), ptr(fmx), nf, ptr(self.box6), ptr(self.child_a), ptr(self.child_b),
-                             ptr(self.parent), ptr(self.sorted_face_ids), ptr(self.prefix_sum_cell),
-                             ptr(self.num_faces), ptr(self.node_min4), ptr(self.node_max4), ptr(self.face_rec8),
-                             ptr(self.grid8), ptr(self.workspace), self.workspace.numel(), stream_handle())
+        sx.sx_cell_bvh_build_copy(ptr(fmn), ptr(fmx), nf, ptr(box6), ptr(self.box6), ptr(self.child_a),
+                                  ptr(self.child_b), ptr(self.parent), ptr(self.sorted_face_ids),
+                                  ptr(self.prefix_sum_cell), ptr(self.num_faces), ptr(self.node_min4),
+                                  ptr(self.node_max4), ptr(self.face_rec8), ptr(self.grid8), ptr(self.workspace),
+                                  self.workspace.numel(), stream_handle())
 
     def traverse(self, points4, padding: float, cap: int, cand, num, status, n_queries=None, stream=None):
         """``traverse_cell_bvh_single`` for boxes ``points4[i] +- padding`` (on
