@@ -1386,44 +1386,52 @@ def main():
     sim.mesh_dy.v4.copy_(v0)
     sim.build_bvhs()
     sim.compute_y(dt_sub)
-    sim.solve_constraints_jacobi_x(dt_sub, first_iteration=True, iteration=0)
+    sim._in_substep = True  # as within a substep: the chunk heads are written where a frame uses them
+    for it in range(2):
+        sim.solve_constraints_jacobi_x(dt_sub, first_iteration=it == 0, iteration=it)
+    headed = sim._heads_on
+    sim._in_substep = sim._heads_on = False
     torch.cuda.synchronize()
     n_pairs = sim.contact_pair_count()
     st_mesh = sim.mesh_st
     Vs = st_mesh.num_verts if st_mesh is not None else 0
 
-    def project():
-        sx.sx_contact_pairs_project_v(V, Vs, ptr(sim._pairs), ptr(sim._pairs_ws), ptr(m.y4),
-                                      ptr(st_mesh.x4) if st_mesh is not None else None, ptr(m.fixed), ptr(m.m_inv),
-                                      sim.dHat, float(sim.compliance_collision), sim.contact_cull_d2(),
-                                      ptr(sim._dx_fix), ptr(sim._nc), ptr(sim.status), None, 0, pp_variant,
-                                      stream_handle())
+    def project(heads):
+        sx.sx_contact_pairs_project_headed(V, Vs, ptr(sim._pairs), ptr(sim._pairs_ws), ptr(m.y4),
+                                           ptr(st_mesh.x4) if st_mesh is not None else None, ptr(m.fixed),
+                                           ptr(m.m_inv), sim.dHat, float(sim.compliance_collision),
+                                           sim.contact_cull_d2(), ptr(sim._dx_fix), ptr(sim._nc), ptr(sim.status),
+                                           None, 0, pp_variant, ptr(sim._heads[0]) if heads else None,
+                                           ptr(sim._heads[2]) if heads else None, stream_handle())
 
-    side = torch.cuda.Stream()
-    side.wait_stream(stream)
-    with torch.cuda.stream(side):
-        project()
-    stream.wait_stream(side)
-    gp = torch.cuda.CUDAGraph()
-    with torch.cuda.graph(gp):
-        for _ in range(30):
-            project()
-    preps = []
-    for _ in range(5):
-        flush.zero_()
-        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        a.record(stream)
-        gp.replay()
-        b.record(stream)
-        torch.cuda.synchronize()
-        preps.append(a.elapsed_time(b) / 30)
+    def project_ms(heads):
+        side = torch.cuda.Stream()
+        side.wait_stream(stream)
+        with torch.cuda.stream(side):
+            project(heads)
+        stream.wait_stream(side)
+        gp = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(gp):
+            for _ in range(30):
+                project(heads)
+        preps = []
+        for _ in range(5):
+            flush.zero_()
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record(stream)
+            gp.replay()
+            b.record(stream)
+            torch.cuda.synchronize()
+            preps.append(a.elapsed_time(b) / 30)
+        return sorted(preps)[len(preps) // 2]
+
+    proj_ms = project_ms(False)
+    headed_ms = project_ms(True) if headed else None
     sim._dx_fix.zero_()
     sim._nc.zero_()
-    proj_ms = sorted(preps)[len(preps) // 2]
     proj_bytes = 16 * n_pairs + 16 * V + 16 * Vs
     proj_gbs = proj_bytes / (proj_ms / 1e3) / 1e9
-    pp_kernel = ("pairs_project_pipe_kernel" if sx.sx_contact_pairs_project_variant_pipelined(pp_variant)
-                 else "pairs_project_kernel")
+    pp_kernel = "pairs_project_kernel"
     roofline = {"kernel": pp_kernel, "bound": "hbm", "achieved": round(proj_gbs, 1), "peak": peak,
                 "unit": "GB/s", "frac": round(proj_gbs / peak, 4),
                 "traffic": ncu_traffic(pp_kernel + "_drape256.md"),
@@ -1432,7 +1440,8 @@ def main():
                 "timing": "CUDA events around a graph of 30 back-to-back projections of one substep's pair list "
                           "(L2 flushed before each replay), median of 5",
                 "launches_per_step": roofline_sweep["launches_per_step"],
-                "share_of_step": round(proj_ms * roofline_sweep["launches_per_step"] / frame_ms, 4),
+                "headed_avg_launch_us": None if headed_ms is None else round(headed_ms * 1e3, 3),
+                "share_of_step": round((headed_ms or proj_ms) * roofline_sweep["launches_per_step"] / frame_ms, 4),
                 "peak_source": roofline_sweep["peak_source"]}
 
     line = {
