@@ -90,6 +90,8 @@ int sx_jacobi_sweep_variant_form(int variant, int* lanes, int* streaming);
  * the size, measured on grid cloths; timing the variants on the mesh itself can
  * only do better). */
 int sx_jacobi_sweep_default_variant(int n_verts, int fast);
+/* The packed form it recommends instead where the packed adjacency exists, or -1. */
+int sx_jacobi_sweep_default_packed_form(int n_verts, int fast);
 int sx_jacobi_sweep_v(const float* x4, const float* y_in4, float* y_out4, const float* fixed, const int* adj_ptr,
                       const int* adj, int n_verts, float k_spring, float k_bend, int bend_on_y, int variant,
                       void* stream);

@@ -50,6 +50,7 @@ SIGNATURES = {
     "sx_jacobi_sweep": ([P, P, P, P, P, P, I, F, F, I, P], I),
     "sx_jacobi_sweep_variants": ([], I),
     "sx_jacobi_sweep_default_variant": ([I, I], I),
+    "sx_jacobi_sweep_default_packed_form": ([I, I], I),
     "sx_jacobi_sweep_variant_info": ([I, P, P], I),
     "sx_jacobi_sweep_variant_form": ([I, P, P], I),
     "sx_set_programmatic_launch": ([I], I),
@@ -207,7 +208,8 @@ def stream_handle(stream=None) -> int:
 
 # entry points whose int result is a value, not a status
 _VALUES = ("sx_version", "sx_mlp_param_count", "sx_mlp_bf16_count", "sx_jacobi_sweep_variants",
-           "sx_jacobi_sweep_packed_forms", "sx_jacobi_sweep_default_variant", "sx_contact_pairs_project_variants",
+           "sx_jacobi_sweep_packed_forms", "sx_jacobi_sweep_default_variant",
+           "sx_jacobi_sweep_default_packed_form", "sx_contact_pairs_project_variants",
            "sx_contact_pairs_project_default_variant", "sx_contact_pairs_project_variant_pipelined", "sx_batched_substep_variants",
            "sx_batched_substep_variant_cluster")
 

@@ -197,6 +197,12 @@ class BatchedSolver:
         # choice for this batch size (autotune() times all of them)
         self.sweep_variant = None
         self._default_variant = [int(sx.sx_jacobi_sweep_default_variant(V, f)) for f in (0, 1)]
+        self._default_packed = [int(sx.sx_jacobi_sweep_default_packed_form(V, f)) if self.adj_nbr16 is not None else -1
+                                for f in (0, 1)]
+        if self.adj.is_inference():  # no version to tell edits by
+            self._default_packed = [-1, -1]
+        else:
+            self._packed_of = (self.adj, self.adj._version)  # what the packed copy was made of
         # the sweep over the packed, shared-memory-staged adjacency
         # (sx_jacobi_sweep_packed; same results; autotune() decides)
         self._packed_sweep = False
@@ -347,21 +353,31 @@ class BatchedSolver:
             self._body_stream = torch.cuda.Stream(device=self.device)
         return self._body_stream
 
+    def _packed_choice(self, fast: int) -> int:
+        """Solver._packed_choice for the concatenated instances."""
+        if self._packed_sweep:
+            return self.packed_form
+        form = self._default_packed[fast] if self.sweep_variant is None else -1
+        if form < 0:
+            return -1
+        return form if self.adj is self._packed_of[0] and self.adj._version == self._packed_of[1] else -1
+
     def _iteration(self, it, s, k_spring, k_bend, conv, ref, check, loop=0, in_loop=False):
         """One Jacobi iteration: sweep (checked in tolerance mode), broad phase
         in the first iteration, obstacle contacts.  Inside a device-side loop
         (in_loop) the contact kernels are not gated; ``loop`` is the loop
         handle, given with the body's checked sweep."""
         fast = 1 if self.fast_math else 0
+        form = self._packed_choice(fast)
         if conv is not None:
             sx.sx_jacobi_sweep_checked_mode(ptr(self.x4), ptr(self.y4), ptr(self._y_other), ptr(self.fixed),
                                             ptr(self.adj_ptr), ptr(self.adj), self.num_verts, k_spring, k_bend, it,
                                             1 if check else 0, float(self.tol), ref, conv, ptr(self._res3),
                                             ptr(self._res_ws), self._res_ws.numel(), loop, self.n_iter, fast, s)
-        elif self.packed_sweep:
+        elif form >= 0:
             sx.sx_jacobi_sweep_packed_v(ptr(self.x4), ptr(self.y4), ptr(self._y_other), ptr(self.fixed),
                                         ptr(self.adj_ptr), ptr(self.adj_nbr16), ptr(self.adj_rest32), self.num_verts,
-                                        k_spring, k_bend, 1 if self.bending_on == "y" else 0, self.packed_form, fast,
+                                        k_spring, k_bend, 1 if self.bending_on == "y" else 0, form, fast,
                                         s)
         else:
             sx.sx_jacobi_sweep_mode(ptr(self.x4), ptr(self.y4), ptr(self._y_other), ptr(self.fixed),
@@ -403,7 +419,7 @@ class BatchedSolver:
             return
         key = (n_substeps, self.dt, self.dHat, self.damping, self.padding, self.g, self.stiffness_stretch,
                self.stiffness_bending, self.n_iter, self.bending_on, self.sweep_variant, self._packed_sweep, self.packed_form,
-               self.fast_math, self.tol,
+               self.fast_math, self._packed_choice(int(self.fast_math)), self.tol,
                self.tol_relative, self.persistent, self.persistent_variant,
                self.check_every,
                id(self.warm) if self.warm is not None else None,

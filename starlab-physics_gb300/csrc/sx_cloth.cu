@@ -511,6 +511,13 @@ extern "C" int sx_jacobi_sweep_default_variant(int n_verts, int fast) {
     return n_verts <= 200000 ? 9 : 5;                   // 2 lanes, 3 entries; 4 entries x 128 threads
 }
 
+// -1: the int2 variant above.  The fast arithmetic of a mesh past the L1s is bound by
+// what it reads, 6 bytes an entry here against 8: batch frames of 186 K / 299 K /
+// 552 K / 986 K vertices 1656 -> 1575, 2238 -> 2051, 3421 -> 3111, 5952 -> 5325 us, one
+// sheet of 180 K / 359 K / 720 K 7.2 -> 6.4, 11.3 -> 10.4, 21.9 -> 18.9 us a sweep; at
+// 137 K 1496 -> 1516.  The exact arithmetic is bound by issue and gains nothing.
+extern "C" int sx_jacobi_sweep_default_packed_form(int n_verts, int fast) { return fast && n_verts > 160000 ? 3 : -1; }
+
 extern "C" int sx_jacobi_sweep_variant_info(int variant, int* g, int* block) {
     SX_REQUIRE(variant >= 0 && variant < kNumSweepVariants && g && block, "sx_jacobi_sweep_variant_info: bad variant");
     *g = kSweepVariants[variant].g;

@@ -123,6 +123,12 @@ class Solver:
         # choice for this mesh size (autotune() times all of them)
         self.sweep_variant = None
         self._default_variant = [int(sx.sx_jacobi_sweep_default_variant(mesh_dy.num_verts, f)) for f in (0, 1)]
+        self._default_packed = [int(sx.sx_jacobi_sweep_default_packed_form(mesh_dy.num_verts, f))
+                                if mesh_dy.adj_nbr16 is not None else -1 for f in (0, 1)]
+        if mesh_dy.adj.is_inference():  # no version to tell edits by
+            self._default_packed = [-1, -1]
+        else:
+            self._packed_of = (mesh_dy.adj, mesh_dy.adj._version)  # what the packed copy was made of
         self._packed_sweep = False
         self.packed_form = 0  # the packed sweep staged per block (0) or read from global memory (1)
         # launch configuration of the contact-pair projection (None: the
@@ -218,6 +224,18 @@ class Solver:
         sx.sx_predict(ptr(m.x4), ptr(m.v4), ptr(m.fixed), ptr(m.y4), m.num_verts, float(dt), g[0], g[1], g[2],
                       stream_handle())
 
+    def _packed_choice(self, fast: int) -> int:
+        """Form of the packed sweep, or -1 for the int2 sweep.  By default only while
+        the adjacency is the one that the packed copy was made of: rest lengths
+        edited in ``mesh.adj`` count in the next sweep."""
+        if self._packed_sweep:
+            return self.packed_form
+        form = self._default_packed[fast] if self.sweep_variant is None else -1
+        if form < 0:
+            return -1
+        adj = self.mesh_dy.adj
+        return form if adj is self._packed_of[0] and adj._version == self._packed_of[1] else -1
+
     def spring_sweep(self, dt, iteration: int = 0, loop: int = 0):
         """init_variables + solve_spring_constraints_x + update_dx
         (XPBD.py:345-348, :141-184, :384-387); ping-pongs ``y``.  In tolerance
@@ -232,10 +250,11 @@ class Solver:
             sx.sx_gs_sweep(ptr(m.y4), ptr(cons), start, n_colors, k_spring, k_bend, stream_handle())
             return
         track = self._track if self._heads_on else (None, None, None)
-        if self.tol is None and self._packed_sweep:
+        form = self._packed_choice(fast)
+        if self.tol is None and form >= 0:
             sx.sx_jacobi_sweep_packed_tracked(ptr(m.x4), ptr(m.y4), ptr(self._y_other), ptr(m.fixed), ptr(m.adj_ptr),
                                               ptr(m.adj_nbr16), ptr(m.adj_rest32), m.num_verts, k_spring, k_bend,
-                                              1 if self.bending_on == "y" else 0, self.packed_form, fast, *track,
+                                              1 if self.bending_on == "y" else 0, form, fast, *track,
                                               stream_handle())
         elif self.tol is None:
             variant = self._default_variant[fast] if self.sweep_variant is None else self.sweep_variant
@@ -758,7 +777,8 @@ class Solver:
                 self.stiffness_bending, self.enable_collision_handling, self.n_iter, self.bending_on, self.rebuild,
                 self.compliance_collision, self.self_collision, self.contact_cull, self.fast_math,
                 self.gauss_seidel, self.sweep_variant, self._packed_sweep, self.packed_form,
-                self.pairs_variant, self.pair_heads, self.concurrent_broadphase, self.enable_edge_edge,
+                self.pairs_variant, self.pair_heads, self._packed_choice(int(self.fast_math)),
+                self.concurrent_broadphase, self.enable_edge_edge,
                 self.enable_velocity_update, self.mu, self.tol,
                 self.tol_relative,
                 self.check_every,

@@ -88,3 +88,41 @@ def test_default_variant_is_compiled(pkg, n, fast):
 
     lib = _lib.load()
     assert 0 <= int(lib.sx_jacobi_sweep_default_variant(n, fast)) < int(lib.sx_jacobi_sweep_variants())
+
+
+@pytest.mark.parametrize("n", [1, 30000, 160000, 160001, 200001, 1 << 30])
+def test_default_packed_form_is_compiled(pkg, n):
+    from starlab_physics_gb300 import _lib
+
+    lib = _lib.load()
+    assert int(lib.sx_jacobi_sweep_default_packed_form(n, 0)) == -1
+    assert -1 <= int(lib.sx_jacobi_sweep_default_packed_form(n, 1)) < int(lib.sx_jacobi_sweep_packed_forms())
+
+
+def test_default_packed_form_equals_the_int2_sweep(pkg):
+    """A sheet past the packed form's line, fast arithmetic: the default and the
+    int2 variant of its size end in the same positions bit for bit."""
+    out = []
+    x, f = _grid(410, 395)
+    for variant in (None, 5):
+        m = pkg.TriMesh(x, f, device="cuda")
+        sim = pkg.Solver(m, None, 4e-6, 1e5, 1e8, (0.0, 0.0, -9.81), 1 / 60, n_iter=3, bending_on="y")
+        sim.fast_math, sim.sweep_variant = True, variant
+        assert sim._default_packed == [-1, 3]
+        m.v4[:, :3] = torch.from_numpy(np.random.default_rng(3).normal(0, 0.2, x.shape).astype(np.float32)).cuda()
+        sim.forward(2)
+        out.append(m.x4.cpu().numpy())
+    assert np.isfinite(out[0]).all() and np.array_equal(out[0], out[1])
+    # rest lengths edited in place: the packed copy is out of date and stays unused
+    sim.sweep_variant = None
+    assert sim._packed_choice(1) == 3
+    m.adj[:, 1] += 0
+    assert sim._packed_choice(1) == -1
+
+
+def _grid(nx, ny):
+    i, j = np.meshgrid(np.arange(nx), np.arange(ny), indexing="ij")
+    x = np.stack([0.01 * i, 0.01 * j, 0.001 * np.sin(0.7 * i)], -1).reshape(-1, 3).astype(np.float32)
+    a = (i[:-1, :-1] * ny + j[:-1, :-1]).reshape(-1)
+    f = np.stack([np.stack([a, a + ny, a + 1], -1), np.stack([a + 1, a + ny, a + ny + 1], -1)], 1).reshape(-1, 3)
+    return x, f.astype(np.int32)
