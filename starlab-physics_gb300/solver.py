@@ -494,6 +494,10 @@ class Solver:
                 and 20 * self.mesh_dy.num_verts >= self.HEADS_MIN_PAIRS and self.contact_cull
                 and self.tol is None and not self.gauss_seidel and not self.record_pairs):
             return False
+        # a sweep or projection of a user's own may move vertices that no tracked sweep sees
+        for name in ("spring_sweep", "solve_collision_constraints_x"):
+            if name in self.__dict__ or getattr(type(self), name) is not getattr(Solver, name):
+                return False
         # a vertex's nearest triangle that does not contain it is about 0.7 edges
         # away (right triangles); where that is within the cull distance no chunk
         # has room to move and the heads are not worth writing

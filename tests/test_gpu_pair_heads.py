@@ -128,6 +128,27 @@ def test_positions_that_are_not_numbers(pkg):
     assert np.isnan(out[0]).any() and np.isfinite(out[0]).any() and np.array_equal(out[0], out[1], equal_nan=True)
 
 
+def test_own_steps_are_not_skipped_over(pkg):
+    """A solver whose collision step moves vertices itself tests every pair."""
+    class Pushed(pkg.Solver):
+        def solve_collision_constraints_x(self, *a, **k):
+            self.mesh_dy.y4[: self.mesh_dy.num_verts // 2, 2] += 2e-3
+            super().solve_collision_constraints_x(*a, **k)
+
+    out = []
+    for heads in (True, False):
+        x, f, v, sx, sf = _scene(pkg, **dict(BASE, layers=2, speed=1.0))
+        m, s = pkg.TriMesh(x, f, device="cuda"), pkg.TriMesh(sx, sf, device="cuda", is_static=True)
+        sim = Pushed(m, s, dHat=(4e-3) ** 2, stiffness_stretch=1e5, stiffness_bending=1e8, g=(0, 0, -9.81),
+                     dt=1 / 60, n_iter=8, rebuild="substep", bending_on="y")
+        sim.enable_collision_handling = True
+        sim.HEADS_MIN_PAIRS, sim.HEADS_MIN_ITERATIONS, sim.pair_heads = 1, 2, heads
+        m.v4[:, :3] = torch.from_numpy(v).cuda()
+        sim.forward(3)
+        out.append(m.x4.cpu().numpy().copy())
+    assert np.isfinite(out[0]).all() and np.array_equal(out[0], out[1])
+
+
 def test_refuses(pkg):
     from starlab_physics_gb300 import _lib
 
