@@ -26,8 +26,8 @@ import numpy as np
 import torch
 
 from ._lib import load, ptr, stream_handle, sx
-from .mesh import bending_pairs, box_mesh, constraint_adjacency, edges_from_faces, grid_cloth, inverse_masses, \
-    packed_adjacency, rest_lengths
+from .mesh import TensorState, bending_pairs, box_mesh, constraint_adjacency, edges_from_faces, grid_cloth, \
+    inverse_masses, packed_adjacency, rest_lengths
 
 
 @dataclass
@@ -155,6 +155,7 @@ class BatchedSolver:
         self.adj_ptr, self.adj = t(adj_ptr), t(adj)
         packed = packed_adjacency(adj_ptr, adj)
         self.adj_nbr16, self.adj_rest32 = (t(packed[0]), t(packed[1])) if packed is not None else (None, None)
+        self._packed_state = TensorState(self.adj, self.adj_nbr16, self.adj_rest32)
         self.fixed, self.m_inv = t(fixed), t(m_inv)
         self.x4 = torch.zeros((V, 4), dtype=torch.float32, device=dev)
         self.x4[:, :3] = t(x)
@@ -199,10 +200,7 @@ class BatchedSolver:
         self._default_variant = [int(sx.sx_jacobi_sweep_default_variant(V, f)) for f in (0, 1)]
         self._default_packed = [int(sx.sx_jacobi_sweep_default_packed_form(V, f)) if self.adj_nbr16 is not None else -1
                                 for f in (0, 1)]
-        if self.adj.is_inference():  # no version to tell edits by
-            self._default_packed = [-1, -1]
-        else:
-            self._packed_of = (self.adj, self.adj._version)  # what the packed copy was made of
+        self._capturing = False  # a frame's graph, whose key tells the sweep's form
         # the sweep over the packed, shared-memory-staged adjacency
         # (sx_jacobi_sweep_packed; same results; autotune() decides)
         self._packed_sweep = False
@@ -358,9 +356,11 @@ class BatchedSolver:
         if self._packed_sweep:
             return self.packed_form
         form = self._default_packed[fast] if self.sweep_variant is None else -1
-        if form < 0:
+        if form < 0 or not self._packed_state.unchanged(self.adj, self.adj_nbr16, self.adj_rest32):
             return -1
-        return form if self.adj is self._packed_of[0] and self.adj._version == self._packed_of[1] else -1
+        if not self._capturing and self.adj.is_cuda and torch.cuda.is_current_stream_capturing():
+            return -1
+        return form
 
     def _iteration(self, it, s, k_spring, k_bend, conv, ref, check, loop=0, in_loop=False):
         """One Jacobi iteration: sweep (checked in tolerance mode), broad phase
@@ -434,11 +434,15 @@ class BatchedSolver:
             side.wait_stream(torch.cuda.current_stream(self.device))
             lib = load()
             n0 = lib.sx_kernel_launches()
-            with torch.cuda.graph(gr, stream=side):
-                self._forward_eager(n_substeps)
-                if self.y4 is not y_start:
-                    y_start.copy_(self.y4)
-                    self._swap_y()
+            self._capturing = True
+            try:
+                with torch.cuda.graph(gr, stream=side):
+                    self._forward_eager(n_substeps)
+                    if self.y4 is not y_start:
+                        y_start.copy_(self.y4)
+                        self._swap_y()
+            finally:
+                self._capturing = False
             torch.cuda.current_stream(self.device).wait_stream(side)
             self.graph_kernel_launches = lib.sx_kernel_launches() - n0
             self._graphs[key] = gr

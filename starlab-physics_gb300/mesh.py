@@ -281,6 +281,34 @@ def packed_adjacency(ptr: np.ndarray, adj: np.ndarray):
     return nbr16, rest32.view(np.int32)
 
 
+class TensorState:
+    """Which tensors something was made of, and their versions then, taken where it
+    is made.  :meth:`unchanged` is false once another tensor stands in the place of
+    one of them or torch has written into one (its version counter).  It can't see
+    writes that torch doesn't count: kernels and libraries that write through the
+    pointer, and ``t.data``.  Tensors without a counter (inference tensors) and
+    copies of this object (a copied or unpickled owner has other tensors) count as
+    changed."""
+
+    def __init__(self, *tensors):
+        self.parts = (None if any(t is not None and t.is_inference() for t in tensors)
+                      else tuple((t, None if t is None else t._version) for t in tensors))
+
+    def unchanged(self, *tensors) -> bool:
+        return (self.parts is not None and len(tensors) == len(self.parts)
+                and all(t is was and (t is None or t._version == version)
+                        for t, (was, version) in zip(tensors, self.parts)))
+
+    @classmethod
+    def _unknown(cls):
+        state = cls()
+        state.parts = None
+        return state
+
+    def __reduce__(self):
+        return TensorState._unknown, ()
+
+
 class _Verts:
     """Attribute bag mirroring ``mesh.verts.{x,y,v,fixed,m_inv}``."""
 
@@ -339,6 +367,7 @@ class TriMesh:
         self.adj = t(adj)
         packed = packed_adjacency(ptr, adj)
         self.adj_nbr16, self.adj_rest32 = (t(packed[0]), t(packed[1])) if packed is not None else (None, None)
+        self._packed_state = TensorState(self.adj, self.adj_nbr16, self.adj_rest32)
 
         V = self.num_verts
         self.x4 = torch.zeros((V, 4), dtype=torch.float32, device=dev)
@@ -359,6 +388,11 @@ class TriMesh:
         self.verts.m_inv = self.m_inv
         self.verts.x0 = self.x0
         self._load_rest()
+
+    def packed_is_current(self) -> bool:
+        """Whether ``adj_nbr16`` / ``adj_rest32`` still are the packed copy of ``adj``
+        (:class:`TensorState` says which edits it sees)."""
+        return self._packed_state.unchanged(self.adj, self.adj_nbr16, self.adj_rest32)
 
     # -- state ---------------------------------------------------------------
     def _load_rest(self):

@@ -125,10 +125,7 @@ class Solver:
         self._default_variant = [int(sx.sx_jacobi_sweep_default_variant(mesh_dy.num_verts, f)) for f in (0, 1)]
         self._default_packed = [int(sx.sx_jacobi_sweep_default_packed_form(mesh_dy.num_verts, f))
                                 if mesh_dy.adj_nbr16 is not None else -1 for f in (0, 1)]
-        if mesh_dy.adj.is_inference():  # no version to tell edits by
-            self._default_packed = [-1, -1]
-        else:
-            self._packed_of = (mesh_dy.adj, mesh_dy.adj._version)  # what the packed copy was made of
+        self._capturing = False  # a frame's graph, whose key tells the sweep's form
         self._packed_sweep = False
         self.packed_form = 0  # the packed sweep staged per block (0) or read from global memory (1)
         # launch configuration of the contact-pair projection (None: the
@@ -226,15 +223,19 @@ class Solver:
 
     def _packed_choice(self, fast: int) -> int:
         """Form of the packed sweep, or -1 for the int2 sweep.  By default only while
-        the adjacency is the one that the packed copy was made of: rest lengths
-        edited in ``mesh.adj`` count in the next sweep."""
+        ``mesh.packed_is_current()``, so that rest lengths edited in ``mesh.adj`` by
+        torch, before or after the solver was made, count in the next sweep; after
+        writes that torch doesn't count (``adj.data``, kernels of a user's own) set
+        ``sweep_variant`` to a number, which keeps to ``mesh.adj``.  A graph that a
+        user captures reads ``mesh.adj`` as well: it may be edited between replays."""
         if self._packed_sweep:
             return self.packed_form
         form = self._default_packed[fast] if self.sweep_variant is None else -1
-        if form < 0:
+        if form < 0 or not self.mesh_dy.packed_is_current():
             return -1
-        adj = self.mesh_dy.adj
-        return form if adj is self._packed_of[0] and adj._version == self._packed_of[1] else -1
+        if not self._capturing and self.mesh_dy.adj.is_cuda and torch.cuda.is_current_stream_capturing():
+            return -1
+        return form
 
     def spring_sweep(self, dt, iteration: int = 0, loop: int = 0):
         """init_variables + solve_spring_constraints_x + update_dx
@@ -798,13 +799,17 @@ class Solver:
         side.wait_stream(torch.cuda.current_stream(self.device))
         lib = load()
         n0 = lib.sx_kernel_launches()
-        with torch.cuda.graph(g, stream=side):
-            self._forward_eager(n_substeps)
-            if m.y4 is not y_start:
-                # an odd number of sweeps left y in the other buffer: copy it back
-                # so that every replay starts from the same buffer assignment
-                y_start.copy_(m.y4)
-                self._swap_y()
+        self._capturing = True
+        try:
+            with torch.cuda.graph(g, stream=side):
+                self._forward_eager(n_substeps)
+                if m.y4 is not y_start:
+                    # an odd number of sweeps left y in the other buffer: copy it back
+                    # so that every replay starts from the same buffer assignment
+                    y_start.copy_(m.y4)
+                    self._swap_y()
+        finally:
+            self._capturing = False
         torch.cuda.current_stream(self.device).wait_stream(side)
         self.graph_kernel_launches = lib.sx_kernel_launches() - n0
         return g
