@@ -442,8 +442,9 @@ int sx_contact_pairs_project_default_variant(void);
  * min_pairs such pairs it writes none.  Afterwards every change of the positions
  * must end in a tracked sweep (sx_jacobi_sweep_tracked with this ref4 and moved)
  * before sx_contact_pairs_project_headed, which then passes over the chunks that
- * cannot have come into reach: the same sums as sx_contact_pairs_project_v.  A
- * new list (sx_contact_pairs_build) drops the heads.  heads:
+ * cannot have come into reach: the same sums as sx_contact_pairs_project_v.  With
+ * cull_d2 <= 0, or a cull_d2 above the heads' own, it tests every pair.  A new
+ * list (sx_contact_pairs_build) drops the heads.  heads:
  * sx_contact_pairs_heads_bytes bytes, 16-byte aligned. */
 size_t sx_contact_pairs_heads_bytes(int n_dy, int cap);
 int sx_contact_pairs_heads(int n_dy, int n_st, int cap, const int* pairs, void* ws, const float* y4, float cull_d2,

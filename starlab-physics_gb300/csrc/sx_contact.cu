@@ -553,8 +553,9 @@ __global__ void __launch_bounds__(128) collision_project_kernel(
 // without the faces __vt_dy skips (incident ones); every iteration then runs
 // one thread per pair.  The per-pair arithmetic is the same code as above and
 // accumulation is order independent, so the result equals the per-query walk.
-// Workspace: block and query totals, then meta[6] = {end of vt_st pairs, end of vt_dy
-// pairs, total pairs, heads in use, heads with a bound, blocks that wrote them}.
+// Workspace: block and query totals, then meta[7] = {end of vt_st pairs, end of vt_dy
+// pairs, total pairs, heads in use, heads with a bound, blocks that wrote them, the
+// heads' cull_d2 as float bits}.
 // ---------------------------------------------------------------------------
 // Two launches, the counts and the pairs, both chains of dependent loads (count,
 // candidate, its face) that a thread a query walked 20 to 30 times: eight lanes take
@@ -898,6 +899,7 @@ __global__ void __launch_bounds__(256) pairs_heads_kernel(int V, int* meta, cons
         if (tid == 0) meta[3] = 0;
         return;
     }
+    if (tid == 0) meta[6] = __float_as_int(cull_d2);
     for (int v = tid; v < V; v += nt) {
         ref[v] = y4[v];
         if ((v & 31) == 0) moved[v >> 5] = 0u;
@@ -1139,8 +1141,9 @@ __global__ void __launch_bounds__(PP_BLOCK, MINB) pairs_project_kernel(const int
     __shared__ int sat_stack[PP_BLOCK / 32][64];
     int* s1 = box_stack[threadIdx.x >> 5];
     int* s2 = sat_stack[threadIdx.x >> 5];
-    pairs_project_body<U, PIPE, HEADED>(c, meta[2], HEADED && heads_in_use(meta) != 0, cull_d2, s1, s2, status, heads,
-                                        moved);
+    // heads bound the motion that brings a pair within their own cull distance
+    const bool in_use = HEADED && heads_in_use(meta) != 0 && cull_d2 <= __int_as_float(meta[6]);
+    pairs_project_body<U, PIPE, HEADED>(c, meta[2], in_use, cull_d2, s1, s2, status, heads, moved);
 }
 
 // update_dx (XPBD.py:384-387) from the fixed-point accumulators; clears them.
@@ -2281,7 +2284,8 @@ extern "C" int sx_contact_pairs_project_headed(int n_dy, int n_st, const int* pa
                "sx_contact_pairs_project_headed: heads (16-byte aligned) and moved go together");
     PairsWs w = pairs_ws(const_cast<void*>(ws), n_dy, n_st);
     const PairsProjectVariant& pv = kPairsProjectVariants[variant];
-    launch(heads ? pv.headed : pv.kern, sm_count() * pv.blocks_per_sm, PP_BLOCK, 0, as_stream(stream),
+    // without a cull every pair is evaluated: the headed body has no such form
+    launch(heads && cull_d2 > 0.0f ? pv.headed : pv.kern, sm_count() * pv.blocks_per_sm, PP_BLOCK, 0, as_stream(stream),
            (const int*)w.meta,
            (const int4*)pairs, (const float4*)y4, (const float4*)xs4, fixed, m_inv, dHat, compliance, cull_d2, dx_fix,
            nc, status, conv, iter, heads, moved);
