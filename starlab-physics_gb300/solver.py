@@ -489,15 +489,20 @@ class Solver:
     # fewer pairs loses up to 1 % of the substep to the launch that finds it so.
     HEADS_MIN_PAIRS = 200_000
     HEADS_MIN_ITERATIONS = 20
+    # the steps that the heads' reckoning is built on
+    HEADS_STEPS = ("solve_constraints_jacobi_x", "spring_sweep", "solve_collision_constraints_x",
+                   "solve_edge_edge_constraints_x", "contact_cull_d2")
 
     def _heads_wanted(self) -> bool:
         if not (self.pair_heads and self.self_collision and self.n_iter >= self.HEADS_MIN_ITERATIONS
                 and 20 * self.mesh_dy.num_verts >= self.HEADS_MIN_PAIRS and self.contact_cull
                 and self.tol is None and not self.gauss_seidel and not self.record_pairs):
             return False
-        # a sweep or projection of a user's own may move vertices that no tracked sweep sees
-        for name in ("spring_sweep", "solve_collision_constraints_x"):
-            if name in self.__dict__ or getattr(type(self), name) is not getattr(Solver, name):
+        # a step of a user's own may move vertices between a sweep and the projection,
+        # or change the cull distance that the heads were made for
+        for name in self.HEADS_STEPS:
+            step = getattr(self, name)
+            if getattr(step, "__func__", None) is not getattr(Solver, name) or step.__self__ is not self:
                 return False
         # a vertex's nearest triangle that does not contain it is about 0.7 edges
         # away (right triangles); where that is within the cull distance no chunk
