@@ -16,6 +16,7 @@ from __future__ import annotations
 import torch
 
 from ._lib import ptr, stream_handle, sx
+from .mesh import TensorState
 
 NUM_CELLS = 32 * 32 * 32
 
@@ -122,6 +123,12 @@ class LBVH:
     (``tie=1``: equal codes ordered by index, always a valid tree; ``tie=0``: the
     reference's rule), bottom-up refit.  ``query(points4, padding, cap)``: stack
     traversal for boxes ``points4[i] +- padding``.
+
+    :meth:`refit` also writes child records, copies of the boxes and ids that a
+    query meets together, which :meth:`query` walks while the tree's arrays are as
+    :meth:`refit` left them (:class:`~.mesh.TensorState` says which edits are seen);
+    after an edit it walks the arrays themselves until the next refit.  A query in a
+    captured graph stays on the form it was captured with.
     """
 
     def __init__(self, num_leafs: int, device="cuda", tie: int = 1, sort_bits: int = 32):
@@ -152,21 +159,28 @@ class LBVH:
         # well-formed hierarchy; written by refit
         self.aux = (torch.empty(int(sx.sx_face_bvh_aux_bytes(n)), dtype=torch.uint8, device=dev) if tie == 1
                     else None)
-        self._aux_valid = False
+        self._aux_of = None  # the arrays whose copy aux is
+
+    def _tree(self):
+        return self.sorted_ids, self.child_a, self.child_b, self.node_min4, self.node_max4
 
     def morton(self, face_min4, face_max4, box6):
+        self._aux_of = None
         sx.sx_face_morton(ptr(face_min4), ptr(face_max4), self.n, ptr(box6), ptr(self.codes), ptr(self.sorted_ids),
                           stream_handle())
 
     def sort(self):
+        self._aux_of = None
         sx.sx_radix_sort_pairs(ptr(self.codes), ptr(self.sorted_ids), self.n, self.sort_bits, ptr(self.workspace),
                                self.workspace.numel(), stream_handle())
 
     def hierarchy(self):
+        self._aux_of = None
         sx.sx_karras_build(ptr(self.codes), self.n, int(self.tie), ptr(self.child_a), ptr(self.child_b),
                            ptr(self.range_l), ptr(self.range_r), ptr(self.parent), stream_handle())
 
     def refit(self, face_min4, face_max4):
+        self._aux_of = None
         if self.tie != 1:
             # the reference's tie rule can give a malformed hierarchy on repeated
             # codes: the plain one-thread-per-leaf climb handles that case
@@ -174,10 +188,12 @@ class LBVH:
                                  ptr(self.child_b), ptr(self.parent), ptr(self.node_min4), ptr(self.node_max4),
                                  ptr(self.flags), ptr(self.status), stream_handle())
             return
+        if self.aux is None:  # tie was changed after construction
+            self.aux = torch.empty(int(sx.sx_face_bvh_aux_bytes(self.n)), dtype=torch.uint8, device=self.device)
         sx.sx_face_bvh_refit_ranges(self.n, ptr(self.sorted_ids), ptr(face_min4), ptr(face_max4), ptr(self.range_l),
                                     ptr(self.range_r), ptr(self.parent), ptr(self.node_min4), ptr(self.node_max4),
                                     ptr(self.aux), self.aux.numel(), stream_handle())
-        self._aux_valid = True
+        self._aux_of = TensorState(*self._tree())
 
     def build(self, face_min4, face_max4, box6):
         self.box6 = box6
@@ -199,7 +215,7 @@ class LBVH:
             # visit the queries in Morton order of the points (normalised by the
             # build's box): a warp's threads then walk nearby parts of the tree
             order = self._query_order(points4, q)
-        if self._aux_valid and self.tie == 1:
+        if self._aux_of is not None and self.tie == 1 and self._aux_of.unchanged(*self._tree()):
             sx.sx_face_bvh_query(self.n, ptr(points4), q, float(padding), ptr(self.sorted_ids), ptr(self.node_min4),
                                  ptr(self.node_max4), ptr(self.aux), int(cap), ptr(cand), ptr(num), ptr(status),
                                  ptr(order), stream_handle())
