@@ -169,10 +169,15 @@ class LBVH:
         sx.sx_face_morton(ptr(face_min4), ptr(face_max4), self.n, ptr(box6), ptr(self.codes), ptr(self.sorted_ids),
                           stream_handle())
 
+    CODE_BITS = 30
+
     def sort(self):
+        """By ``sort_bits`` of the codes, at least all that :meth:`morton` writes: the
+        Karras build over codes in no full order leaves nodes without a parent,
+        whose links the refit would follow."""
         self._aux_of = None
-        sx.sx_radix_sort_pairs(ptr(self.codes), ptr(self.sorted_ids), self.n, self.sort_bits, ptr(self.workspace),
-                               self.workspace.numel(), stream_handle())
+        sx.sx_radix_sort_pairs(ptr(self.codes), ptr(self.sorted_ids), self.n, max(self.sort_bits, self.CODE_BITS),
+                               ptr(self.workspace), self.workspace.numel(), stream_handle())
 
     def hierarchy(self):
         self._aux_of = None
