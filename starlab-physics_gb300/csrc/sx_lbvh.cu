@@ -6,6 +6,7 @@
 #include <mutex>
 
 #include "sx_common.cuh"
+#include "sx_per_device.h"
 
 namespace sx {
 
@@ -199,15 +200,16 @@ __global__ void __launch_bounds__(1024) scan_single_block(unsigned* data, int n,
     }
 }
 
-// The shared-memory limit is raised once per process; sx_cell_bvh_init does it
-// first, outside any stream capture.
+// The shared-memory limit is raised once per device.
 static cudaError_t scan_smem_attr() {
-    static std::once_flag once;
-    static cudaError_t attr = cudaSuccess;
-    std::call_once(once, [] {
-        attr = cudaFuncSetAttribute(scan_single_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SCAN_SMEM);
+    static PerDevice attr;
+    int dev = -1;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    return (cudaError_t)attr.get(dev, [] {
+        return (int)cudaFuncSetAttribute(scan_single_block, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)SCAN_SMEM);
     });
-    return attr;
 }
 
 static int launch_scan_single_block(unsigned* data, int n, int inclusive, cudaStream_t s) {
@@ -427,19 +429,23 @@ static ClusterSort cluster_sort_kernel(int items) {
     return items == 1 ? rs_cluster_kernel<1> : items == 2 ? rs_cluster_kernel<2>
                                            : rs_cluster_kernel<RC_MAX_ITEMS>;
 }
-// Largest cluster of the sort that the device can hold, 0 for none.  The kernels'
-// limits are raised once per process.
+// Largest cluster of the sort that the current device can hold, 0 for none.  The
+// kernels' limits are raised once per device.
 static int cluster_sort_blocks() {
-    static std::once_flag once;
-    static int blocks = 0;
-    std::call_once(once, [] {
+    static PerDevice blocks;
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return blocks.get(dev, [] {
         for (int items = 1; items <= RC_MAX_ITEMS; items *= 2) {
             const ClusterSort k = cluster_sort_kernel(items);
             if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rc_smem(items)) !=
                     cudaSuccess ||
                 cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
                 cudaGetLastError();
-                return;
+                return 0;
             }
         }
         for (int c = RC_CLUSTER; c >= 8; c /= 2) {
@@ -454,14 +460,12 @@ static int cluster_sort_blocks() {
             cfg.numAttrs = 1;
             int active = 0;
             if (cudaOccupancyMaxActiveClusters(&active, rs_cluster_kernel<RC_MAX_ITEMS>, &cfg) == cudaSuccess &&
-                active > 0) {
-                blocks = c;
-                return;
-            }
+                active > 0)
+                return c;
             cudaGetLastError();
         }
+        return 0;
     });
-    return blocks;
 }
 
 int scan_u32(unsigned* data, int n, int inclusive, cudaStream_t s) {
