@@ -24,6 +24,28 @@ from ._lib import load, ptr, stream_handle, sx
 _cache: dict = {}
 
 
+class LibraryChoice(int):
+    """The sweep variant that the library chooses for a mesh, as ``sweep_variant``
+    reads where none was set.  Set on a solver (put back after a trial, for one), it
+    leaves the choice to the library, as None does: for the mesh's size, and the
+    packed form where that is faster."""
+
+
+class SweepVariant:
+    """``sweep_variant`` of a solver: the launch configuration of its fixed-count
+    sweep, a number of :func:`variants`."""
+
+    def __get__(self, sim, owner=None):
+        if sim is None:
+            return self
+        if sim._sweep_variant is None:
+            return LibraryChoice(sim._default_variant[1 if sim.fast_math else 0])
+        return sim._sweep_variant
+
+    def __set__(self, sim, variant):
+        sim._sweep_variant = None if variant is None or isinstance(variant, LibraryChoice) else int(variant)
+
+
 def variants() -> list[tuple[int, int]]:
     """(entries per load batch, threads per block) of every compiled variant."""
     L = load()

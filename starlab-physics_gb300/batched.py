@@ -26,6 +26,7 @@ import numpy as np
 import torch
 
 from ._lib import load, ptr, stream_handle, sx
+from .autotune import SweepVariant
 from .mesh import TensorState, bending_pairs, box_mesh, constraint_adjacency, edges_from_faces, grid_cloth, \
     inverse_masses, packed_adjacency, rest_lengths
 
@@ -82,6 +83,8 @@ def shard_instances(instances, rank: int, world: int):
 
 class BatchedSolver:
     """XPBD substep for a batch of independent cloths with obstacles."""
+
+    sweep_variant = SweepVariant()
 
     def __init__(self, instances, dHat, stiffness_stretch, stiffness_bending, g, dt, *, n_iter=20, cap=40,
                  bending_on="y", padding=8e-3, damping=0.001, device="cuda"):
@@ -194,9 +197,9 @@ class BatchedSolver:
                                  device=dev)
         # learned warm start (learned.WarmStart) run after each prediction
         self.warm = None
-        # launch configuration of the fixed-count sweep: None = the library's
-        # choice for this batch size (autotune() times all of them)
-        self.sweep_variant = None
+        # launch configuration of the fixed-count sweep (sweep_variant): None = the
+        # library's choice for this batch size (autotune() times all of them)
+        self._sweep_variant = None
         self._default_variant = [int(sx.sx_jacobi_sweep_default_variant(V, f)) for f in (0, 1)]
         self._default_packed = [int(sx.sx_jacobi_sweep_default_packed_form(V, f)) if self.adj_nbr16 is not None else -1
                                 for f in (0, 1)]
@@ -355,7 +358,7 @@ class BatchedSolver:
         """Solver._packed_choice for the concatenated instances."""
         if self._packed_sweep:
             return self.packed_form
-        form = self._default_packed[fast] if self.sweep_variant is None else -1
+        form = self._default_packed[fast] if self._sweep_variant is None else -1
         if form < 0 or not self._packed_state.unchanged(self.adj, self.adj_nbr16, self.adj_rest32):
             return -1
         if not self._capturing and self.adj.is_cuda and torch.cuda.is_current_stream_capturing():
@@ -383,7 +386,8 @@ class BatchedSolver:
             sx.sx_jacobi_sweep_mode(ptr(self.x4), ptr(self.y4), ptr(self._y_other), ptr(self.fixed),
                                     ptr(self.adj_ptr), ptr(self.adj), self.num_verts, k_spring, k_bend,
                                     1 if self.bending_on == "y" else 0,
-                                    self._default_variant[fast] if self.sweep_variant is None else self.sweep_variant,
+                                    self._default_variant[fast] if self._sweep_variant is None
+                                    else self._sweep_variant,
                                     fast, s)
         self._swap_y()
         if it == 0:
@@ -418,8 +422,8 @@ class BatchedSolver:
             self._forward_eager(n_substeps)
             return
         key = (n_substeps, self.dt, self.dHat, self.damping, self.padding, self.g, self.stiffness_stretch,
-               self.stiffness_bending, self.n_iter, self.bending_on, self.sweep_variant, self._packed_sweep, self.packed_form,
-               self.fast_math, self._packed_choice(int(self.fast_math)), self.tol,
+               self.stiffness_bending, self.n_iter, self.bending_on, self._sweep_variant, self._packed_sweep,
+               self.packed_form, self.fast_math, self._packed_choice(int(self.fast_math)), self.tol,
                self.tol_relative, self.persistent, self.persistent_variant,
                self.check_every,
                id(self.warm) if self.warm is not None else None,

@@ -75,10 +75,13 @@ import numpy as np
 import torch
 
 from ._lib import load, ptr, stream_handle, sx
+from .autotune import SweepVariant
 from .lbvh import LBVH_CELL
 
 
 class Solver:
+    sweep_variant = SweepVariant()
+
     def __init__(self, mesh_dy, mesh_st, dHat, stiffness_stretch, stiffness_bending, g, dt, *, n_iter: int = 1,
                  rebuild: str = "frame", cap: int = 40, record_pairs: bool = False, bending_on: str = "x"):
         if rebuild not in ("frame", "substep"):
@@ -119,9 +122,9 @@ class Solver:
         self.enable_edge_edge = False
         self._ee = None
         self._sewing = None  # (sewn, sptr, partner, scratch, stiffness)
-        # launch configuration of the fixed-count sweep: None = the library's
-        # choice for this mesh size (autotune() times all of them)
-        self.sweep_variant = None
+        # launch configuration of the fixed-count sweep (sweep_variant): None = the
+        # library's choice for this mesh size (autotune() times all of them)
+        self._sweep_variant = None
         self._default_variant = [int(sx.sx_jacobi_sweep_default_variant(mesh_dy.num_verts, f)) for f in (0, 1)]
         self._default_packed = [int(sx.sx_jacobi_sweep_default_packed_form(mesh_dy.num_verts, f))
                                 if mesh_dy.adj_nbr16 is not None else -1 for f in (0, 1)]
@@ -230,7 +233,7 @@ class Solver:
         user captures reads ``mesh.adj`` as well: it may be edited between replays."""
         if self._packed_sweep:
             return self.packed_form
-        form = self._default_packed[fast] if self.sweep_variant is None else -1
+        form = self._default_packed[fast] if self._sweep_variant is None else -1
         if form < 0 or not self.mesh_dy.packed_is_current():
             return -1
         if not self._capturing and self.mesh_dy.adj.is_cuda and torch.cuda.is_current_stream_capturing():
@@ -258,7 +261,7 @@ class Solver:
                                               1 if self.bending_on == "y" else 0, form, fast, *track,
                                               stream_handle())
         elif self.tol is None:
-            variant = self._default_variant[fast] if self.sweep_variant is None else self.sweep_variant
+            variant = self._default_variant[fast] if self._sweep_variant is None else self._sweep_variant
             sx.sx_jacobi_sweep_tracked(ptr(m.x4), ptr(m.y4), ptr(self._y_other), ptr(m.fixed), ptr(m.adj_ptr),
                                        ptr(m.adj), m.num_verts, k_spring, k_bend, 1 if self.bending_on == "y" else 0,
                                        variant, fast, *track, stream_handle())
@@ -786,7 +789,7 @@ class Solver:
         return (n_substeps, self.dt, self.dHat, self.damping, self.padding, self.g, self.stiffness_stretch,
                 self.stiffness_bending, self.enable_collision_handling, self.n_iter, self.bending_on, self.rebuild,
                 self.compliance_collision, self.self_collision, self.contact_cull, self.fast_math,
-                self.gauss_seidel, self.sweep_variant, self._packed_sweep, self.packed_form,
+                self.gauss_seidel, self._sweep_variant, self._packed_sweep, self.packed_form,
                 self.pairs_variant, self.pair_heads, self._packed_choice(int(self.fast_math)),
                 self.concurrent_broadphase, self.enable_edge_edge,
                 self.enable_velocity_update, self.mu, self.tol,
