@@ -57,8 +57,9 @@ __global__ void inc_fill_kernel(int E, const int* __restrict__ edges, const int*
 // * few seeds (a sheet numbered row by row has one): color_chain_kernel, a
 //   single block, since the chain of dependent edges is the limit and not the
 //   width (the 256 x 256 sheet's 195 388 edges: 2 037 steps, up to 170 edges
-//   wide).  Only the messages under way have to be kept, a few per edge of the
-//   front, so they live in a hash table in shared memory.
+//   wide).  Only the messages under way have to be kept, up to two per edge of
+//   the front, so they live in a hash table in shared memory, and those that find
+//   their bucket full in global memory.
 // * many seeds (concatenated sheets, shuffled numbering): color_push_kernel,
 //   every SM.  Messages are 64-bit atomic adds on the edge's word, and the add
 //   that completes the word returns both sets; a link costs an atomic's round
@@ -67,10 +68,13 @@ __global__ void inc_fill_kernel(int E, const int* __restrict__ edges, const int*
 // The former form, in which each edge's thread waited for the one neighbour that
 // blocked it and then read all neighbours' colours again, took 3 us a link.
 //
-// A step of the single block takes 0.9 us: the successors' own successors come
+// A step of the single block takes 0.85 us: the successors' own successors come
 // from L2 (prefetching or loading their lines a step ahead made it slower), then
 // a barrier, the table and the ring.  With the messages in global memory it took
-// 1 us (plain stores: a line just stored misses L1), with atomics 1.5 us.
+// 1 us (plain stores: a line just stored misses L1), with atomics 1.5 us.  Sheets
+// of 256 x 256 / 512 x 512 / 1024 x 1024, ms: 1.75 / 4.0 / 10.7, with bending pairs
+// 2.4 / 6.0 / 21.6; a table that lost the messages of a full bucket, and left the
+// rest to color_edges_kernel, took 1.78 / 4.6 / 17 to 57 and 2.6 / 26 / 116.
 //
 // A message: bits 0-29 colours 0-29, bit 30: a higher colour is among them and
 // the whole set is in msg.  Word of an edge: bits 0-30 the message at endpoint
@@ -198,34 +202,49 @@ __device__ __forceinline__ void ring_push(int4* ring, unsigned* ring_b, int* s_t
         ring_b[i] = m1.y;
     }
 }
-// n edges leave the ring and, past a barrier, at most 2 n enter it
-__device__ __forceinline__ int ring_take(int held) {
-    const int n = held < CP_THREADS ? held : CP_THREADS;
-    return n < CP_RING - held ? n : CP_RING - held;
+// n edges leave the ring and, past a barrier, at most 2 n enter it (n < 0: held < 0)
+__device__ __forceinline__ int ring_take(int held, int threads) {
+    return min(min(held, threads), CP_RING - max(held, 0));
 }
 
-// The messages under way: {edge + 1, endpoint << 31 | message} in the edge's
-// bucket, 0 when free.  A step looks up the partners of all its messages (and
-// takes out those found), then, past a barrier, enters the messages without
-// one: two sent in the same step meet there, since both walk the bucket from its
-// start and nothing is taken out meanwhile.
+// The messages under way: {edge + 1, message} in the edge's bucket, 0 when free.  A
+// step looks up the partners of all its messages (and takes out those found), then,
+// past a barrier, enters the messages without one: two sent in the same step meet
+// there, since both walk the bucket from its start and nothing is taken out
+// meanwhile.  A message that finds its bucket full is parked in the edge's word in
+// global memory, where its partner, which finds the bucket full in the same step,
+// or parked[bucket] above 0 in a later one, meets it.
 __device__ __forceinline__ int bucket_of(unsigned f) { return (int)((f * 2654435761u) >> 21); }
 static_assert(CP_BUCKETS == 1 << 11, "bucket_of keeps 11 bits");
+constexpr unsigned long long kParked = 1ull << 62;  // (word of an edge that waits for two messages: 0 before)
+constexpr int kSomeParked = (int)0x80000000u;       // in the ring's tail: messages have been parked
 
 __device__ __forceinline__ bool table_take(unsigned long long* table, unsigned s, unsigned* other) {
     const unsigned f = s >> 2;
     unsigned long long* bucket = table + 4 * bucket_of(f);
-    bool found = false;
+    const ulonglong2* two = reinterpret_cast<const ulonglong2*>(bucket);
+    const ulonglong2 p = two[0], q = two[1];
+    const unsigned long long v[4] = {p.x, p.y, q.x, q.y};
+    int at = -1;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const unsigned long long v = bucket[i];
-        if ((unsigned)(v >> 32) == f + 1u) {
-            *other = (unsigned)v & 0x7fffffffu;
-            bucket[i] = 0ull;
-            found = true;
+    for (int i = 0; i < 4; ++i)
+        if ((unsigned)(v[i] >> 32) == f + 1u) {
+            *other = (unsigned)v[i] & 0x7fffffffu;
+            at = i;
         }
-    }
+    const bool found = at >= 0;
+    if (found) bucket[at] = 0ull;
     return found;
+}
+__device__ __forceinline__ bool parked_take(int* parked, const unsigned long long* word, unsigned s, unsigned* other) {
+    const unsigned f = s >> 2;
+    int* count = parked + bucket_of(f);
+    if (*count <= 0) return false;
+    const unsigned long long v = __ldcg(word + f);
+    if (!(v & kParked)) return false;
+    *other = (unsigned)v & 0x7fffffffu;
+    atomicSub(count, 1);
+    return true;
 }
 // >= 0: entry of the partner, which also entered in this step; -1: entered; -2: bucket full
 __device__ __forceinline__ int table_enter(unsigned long long* table, unsigned s, unsigned m, unsigned* other) {
@@ -242,68 +261,109 @@ __device__ __forceinline__ int table_enter(unsigned long long* table, unsigned s
     }
     return -2;
 }
+// Parks a message; whether its partner stands there from this step
+__device__ __forceinline__ bool park(int* parked, unsigned long long* word, int* s_tail, unsigned s, unsigned m,
+                                     unsigned* other) {
+    const unsigned f = s >> 2;
+    const unsigned long long old = atomicCAS(word + f, 0ull, kParked | m);
+    atomicAdd(parked + bucket_of(f), old == 0ull ? 1 : -1);
+    atomicOr(s_tail, kSomeParked);
+    if (old != 0ull) *other = (unsigned)old & 0x7fffffffu;
+    return old != 0ull;
+}
 
-__global__ void __launch_bounds__(CP_THREADS) color_chain_kernel(const uint2* __restrict__ succ, uint4* msg,
-                                                                 int max_colors, int* color,
-                                                                 const int* __restrict__ n_seeds,
-                                                                 const int* __restrict__ seeds, int* spill) {
-    pdl_entry();
-    const int ns = *n_seeds;
-    if (ns > kManySeeds) return;
-    extern __shared__ int4 ring[];  // {edge, successor slots, message 0}
-    unsigned* ring_b = reinterpret_cast<unsigned*>(ring + CP_RING);  // message 1
-    unsigned long long* table = reinterpret_cast<unsigned long long*>(ring_b + CP_RING);
-    __shared__ int s_tail;
+struct Chain {
+    const uint2* succ;
+    unsigned long long* word;
+    uint4* msg;
+    int max_colors;
+    int *color, *spill;
+    int4* ring;  // {edge, successor slots, message 0}
+    unsigned* ring_b;  // message 1
+    unsigned long long* table;
+    int *parked, *s_tail;
+};
+// Steps until the ring is empty or full, and without PARKED until a message has been
+// parked (the loop of its own saves a step the look at parked, 8 % of it).
+template <int THREADS, bool PARKED>
+__device__ __forceinline__ void chain_steps(const Chain& c, int& head, int& done0, int& done1) {
     const int tid = threadIdx.x;
-    for (int i = tid; i < 4 * CP_BUCKETS; i += CP_THREADS) table[i] = 0ull;
-    if (tid == 0) s_tail = ns;
-    if (tid < ns) {
-        const uint2 s = __ldg(succ + seeds[tid]);
-        ring[tid] = make_int4(seeds[tid], (int)s.x, (int)s.y, 0);
-        ring_b[tid] = 0u;
-    }
-    int head = 0, done0 = -1, done1 = -1;
     for (;;) {
         __syncthreads();
-        const int held = s_tail - head, n = ring_take(held);
-        if (n == 0) {
-            if (held > 0 && tid == 0) atomicOr(spill, 1);
+        const int tail = *c.s_tail;
+        const int held = (PARKED ? tail & ~kSomeParked : tail) - head, n = ring_take(held, THREADS);
+        if (n <= 0) {  // (without PARKED held is below 0 from then on)
+            if (held > 0 && tid == 0) atomicOr(c.spill, 1);
             break;
         }
         // partners that met while entering in the last step
-        if (done0 >= 0) table[done0] = 0ull;
-        if (done1 >= 0) table[done1] = 0ull;
+        if (done0 >= 0) c.table[done0] = 0ull;
+        if (done1 >= 0) c.table[done1] = 0ull;
         done0 = done1 = -1;
         uint2 s = make_uint2(kNone, kNone), n0 = s, n1 = s;
         unsigned ma = 0u, mb = 0u, oa = 0u, ob = 0u;
         bool r0 = false, r1 = false;
         if (tid < n) {
             const int at = (head + tid) & (CP_RING - 1);
-            const int4 r = ring[at];
+            const int4 r = c.ring[at];
             ma = (unsigned)r.w;
-            mb = ring_b[at];
+            mb = c.ring_b[at];
             s = make_uint2((unsigned)r.y, (unsigned)r.z);
-            if (s.x != kNone) n0 = __ldg(succ + (s.x >> 2));
-            if (s.y != kNone) n1 = __ldg(succ + (s.y >> 2));
-            color[r.x] = color_edge(r.x, &ma, &mb, s, msg, max_colors);
-            if (s.x != kNone) r0 = (s.x & 2u) || table_take(table, s.x, &oa);
-            if (s.y != kNone) r1 = (s.y & 2u) || table_take(table, s.y, &ob);
+            if (s.x != kNone) n0 = __ldg(c.succ + (s.x >> 2));
+            if (s.y != kNone) n1 = __ldg(c.succ + (s.y >> 2));
+            c.color[r.x] = color_edge(r.x, &ma, &mb, s, c.msg, c.max_colors);
+            if (s.x != kNone) r0 = (s.x & 2u) || table_take(c.table, s.x, &oa);
+            if (s.y != kNone) r1 = (s.y & 2u) || table_take(c.table, s.y, &ob);
+            if (PARKED) {
+                if (s.x != kNone && !r0) r0 = parked_take(c.parked, c.word, s.x, &oa);
+                if (s.y != kNone && !r1) r1 = parked_take(c.parked, c.word, s.y, &ob);
+            }
         }
         head += n;
         __syncthreads();
         if (s.x != kNone && !r0) {
-            done0 = table_enter(table, s.x, ma, &oa);
+            done0 = table_enter(c.table, s.x, ma, &oa);
             r0 = done0 >= 0;
-            if (done0 == -2) atomicOr(spill, 1);
+            if (done0 == -2) r0 = park(c.parked, c.word, c.s_tail, s.x, ma, &oa);
         }
         if (s.y != kNone && !r1) {
-            done1 = table_enter(table, s.y, mb, &ob);
+            done1 = table_enter(c.table, s.y, mb, &ob);
             r1 = done1 >= 0;
-            if (done1 == -2) atomicOr(spill, 1);
+            if (done1 == -2) r1 = park(c.parked, c.word, c.s_tail, s.y, mb, &ob);
         }
-        ring_push(ring, ring_b, &s_tail, r0, r1, s, n0, n1, (s.x & 1u) ? make_uint2(oa, ma) : make_uint2(ma, oa),
+        ring_push(c.ring, c.ring_b, c.s_tail, r0, r1, s, n0, n1, (s.x & 1u) ? make_uint2(oa, ma) : make_uint2(ma, oa),
                   (s.y & 1u) ? make_uint2(ob, mb) : make_uint2(mb, ob));
     }
+}
+
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) color_chain_kernel(const uint2* __restrict__ succ, unsigned long long* word,
+                                                              uint4* msg, int max_colors, int* color,
+                                                              const int* __restrict__ n_seeds,
+                                                              const int* __restrict__ seeds, int* spill) {
+    pdl_entry();
+    const int ns = *n_seeds;
+    if (ns > kManySeeds) return;
+    extern __shared__ int4 ring[];
+    __shared__ int s_tail;
+    Chain c{succ, word, msg, max_colors, color, spill, ring};
+    c.ring_b = reinterpret_cast<unsigned*>(ring + CP_RING);
+    c.table = reinterpret_cast<unsigned long long*>(c.ring_b + CP_RING);
+    c.parked = reinterpret_cast<int*>(c.table + 4 * CP_BUCKETS);
+    c.s_tail = &s_tail;
+    const int tid = threadIdx.x;
+    for (int i = tid; i < 4 * CP_BUCKETS; i += THREADS) c.table[i] = 0ull;
+    for (int i = tid; i < CP_BUCKETS; i += THREADS) c.parked[i] = 0;
+    if (tid == 0) s_tail = ns;
+    if (tid < ns) {
+        const uint2 s = __ldg(succ + seeds[tid]);
+        c.ring[tid] = make_int4(seeds[tid], (int)s.x, (int)s.y, 0);
+        c.ring_b[tid] = 0u;
+    }
+    int head = 0, done0 = -1, done1 = -1;
+    chain_steps<THREADS, false>(c, head, done0, done1);
+    __syncthreads();
+    if (s_tail < 0) chain_steps<THREADS, true>(c, head, done0, done1);
 }
 
 // adds a message to successor slot s; the successor's word afterwards
@@ -344,7 +404,7 @@ __global__ void __launch_bounds__(CP_THREADS) color_push_kernel(int E, const uin
             __syncthreads();
             tail = s_tail;
         }
-        const int held = tail - head, n = ring_take(held);
+        const int held = tail - head, n = ring_take(held, CP_THREADS);
         if (n == 0) {
             if (held > 0 && tid == 0) atomicOr(spill, 1);
             break;
@@ -596,10 +656,20 @@ extern "C" int sx_color_edges_greedy(const int* edges, int n_edges, int n_verts,
            succ, word, waits, color, sorted_edges, n_seeds, seeds);
     launch(color_lone_kernel, grid_for(n_edges, 256), 256, 0, s, n_edges, succ, (const unsigned char*)waits);
     constexpr size_t smem = (size_t)CP_RING * (sizeof(int4) + sizeof(unsigned));
-    constexpr size_t smem_table = smem + (size_t)4 * CP_BUCKETS * sizeof(unsigned long long);
-    SX_CUDA(cudaFuncSetAttribute(color_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_table));
+    constexpr size_t smem_table = smem + CP_BUCKETS * (4 * sizeof(unsigned long long) + sizeof(int));
+    // as many threads as a sheet of that many edges has edges ready at once (64 x 64: 60,
+    // 256 x 256: 170 to 255, 512 x 512 with bending pairs: 770); a step of more threads
+    // costs more.  256 / 512 / 1024 threads, ms, the two numberings of a sheet that the
+    // package makes: 195 585 edges 1.75 / 1.85 / 2.03 and 1.39 / 1.46 / 1.58, 390 150
+    // 2.33 / 2.42 / 2.58 and 2.54 / 2.05 / 2.17, 1 566 726 9.2 / 6.0 / 6.2 and 9.8 / 7.4 /
+    // 8.0, 3 141 633 17.4 / 11.2 / 10.7 and 17.5 / 11.9 / 10.6
+    const int chain_threads = n_edges <= 350000 ? 256 : n_edges <= 2500000 ? 512 : 1024;
+    const auto chain = chain_threads == 256   ? color_chain_kernel<256>
+                       : chain_threads == 512 ? color_chain_kernel<512>
+                                              : color_chain_kernel<1024>;
+    SX_CUDA(cudaFuncSetAttribute(chain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_table));
     SX_CUDA(cudaFuncSetAttribute(color_push_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    launch(color_chain_kernel, 1, CP_THREADS, smem_table, s, (const uint2*)succ, msg, max_colors, color,
+    launch(chain, 1, chain_threads, smem_table, s, (const uint2*)succ, word, msg, max_colors, color,
            (const int*)n_seeds, (const int*)seeds, spill);
     const int blocks = grid_for(n_edges, 4 * CP_THREADS);  // one block per SM at most
     launch(color_push_kernel, blocks < 152 ? blocks : 152, CP_THREADS, smem, s, n_edges, (const uint2*)succ, word, msg, max_colors, color, (const int*)n_seeds, spill);
