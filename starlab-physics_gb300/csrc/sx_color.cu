@@ -63,7 +63,11 @@ __global__ void inc_fill_kernel(int E, const int* __restrict__ edges, const int*
 // * many seeds (concatenated sheets, shuffled numbering): color_push_kernel,
 //   every SM.  Messages are 64-bit atomic adds on the edge's word, and the add
 //   that completes the word returns both sets; a link costs an atomic's round
-//   trip and the ring's bookkeeping, 1.5 us.
+//   trip and the ring's bookkeeping, 1.5 us.  The seeds are dealt evenly to the
+//   blocks: a block that runs dry ends, so with those of a range of edges each the
+//   work came down to a few blocks (us; dealt / by ranges / color_edges_kernel
+//   alone: 195 585 edges of a sheet in random order 212 / 432 / 261, an icosphere's
+//   122 880 226 / 539 / 278, 1000 8 x 8 sheets 195 / 205 / 369).
 //
 // The former form, in which each edge's thread waited for the one neighbour that
 // blocked it and then read all neighbours' colours again, took 3 us a link.
@@ -87,7 +91,6 @@ constexpr int CP_BUCKETS = 2048;  // of four messages each
 constexpr unsigned kNone = 0xffffffffu;
 constexpr unsigned kMsgLow = 0x3fffffffu, kMsgMore = 0x40000000u;
 constexpr int kManySeeds = 64;
-constexpr int kSeed = -2;  // colour of an edge without predecessors; -1: of any other uncoloured edge
 
 // Chains: waits[e] bit s: edge e has a predecessor at endpoint s.  An edge (v, v)
 // counts as having endpoint 0 only.
@@ -115,12 +118,9 @@ __global__ void color_waits_kernel(int E, const int* __restrict__ edges, const i
     succ[e] = make_uint2(next[0], next[1]);
     waits[e] = (unsigned char)w;
     word[e] = (unsigned long long)(2 - __popc(w)) << 62;
-    color[e] = w == 0 ? kSeed : -1;
+    color[e] = -1;
     ids[e] = e;
-    if (w == 0) {
-        const int k = atomicAdd(n_seeds, 1);
-        if (k < kManySeeds) seeds[k] = e;
-    }
+    if (w == 0) seeds[atomicAdd(n_seeds, 1)] = e;
 }
 __global__ void color_lone_kernel(int E, uint2* __restrict__ succ, const unsigned char* __restrict__ waits) {
     pdl_entry();
@@ -376,27 +376,27 @@ __device__ __forceinline__ unsigned long long color_send(unsigned s, unsigned m,
 __global__ void __launch_bounds__(CP_THREADS) color_push_kernel(int E, const uint2* __restrict__ succ,
                                                                 unsigned long long* word, uint4* msg, int max_colors,
                                                                 int* color, const int* __restrict__ n_seeds,
-                                                                int* spill) {
+                                                                const int* __restrict__ seeds, int* spill) {
     pdl_entry();
-    if (*n_seeds <= kManySeeds) return;
+    const int ns = *n_seeds;
+    if (ns <= kManySeeds) return;
     extern __shared__ int4 ring[];  // {edge, successor slots, message 0}
     unsigned* ring_b = reinterpret_cast<unsigned*>(ring + CP_RING);  // message 1
     __shared__ int s_tail;
     const int tid = threadIdx.x;
     if (tid == 0) s_tail = 0;
-    const int share = (int)(((long long)E + gridDim.x - 1) / gridDim.x);
-    const long long lo = (long long)blockIdx.x * share;
-    int scan = (int)min(lo, (long long)E);
-    const int hi = (int)min(lo + share, (long long)E);
+    const int share = (ns + (int)gridDim.x - 1) / (int)gridDim.x;
+    int scan = (int)min((long long)blockIdx.x * share, (long long)ns);
+    const int hi = min(scan + share, ns);
     int head = 0;  // uniform; head and tail count up to E at most
     for (;;) {
         __syncthreads();
         int tail = s_tail;
-        // the share's seeds, while there is room
+        // the block's seeds, while there is room
         while (scan < hi && tail - head <= CP_RING / 2 - CP_THREADS) {
             __syncthreads();
-            const int e = scan + tid;
-            const bool seed = e < hi && color[e] == kSeed;
+            const bool seed = scan + tid < hi;
+            const int e = seed ? seeds[scan + tid] : 0;
             const uint2 none = make_uint2(kNone, kNone), zero = make_uint2(0u, 0u);
             ring_push(ring, ring_b, &s_tail, seed, false, make_uint2(4u * (unsigned)e, kNone), seed ? succ[e] : none,
                       none, zero, zero);
@@ -611,7 +611,7 @@ __global__ void __launch_bounds__(128) color_prefix_kernel(int max_colors, const
 
 using namespace sx;
 
-// workspace: [status, spill, seed count, 64 seeds][ptr V+1][cursor V][inc 2E][succ E][word E][waits E][msg 2E][keys E][hist 128][radix ws E]
+// workspace: [status, spill, seed count][ptr V+1][cursor V][inc 2E][succ E][word E][waits E][msg 2E][keys E][hist 128][radix ws E]
 extern "C" size_t sx_color_workspace_bytes(int n_verts, int n_edges) {
     size_t V = (size_t)(n_verts > 0 ? n_verts : 1), E = (size_t)(n_edges > 0 ? n_edges : 1);
     return 1024 + a256((V + 1) * 4) + a256(V * 4) + a256(2 * E * 4) + a256(E * 8) + a256(E * 8) + a256(E) +
@@ -633,8 +633,8 @@ extern "C" int sx_color_edges_greedy(const int* edges, int n_edges, int n_verts,
                "sx_color_edges_greedy: workspace too small");
     const size_t V = (size_t)(n_verts > 0 ? n_verts : 1), E = (size_t)n_edges;
     int* status = (int*)ws;
-    int *spill = status + 1, *n_seeds = status + 2, *seeds = status + 3;
-    char* p = (char*)(((uintptr_t)(seeds + kManySeeds) + 255) & ~(uintptr_t)255);
+    int *spill = status + 1, *n_seeds = status + 2;
+    char* p = (char*)(((uintptr_t)(n_seeds + 1) + 255) & ~(uintptr_t)255);
     int* ptr = (int*)p; p += a256((V + 1) * 4);
     int* cursor = (int*)p; p += a256(V * 4);
     int* inc = (int*)p; p += a256(2 * E * 4);
@@ -645,6 +645,7 @@ extern "C" int sx_color_edges_greedy(const int* edges, int n_edges, int n_verts,
     unsigned* keys = (unsigned*)p; p += a256(E * 4);
     unsigned* hist = (unsigned*)p; p += a256(128 * 4);
     void* rws = p;
+    int* seeds = (int*)keys;  // until the colours' keys are written
 
     // status, spill, ptr and cursor lie together at the start
     SX_CUDA(cudaMemsetAsync(ws, 0, (size_t)((char*)(cursor + V) - (char*)ws), s));
@@ -672,7 +673,7 @@ extern "C" int sx_color_edges_greedy(const int* edges, int n_edges, int n_verts,
     launch(chain, 1, chain_threads, smem_table, s, (const uint2*)succ, word, msg, max_colors, color,
            (const int*)n_seeds, (const int*)seeds, spill);
     const int blocks = grid_for(n_edges, 4 * CP_THREADS);  // one block per SM at most
-    launch(color_push_kernel, blocks < 152 ? blocks : 152, CP_THREADS, smem, s, n_edges, (const uint2*)succ, word, msg, max_colors, color, (const int*)n_seeds, spill);
+    launch(color_push_kernel, blocks < 152 ? blocks : 152, CP_THREADS, smem, s, n_edges, (const uint2*)succ, word, msg, max_colors, color, (const int*)n_seeds, (const int*)seeds, spill);
     rc = check_launch("colour propagation");
     if (rc) return rc;
     // every block resident (its threads wait on one another)

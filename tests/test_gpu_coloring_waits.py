@@ -58,3 +58,35 @@ def test_the_block_finishes(pkg, po, name):
     assert status == 0 and spill == 0
     assert np.array_equal(out[0].cpu().numpy(), color) and np.array_equal(out[1].cpu().numpy(), order)
     assert np.array_equal(prefix.cpu().numpy(), start)
+
+
+def _paths(n, length):
+    """n paths of as many edges, one seed each, numbered one after the other."""
+    first = np.arange(n)[:, None] * (length + 1)
+    a = (first + np.arange(length)[None]).reshape(-1)
+    return n * (length + 1), np.stack([a, a + 1], 1)
+
+
+@pytest.mark.parametrize("name", ["64 paths", "65 paths", "153 paths", "20000 paths", "matching", "icosphere",
+                                  "shuffled", "few blocks"])
+def test_many_seeds(pkg, po, name):
+    from starlab_physics_gb300.mesh import edges_from_faces
+
+    rng = np.random.default_rng(7)
+    if name.endswith("paths"):
+        n = int(name.split()[0])
+        nv, e = _paths(n, 37 if n < 1000 else 4)
+    elif name == "matching":
+        nv, e = 40000, np.arange(40000).reshape(-1, 2)
+    elif name == "few blocks":  # fewer edges than a block of each SM takes, most of them seeds
+        nv, e = _paths(90, 2)
+    else:
+        f = pkg.icosphere(5, 0.3, (0.0, 0.0, 0.0))[1] if name == "icosphere" else pkg.grid_cloth(150)[1]
+        e, nv = edges_from_faces(f), int(f.max()) + 1
+        if name == "shuffled":
+            e = e[rng.permutation(len(e))]
+    gc = pkg.GraphColoring(nv, e.astype(np.int32))
+    color, order, start = po.color_edges(nv, np.ascontiguousarray(e, np.int32))
+    assert np.array_equal(gc.edges_color.cpu().numpy(), color)
+    assert np.array_equal(gc.sorted_edges_sequence_for_color.cpu().numpy(), order)
+    assert np.array_equal(gc.color_prefix_sum.cpu().numpy(), start)
