@@ -201,31 +201,39 @@ struct PairSolve {
 __device__ __forceinline__ int moved_mask(int kind, int dt) {
     return region_mask(dt) & (kind == VT_ST ? 0x1 : kind == TV_ST ? 0xE : 0xF);
 }
+template <typename A>
+__device__ __forceinline__ void pair_classify(A& ar, const V3 x[4], PairSolve& r) {
+    r.dt = d_type_PT(ar, x[0], x[1], x[2], x[3]);
+    r.d = pt_distance(ar, r.dt, x);
+}
+// gradients, schur complement and multiplier of a pair in contact
+template <typename A>
+__device__ __forceinline__ void pair_correction(A& ar, int kind, const V3 x[4], const float w[4], float dHat,
+                                                float compliance, PairSolve& r) {
+    pt_gradient(ar, r.dt, x, r.g);
+    const int m = moved_mask(kind, r.dt);
+    float s = 0.0f;
+    bool first = true;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float t = w[k] * dot(r.g[k], r.g[k]);
+        if (m & (1 << k)) {
+            s = first ? t : s + t;
+            first = false;
+        }
+    }
+    const float gap = dHat - r.d;
+    if (kind == VT_DY) s = s + 1e-4f;
+    r.ld = ar.div(kind == VT_DY ? gap : compliance * gap, kind == VT_DY ? s : compliance * s + 1.0f);
+    r.schur = s;
+}
 template <bool IEEE>
 __device__ __forceinline__ bool pair_solve(int kind, const V3 x[4], const float w[4], float dHat, float compliance,
                                            PairSolve& r) {
     Arith<IEEE> ar;
-    r.dt = d_type_PT(ar, x[0], x[1], x[2], x[3]);
-    r.d = pt_distance(ar, r.dt, x);
+    pair_classify(ar, x, r);
     r.schur = r.ld = 0.0f;
-    if (r.d < dHat) {
-        pt_gradient(ar, r.dt, x, r.g);
-        const int m = moved_mask(kind, r.dt);
-        float s = 0.0f;
-        bool first = true;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const float t = w[k] * dot(r.g[k], r.g[k]);
-            if (m & (1 << k)) {
-                s = first ? t : s + t;
-                first = false;
-            }
-        }
-        const float gap = dHat - r.d;
-        if (kind == VT_DY) s = s + 1e-4f;
-        r.ld = ar.div(kind == VT_DY ? gap : compliance * gap, kind == VT_DY ? s : compliance * s + 1.0f);
-        r.schur = s;
-    }
+    if (r.d < dHat) pair_correction(ar, kind, x, w, dHat, compliance, r);
     return ar.ok();
 }
 
@@ -307,6 +315,28 @@ __device__ __forceinline__ void pair_project(int kind, int4 v, const V3 x[4], co
         *bad |= pair_project_ieee(kind, v, x[0], x[1], x[2], x[3], fixed, m_inv, dHat, compliance, dx, nc);
     else if (r.d < dHat)
         pair_apply(kind, vv, mi, w, r, dx, nc, bad);
+}
+
+// The same for kernels that are short of registers: without a call, the weights and
+// gradients (with '/', which takes fewer) only of a pair in contact.  In the
+// persistent substep, 64 registers a thread, pair_project spills and its call keeps
+// registers from the sweep: frames of 512 / 64 falling cloths in fast arithmetic 24.1 /
+// 4.9 ms with it, 23.1 / 4.6 with this (23.3 / 4.6 with no projection in the kernel),
+// of 512 lying on their boxes 57.9 and 50.5.
+__device__ __forceinline__ void pair_project_lean(int kind, int4 v, const V3 x[4], const float* __restrict__ fixed,
+                                                  const float* __restrict__ m_inv, float dHat, float compliance,
+                                                  long long* dx, int* nc, int* bad) {
+    PairSolve r;
+    Arith<false> ar;
+    Arith<true> ieee;
+    pair_classify(ar, x, r);
+    if (!ar.ok()) pair_classify(ieee, x, r);
+    if (!(r.d < dHat)) return;
+    const int vv[4] = {v.x, v.y, v.z, v.w};
+    float mi[4], w[4];
+    pair_weights(kind, vv, fixed, m_inv, mi, w);
+    pair_correction(ieee, kind, x, w, dHat, compliance, r);
+    pair_apply(kind, vv, mi, w, r, dx, nc, bad);
 }
 
 // The same, for the walk that records its pairs: r also receives the region,
@@ -1778,8 +1808,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) batched_substep_kernel(BatchedSub
                             const int f = of0 + kk;
                             const V3 x[4] = {x0, mk(A.xs4[A.ob_faces[3 * f]]), mk(A.xs4[A.ob_faces[3 * f + 1]]),
                                              mk(A.xs4[A.ob_faces[3 * f + 2]])};
-                            pair_project(VT_ST, make_int4(v, -1, -1, -1), x, A.fixed, A.m_inv, A.dHat, A.compliance,
-                                         A.dx, A.nc, &bad);
+                            pair_project_lean(VT_ST, make_int4(v, -1, -1, -1), x, A.fixed, A.m_inv, A.dHat,
+                                              A.compliance, A.dx, A.nc, &bad);
                         }
                     }
                 } else {
@@ -1789,7 +1819,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) batched_substep_kernel(BatchedSub
                         const int fd = A.tv_cand[(size_t)s * A.cap + j];
                         const int4 vv = make_int4(-1, A.faces[3 * fd], A.faces[3 * fd + 1], A.faces[3 * fd + 2]);
                         const V3 x[4] = {mk(A.xs4[s]), mk(yout[vv.y]), mk(yout[vv.z]), mk(yout[vv.w])};
-                        pair_project(TV_ST, vv, x, A.fixed, A.m_inv, A.dHat, A.compliance, A.dx, A.nc, &bad);
+                        pair_project_lean(TV_ST, vv, x, A.fixed, A.m_inv, A.dHat, A.compliance, A.dx, A.nc, &bad);
                     }
                 }
             }
