@@ -652,7 +652,7 @@ __device__ __forceinline__ V3 load_cg(const float4* p) {
 // root, r when it is a left child (l / s even) and l when it is a right child;
 // a leaf is slot + 32767.  The refit therefore needs no climbing: one block
 // per z-column (32 leaves, an aligned subtree) fits its leaves and the
-// subtree's 31 nodes in shared memory, and a second kernel fits the 1023
+// subtree's 31 nodes in shared memory, and the last block to finish fits the 1023
 // nodes above the columns level by level.
 __device__ __forceinline__ int cell_node_index(int l, int size) {
     if (size == kNumCells) return 0;
@@ -1453,7 +1453,7 @@ __global__ void __launch_bounds__(128) face_traverse_kernel(int n, int Q, const 
 using namespace sx;
 
 // ---- workspace layouts --------------------------------------------------------
-// cell BVH: [keys F][radix ws F][flags NC] ; init uses [codes NC][radix ws NC]
+// cell BVH: [keys F][radix ws F] ; init uses [codes NC][radix ws NC]
 extern "C" size_t sx_radix_sort_workspace_bytes(int n) { return rs_ws_bytes(n); }
 
 extern "C" size_t sx_cell_bvh_workspace_bytes(int n_faces) {

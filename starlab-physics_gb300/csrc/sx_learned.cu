@@ -498,7 +498,7 @@ __device__ __forceinline__ float2 silu2(float2 z) {
 
 // 32 accumulator columns of this thread's row (at taddr) + bias -> SiLU ->
 // BF16 columns [c0, c0 + 32) of row `row` of A; 16 at a time, which keeps the
-// kernel at 40 registers
+// kernel at 48 registers
 __device__ __forceinline__ void tc_hidden_half(unsigned taddr, const float* bias, unsigned short* A, int row, int c0) {
 #pragma unroll
     for (int p = 0; p < 2; ++p) {
