@@ -346,10 +346,10 @@ class Solver:
             s1.wait_event(fork)
             s2.wait_event(fork)
         if self.mesh_st is not None:
-            self.lbvh_st.traverse(m.y4, self.padding, cap, self.vt_st_candidates, self.vt_st_candidates_num,
-                                  self.status, stream=s1)
-            self.lbvh_dy.traverse(self.mesh_st.x4, self.padding, cap, self.tv_st_candidates,
-                                  self.tv_st_candidates_num, self.status, stream=s2)
+            self._traverse_on(s1, self.lbvh_st, m.y4, self.padding, cap, self.vt_st_candidates,
+                              self.vt_st_candidates_num, self.status)
+            self._traverse_on(s2, self.lbvh_dy, self.mesh_st.x4, self.padding, cap, self.tv_st_candidates,
+                              self.tv_st_candidates_num, self.status)
         if self.self_collision:
             self.lbvh_dy.traverse(m.y4, self.padding, cap, self.vt_dy_candidates, self.vt_dy_candidates_num,
                                   self.status)
@@ -368,6 +368,19 @@ class Solver:
                                             ee["st_n"], self.status)
             self.lbvh_dy.traverse_edges(m.edge_indices, m.num_edges, m.y4, self.padding, cap, ee["dy_c"], ee["dy_n"],
                                         self.status)
+
+    @staticmethod
+    def _traverse_on(stream, tree, *args):
+        """``tree.traverse`` on a stream (None: the current one).  The library's own
+        takes the stream as an argument, which spares making it current; a tree of a
+        user's own finds it current."""
+        if stream is None:
+            tree.traverse(*args)
+        elif getattr(tree.traverse, "__func__", None) is LBVH_CELL.traverse:
+            tree.traverse(*args, stream=stream)
+        else:
+            with torch.cuda.stream(stream):
+                tree.traverse(*args)
 
     def _ensure_ee(self):
         """Edge-edge candidate lists (and records with record_pairs): blocks of
