@@ -392,7 +392,8 @@ class TriMesh:
     def packed_is_current(self) -> bool:
         """Whether ``adj_nbr16`` / ``adj_rest32`` still are the packed copy of ``adj``
         (:class:`TensorState` says which edits it sees)."""
-        return self._packed_state.unchanged(self.adj, self.adj_nbr16, self.adj_rest32)
+        state = getattr(self, "_packed_state", None)  # (a mesh pickled before it was kept has none)
+        return state is not None and state.unchanged(self.adj, self.adj_nbr16, self.adj_rest32)
 
     # -- state ---------------------------------------------------------------
     def _load_rest(self):

@@ -127,7 +127,8 @@ class Solver:
         self._sweep_variant = None
         self._default_variant = [int(sx.sx_jacobi_sweep_default_variant(mesh_dy.num_verts, f)) for f in (0, 1)]
         self._default_packed = [int(sx.sx_jacobi_sweep_default_packed_form(mesh_dy.num_verts, f))
-                                if mesh_dy.adj_nbr16 is not None else -1 for f in (0, 1)]
+                                if getattr(mesh_dy, "adj_nbr16", None) is not None
+                                and hasattr(mesh_dy, "packed_is_current") else -1 for f in (0, 1)]
         self._capturing = False  # a frame's graph, whose key tells the sweep's form
         self._packed_sweep = False
         self.packed_form = 0  # the packed sweep staged per block (0) or read from global memory (1)

@@ -97,3 +97,19 @@ def test_a_users_own_graph_reads_the_adjacency(pkg):
     sim.spring_sweep(1e-3)
     torch.cuda.synchronize()
     assert torch.equal(got, mesh.y4) and not torch.equal(got, start)
+
+
+def test_meshes_without_the_copys_state(pkg, monkeypatch):
+    """A mesh from a file that has no state, and one of a user's own class without
+    packed arrays: swept over ``mesh.adj``."""
+    mesh = _mesh(pkg)
+    sim = _solver(pkg, mesh, monkeypatch)
+    del mesh._packed_state
+    assert sim._packed_choice(1) == -1
+
+    class Own:
+        def __init__(self, m):
+            self.__dict__.update({k: v for k, v in vars(m).items() if k not in ("adj_nbr16", "adj_rest32")})
+
+    sim = pkg.Solver(Own(mesh), None, 4e-6, 1e5, 1e8, (0.0, 0.0, -9.81), 1 / 60, bending_on="y")
+    assert sim._default_packed == [-1, -1] and sim._packed_choice(1) == -1
