@@ -254,7 +254,7 @@ class Solver:
             cons, start, n_colors = self.gs_setup()
             sx.sx_gs_sweep(ptr(m.y4), ptr(cons), start, n_colors, k_spring, k_bend, stream_handle())
             return
-        track = self._track if self._heads_on else (None, None, None)
+        track = self._track() if self._heads_on else (None, None, None)
         form = self._packed_choice(fast)
         if self.tol is None and form >= 0:
             sx.sx_jacobi_sweep_packed_tracked(ptr(m.x4), ptr(m.y4), ptr(self._y_other), ptr(m.fixed), ptr(m.adj_ptr),
@@ -535,9 +535,11 @@ class Solver:
             self._heads = (torch.zeros(nb, dtype=torch.uint8, device=dev),
                            torch.zeros((V, 4), dtype=torch.float32, device=dev),
                            torch.zeros((V + 31) // 32, dtype=torch.int32, device=dev))
-            # reference positions, motion, the pair list's counts
-            self._track = (ptr(self._heads[1]), ptr(self._heads[2]),
-                           ptr(self._pairs_ws) + self._pairs_ws.numel() - 256)
+
+    def _track(self):
+        """Reference positions, motion and the pair list's counts for a tracked sweep."""
+        _, ref, moved = self._heads
+        return ptr(ref), ptr(moved), ptr(self._pairs_ws) + self._pairs_ws.numel() - 256
 
     def _write_heads(self):
         """Heads of this substep's pair list (sx_contact_pairs_heads); from here to
